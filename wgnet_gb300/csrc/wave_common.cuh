@@ -38,6 +38,8 @@ struct Grid {
   int nt;
   const float* prof;   // ax bx dbx (nx each) | az bz dbz (nz each)
   const float* wavelet;  // [nt]
+  // -0, for products that must not be contracted with the sum that reads them (wave_kernels3.cuh)
+  alignas(8) float nz2[2] = {-0.0f, -0.0f};
 };
 
 // Sources and receivers: 4 bilinear corners each (wave_wgpu.rs:217-230).

@@ -110,8 +110,55 @@ struct FastCoef {
   __device__ __forceinline__ float d1(float dd1, float dd2) const { return fmaf(e2, dd2, e1 * dd1); }
 };
 
+// Packed FP32 arithmetic: a thread's column pair is one operand, each half rounded to nearest as the
+// scalar operation is. ptxas contracts a packed product and sum into a packed fma even under
+// -fmad=false and with explicit .rn, which would round once where the reference rounds twice. So a
+// product that feeds a sum is formed as fma(a, b, -0) with the -0 taken from the kernel's arguments,
+// where the compiler cannot see it: a b + (-0) is the rounded product bit for bit (signs of zeros
+// included), and an fma is not contracted again.
+//
+// The forward's row update is packed: 320 units x 200 steps on the 70 x 70 grid take 2.98 against
+// 3.15 ms recording traces and 1.50 against 1.61 ms storing terms (100 steps). The packed fma issues
+// at half rate, so the arithmetic itself is no faster; what is saved are issue slots. The adjoint
+// stays scalar: packed, it took 5.28 against 4.84 ms (it waits on shared memory and instruction
+// fetch, not on issue slots).
+struct Pk {
+  float2 nz;  // (-0, -0), opaque
+  __device__ __forceinline__ float2 mul(float2 a, float2 b) const { return __ffma2_rn(a, b, nz); }
+  __device__ __forceinline__ float2 scale(float a, float2 b) const { return mul(make_float2(a, a), b); }
+  // (((D2A u + D2B s1) - D2C s2) ka) kb; s1 / s2: sums of the neighbours at distance 1 / 2 (the
+  // adjoint's (x + (-D2C) s2) is the same value)
+  __device__ __forceinline__ float2 second(float2 u, float2 s1, float2 s2, float ka, float kb) const;
+  // ((D1A d1) - D1B d2) rh; d1 / d2: differences of the neighbours at distance 1 / 2
+  __device__ __forceinline__ float2 first(float2 d1, float2 d2, float rh) const;
+};
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tsub.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+// a product that no sum reads (its reader is a store or another product)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 scale2(float a, float2 b) { return mul2(dup2(a), b); }
+// Sums and differences at distance 1 along x of the own pair u between the pairs a (left) and b
+// (right): they join an own column and a neighbour's, so they are formed per column.
+__device__ __forceinline__ float2 side_sum(float2 a, float2 u, float2 b) { return make_float2(u.y + a.y, b.x + u.x); }
+__device__ __forceinline__ float2 side_diff(float2 a, float2 u, float2 b) { return make_float2(u.y - a.y, b.x - u.x); }
+__device__ __forceinline__ float2 Pk::second(float2 u, float2 s1, float2 s2, float ka, float kb) const {
+  return scale(kb, scale2(ka, add2(add2(scale(F_D2A, u), scale(F_D2B, s1)), scale(-F_D2C, s2))));
+}
+__device__ __forceinline__ float2 Pk::first(float2 d1, float2 d2, float rh) const {
+  return scale(rh, add2(scale(F_D1A, d1), scale(-F_D1B, d2)));
+}
+
 __device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void sts2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void sts2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
 // Store to the peer CTA's copy of a shared array. The address translation is a pure function; the
 // store has no memory clobber, so it does not pin this thread's other shared-memory accesses, none
@@ -146,6 +193,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   const int sw = g.sw, region = g.region, nrec = p.st.nrec;
   const float rh = g.rh, dt2 = g.dt2, d2a = g.d2a, d2b = g.d2b;
   const FastCoef fc = FastCoef::make(rh);
+  const Pk pk{make_float2(g.nz2[0], g.nz2[1])};
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int seg = warp / (1 + NI), wk = warp_role<NI>(warp);
   const int rank = (C > 1) ? static_cast<int>(cluster_rank()) : 0;
@@ -208,8 +256,10 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
     dbx1 = g.prof[2 * NX + x + 1];
   }
   const float opbx0 = 1.0f + bx0, opbx1 = 1.0f + bx1;
+  const float2 ax = make_float2(ax0, ax1), bx = make_float2(bx0, bx1), dbx = make_float2(dbx0, dbx1),
+               opbx = make_float2(opbx0, opbx1);
 
-  float uA[S][2], uB[S][2];
+  float2 uA[S], uB[S];
   unsigned srcmask = 0;
   const int* sc = p.st.src_cell + 4 * shot;
   const float* vel = p.vel + static_cast<size_t>(model) * cells + gbase;
@@ -232,7 +282,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   float* C2o = sm + L.off_c2 + (zb - r0) * NX + x;
 #pragma unroll
   for (int i = 0; i < S; ++i) {
-    uA[i][0] = uA[i][1] = uB[i][0] = uB[i][1] = 0.f;
+    uA[i] = uB[i] = make_float2(0.f, 0.f);
     if (i < nrows) {
       const float2 v = __ldg(reinterpret_cast<const float2*>(vel + i * NX));
       sts2(V2o + i * NX, v.x * v.x * dt2, v.y * v.y * dt2);
@@ -266,8 +316,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int xx = x + j;
-          uA[i][j] = cU[z * NX + xx];
-          uB[i][j] = cP[z * NX + xx];
+          (j ? uA[i].y : uA[i].x) = cU[z * NX + xx];
+          (j ? uB[i].y : uB[i].x) = cP[z * NX + xx];
           if (xx < sw || xx >= NX - sw) {
             const int xc = strip_col(xx, NX, sw);
             APX[abase + i * 2 * SW + j] = cAX[z * 2 * sw + xc];
@@ -289,7 +339,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 
   const int pr_lo = (rank > 0) ? split_row(nz, C, rank - 1) - FD_PAD : 0;
 
-  auto step = [&](int t, float (&uc)[S][2], float (&un)[S][2]) {
+  auto step = [&](int t, float2 (&uc)[S], float2 (&un)[S]) {
     const int par = (t - p.t0) & 1;
     const float* Uc = U + par * ustride + ubase;
     float* Un = U + (1 - par) * ustride + ubase;
@@ -313,8 +363,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             const int xx = x + j;
-            ck[z * NX + xx] = uc[i][j];
-            ck[cells + z * NX + xx] = un[i][j];
+            ck[z * NX + xx] = j ? uc[i].y : uc[i].x;
+            ck[cells + z * NX + xx] = j ? un[i].y : un[i].x;
             if (xx < sw || xx >= NX - sw) {
               const int xc = strip_col(xx, NX, sw);
               cAX[z * 2 * sw + xc] = APXc[i * 2 * SW + j];
@@ -342,40 +392,13 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
           const int z = zb + i;
           const float2 A = lds2(Uc + i * NX - 2);
           const float2 B = lds2(Uc + i * NX + 2);
-          float zm2[2], zm1[2], zp1[2], zp2[2];
-          if (i >= 2) {
-            zm2[0] = uc[i - 2][0];
-            zm2[1] = uc[i - 2][1];
-          } else {
-            const float2 q = lds2(Uc + (i - 2) * NX);
-            zm2[0] = q.x;
-            zm2[1] = q.y;
-          }
-          if (i >= 1) {
-            zm1[0] = uc[i - 1][0];
-            zm1[1] = uc[i - 1][1];
-          } else {
-            const float2 q = lds2(Uc + (i - 1) * NX);
-            zm1[0] = q.x;
-            zm1[1] = q.y;
-          }
-          if (i + 1 < S && (FULL || i + 1 < nrows)) {
-            zp1[0] = uc[i + 1 < S ? i + 1 : i][0];
-            zp1[1] = uc[i + 1 < S ? i + 1 : i][1];
-          } else {
-            const float2 q = lds2(Uc + (i + 1) * NX);
-            zp1[0] = q.x;
-            zp1[1] = q.y;
-          }
-          if (i + 2 < S && (FULL || i + 2 < nrows)) {
-            zp2[0] = uc[i + 2 < S ? i + 2 : i][0];
-            zp2[1] = uc[i + 2 < S ? i + 2 : i][1];
-          } else {
-            const float2 q = lds2(Uc + (i + 2) * NX);
-            zp2[0] = q.x;
-            zp2[1] = q.y;
-          }
-          const float u0 = uc[i][0], u1 = uc[i][1];
+          // rows of the segment sit in registers, the rows around it in shared memory
+          const float2 zm2 = i >= 2 ? uc[i >= 2 ? i - 2 : 0] : lds2(Uc + (i - 2) * NX);
+          const float2 zm1 = i >= 1 ? uc[i >= 1 ? i - 1 : 0] : lds2(Uc + (i - 1) * NX);
+          const float2 zp1 = i + 1 < S && (FULL || i + 1 < nrows) ? uc[i + 1 < S ? i + 1 : i] : lds2(Uc + (i + 1) * NX);
+          const float2 zp2 = i + 2 < S && (FULL || i + 2 < nrows) ? uc[i + 2 < S ? i + 2 : i] : lds2(Uc + (i + 2) * NX);
+          const float2 u = uc[i];
+          const float u0 = u.x, u1 = u.y;
           float n0, n1;
           if constexpr (FA) {
             // the same update, reassociated: 1/h and 1/h^2 folded into the stencil weights, the
@@ -402,12 +425,12 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               sts2(zxo + i * 2 * SW, fmaf(bx0, tmp0, az0), fmaf(bx1, tmp1, az1));
               sts2(apxn + i * 2 * SW, ax0 * fmaf(bx0, d10, P1.x), ax1 * fmaf(bx1, d11, P1.y));
               if (!zpml) {
-                w0 = fc.d2acc(w0, u0, zp1[0] + zm1[0], zp2[0] + zm2[0]);
-                w1 = fc.d2acc(w1, u1, zp1[1] + zm1[1], zp2[1] + zm2[1]);
+                w0 = fc.d2acc(w0, u0, zp1.x + zm1.x, zp2.x + zm2.x);
+                w1 = fc.d2acc(w1, u1, zp1.y + zm1.y, zp2.y + zm2.y);
               }
             } else if (!zpml) {  // interior in both axes: one weighted sum of both axes' neighbours
-              w0 = fc.lap(u0, (u1 + A.y) + (zp1[0] + zm1[0]), (B.x + A.x) + (zp2[0] + zm2[0]));
-              w1 = fc.lap(u1, (B.x + u0) + (zp1[1] + zm1[1]), (B.y + A.y) + (zp2[1] + zm2[1]));
+              w0 = fc.lap(u0, (u1 + A.y) + (zp1.x + zm1.x), (B.x + A.x) + (zp2.x + zm2.x));
+              w1 = fc.lap(u1, (B.x + u0) + (zp1.y + zm1.y), (B.y + A.y) + (zp2.y + zm2.y));
             } else {
               w0 = fc.d2(u0, u1 + A.y, B.x + A.x);
               w1 = fc.d2(u1, B.x + u0, B.y + A.y);
@@ -421,10 +444,10 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               const float2 Qp1 = lds2(APZc + (i + 1) * NX);
               const float2 Qp2 = lds2(APZc + (i + 2) * NX);
               const float2 Z = lds2(zzo + i * NX);
-              const float d2z0 = fc.d2(u0, zp1[0] + zm1[0], zp2[0] + zm2[0]);
-              const float d2z1 = fc.d2(u1, zp1[1] + zm1[1], zp2[1] + zm2[1]);
-              const float d10 = fc.d1(zp1[0] - zm1[0], zp2[0] - zm2[0]);
-              const float d11 = fc.d1(zp1[1] - zm1[1], zp2[1] - zm2[1]);
+              const float d2z0 = fc.d2(u0, zp1.x + zm1.x, zp2.x + zm2.x);
+              const float d2z1 = fc.d2(u1, zp1.y + zm1.y, zp2.y + zm2.y);
+              const float d10 = fc.d1(zp1.x - zm1.x, zp2.x - zm2.x);
+              const float d11 = fc.d1(zp1.y - zm1.y, zp2.y - zm2.y);
               const float da0 = fc.d1(Qp1.x - Qm1.x, Qp2.x - Qm2.x);
               const float da1 = fc.d1(Qp1.y - Qm1.y, Qp2.y - Qm2.y);
               const float tmp0 = fmaf(opbz, d2z0, fmaf(dbz, d10, da0));
@@ -440,68 +463,48 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               const float2 cc = lds2(C2o + i * NX);
               *reinterpret_cast<float2*>(stg + i * NX) = make_float2(cc.x * w0, cc.y * w1);
             }
-            n0 = fmaf(vv.x, w0, fmaf(2.0f, u0, -un[i][0]));
-            n1 = fmaf(vv.y, w1, fmaf(2.0f, u1, -un[i][1]));
+            n0 = fmaf(vv.x, w0, fmaf(2.0f, u0, -un[i].x));
+            n1 = fmaf(vv.y, w1, fmaf(2.0f, u1, -un[i].y));
           } else {
-            const float d2x0 = (((F_D2A * u0 + F_D2B * (u1 + A.y)) - F_D2C * (B.x + A.x)) * d2a) * d2b;
-            const float d2x1 = (((F_D2A * u1 + F_D2B * (B.x + u0)) - F_D2C * (B.y + A.y)) * d2a) * d2b;
-            float w0, w1;
+            float2 w = pk.second(u, side_sum(A, u, B), add2(B, A), d2a, d2b);
             if (pml) {
               const float2 P0 = lds2(APXc + i * 2 * SW - 2);
               const float2 P1 = lds2(APXc + i * 2 * SW);
               const float2 P2 = lds2(APXc + i * 2 * SW + 2);
               const float2 Z = lds2(zxo + i * 2 * SW);
-              const float d10 = ((F_D1A * (u1 - A.y)) - F_D1B * (B.x - A.x)) * rh;
-              const float d11 = ((F_D1A * (B.x - u0)) - F_D1B * (B.y - A.y)) * rh;
-              const float da0 = ((F_D1A * (P1.y - P0.y)) - F_D1B * (P2.x - P0.x)) * rh;
-              const float da1 = ((F_D1A * (P2.x - P1.x)) - F_D1B * (P2.y - P0.y)) * rh;
-              const float tmp0 = ((opbx0 * d2x0) + (dbx0 * d10)) + da0;
-              const float tmp1 = ((opbx1 * d2x1) + (dbx1 * d11)) + da1;
-              w0 = (opbx0 * tmp0) + (ax0 * Z.x);
-              w1 = (opbx1 * tmp1) + (ax1 * Z.y);
-              const float psi0 = (bx0 * d10) + P1.x;
-              const float psi1 = (bx1 * d11) + P1.y;
-              sts2(zxo + i * 2 * SW, (bx0 * tmp0) + (ax0 * Z.x), (bx1 * tmp1) + (ax1 * Z.y));
-              sts2(apxn + i * 2 * SW, ax0 * psi0, ax1 * psi1);
-            } else {
-              w0 = d2x0;
-              w1 = d2x1;
+              const float2 d1 = pk.first(side_diff(A, u, B), sub2(B, A), rh);
+              const float2 da = pk.first(side_diff(P0, P1, P2), sub2(P2, P0), rh);
+              const float2 tmp = add2(add2(pk.mul(opbx, w), pk.mul(dbx, d1)), da);
+              const float2 az = pk.mul(ax, Z);
+              w = add2(pk.mul(opbx, tmp), az);
+              sts2(zxo + i * 2 * SW, add2(pk.mul(bx, tmp), az));
+              sts2(apxn + i * 2 * SW, mul2(ax, add2(pk.mul(bx, d1), P1)));
             }
-            const float d2z0 = (((F_D2A * u0 + F_D2B * (zp1[0] + zm1[0])) - F_D2C * (zp2[0] + zm2[0])) * d2a) * d2b;
-            const float d2z1 = (((F_D2A * u1 + F_D2B * (zp1[1] + zm1[1])) - F_D2C * (zp2[1] + zm2[1])) * d2a) * d2b;
+            const float2 d2z = pk.second(u, add2(zp1, zm1), add2(zp2, zm2), d2a, d2b);
             if (z < region || z >= nz - region) {
-              const float az = sAZ[z], bz = sBZ[z], dbz = sDBZ[z];
-              const float opbz = 1.0f + bz;
+              const float2 az = dup2(sAZ[z]), bz = dup2(sBZ[z]), dbz = dup2(sDBZ[z]);
+              const float2 opbz = dup2(1.0f + bz.x);
               const float2 Qm2 = lds2(APZc + (i - 2) * NX);
               const float2 Qm1 = lds2(APZc + (i - 1) * NX);
               const float2 Q0 = lds2(APZc + i * NX);
               const float2 Qp1 = lds2(APZc + (i + 1) * NX);
               const float2 Qp2 = lds2(APZc + (i + 2) * NX);
               const float2 Z = lds2(zzo + i * NX);
-              const float d10 = ((F_D1A * (zp1[0] - zm1[0])) - F_D1B * (zp2[0] - zm2[0])) * rh;
-              const float d11 = ((F_D1A * (zp1[1] - zm1[1])) - F_D1B * (zp2[1] - zm2[1])) * rh;
-              const float da0 = ((F_D1A * (Qp1.x - Qm1.x)) - F_D1B * (Qp2.x - Qm2.x)) * rh;
-              const float da1 = ((F_D1A * (Qp1.y - Qm1.y)) - F_D1B * (Qp2.y - Qm2.y)) * rh;
-              const float tmp0 = ((opbz * d2z0) + (dbz * d10)) + da0;
-              const float tmp1 = ((opbz * d2z1) + (dbz * d11)) + da1;
-              w0 = w0 + ((opbz * tmp0) + (az * Z.x));
-              w1 = w1 + ((opbz * tmp1) + (az * Z.y));
-              const float psi0 = (bz * d10) + Q0.x;
-              const float psi1 = (bz * d11) + Q0.y;
-              sts2(zzo + i * NX, (bz * tmp0) + (az * Z.x), (bz * tmp1) + (az * Z.y));
-              sts2(apzn + i * NX, az * psi0, az * psi1);
+              const float2 d1 = pk.first(sub2(zp1, zm1), sub2(zp2, zm2), rh);
+              const float2 da = pk.first(sub2(Qp1, Qm1), sub2(Qp2, Qm2), rh);
+              const float2 tmp = add2(add2(pk.mul(opbz, d2z), pk.mul(dbz, d1)), da);
+              const float2 aZ = pk.mul(az, Z);
+              w = add2(w, add2(pk.mul(opbz, tmp), aZ));
+              sts2(zzo + i * NX, add2(pk.mul(bz, tmp), aZ));
+              sts2(apzn + i * NX, mul2(az, add2(pk.mul(bz, d1), Q0)));
             } else {
-              w0 = w0 + d2z0;
-              w1 = w1 + d2z1;
+              w = add2(w, d2z);
             }
-            const float2 vv = lds2(V2o + i * NX);
-            const float v20 = vv.x, v21 = vv.y;
-            if (STORE) {  // written as the row is updated: holding them for after the barrier spilled registers
-              const float2 cc = lds2(C2o + i * NX);
-              *reinterpret_cast<float2*>(stg + i * NX) = make_float2(cc.x * w0, cc.y * w1);
-            }
-            n0 = ((v20 * w0) + (2.0f * u0)) - un[i][0];
-            n1 = ((v21 * w1) + (2.0f * u1)) - un[i][1];
+            // written as the row is updated: holding them for after the barrier spilled registers
+            if (STORE) *reinterpret_cast<float2*>(stg + i * NX) = mul2(lds2(C2o + i * NX), w);
+            const float2 n = sub2(add2(pk.mul(lds2(V2o + i * NX), w), add2(u, u)), un[i]);
+            n0 = n.x;
+            n1 = n.y;
           }
           if (wsrc & (3u << (2 * i))) {
             const int cell = gbase + i * NX;
@@ -514,8 +517,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               n1 = (cell + 1 == c) ? a1 : n1;
             }
           }
-          un[i][0] = n0;
-          un[i][1] = n1;
+          un[i] = make_float2(n0, n1);
           sts2(uw + i * NX, n0, n1);
           if constexpr (C > 1) {
             if (rank > 0 && z < r0 + FD_PAD) st_peer_v2(U + (1 - par) * ustride + (z - pr_lo) * NX + x, rank - 1, n0, n1);
