@@ -220,6 +220,32 @@ int wg_pc_mse(const float* d_out, int ld, const float* d_target, float scale, lo
 int wg_pc_adam(const float* d_partial, int splits, int n, int kp, float* d_w32, float* d_m1, float* d_m2, float lr,
                float b1, float b2, float eps, int step, void* d_w_bf16, void* d_wt_bf16, void* stream);
 
+/* Same-padded 3x3 convolution (dilation dil <= 60) of activations [batch][h][w][64] bf16 with a fused
+ * epilogue; y is the FP32 result per pixel and channel. mode
+ *   0: out16 = bf16(max(y, 0))
+ *   1: out16 = bf16(max(y, 0)), out32 = out16 > 0 ? y : 0; d_act is a matrix [pixels][kp] (columns)
+ *   2: out32 = add + y, out16 = bf16(out32) (out32 may be add)
+ *   3: out32[pixel] = y of channel 0
+ * and, the data gradient (d_act = dL/dy as bf16):
+ *   4: out16 = bf16(mask > 0 ? y : 0)
+ *   5: out32 = add + y, out16 = bf16(out32) (out32 may be add)
+ *   6: out16 = bf16(mask > 0 ? add + y : 0)
+ * Modes 0-3 take the weights [64][kp], modes 4-6 their transpose [kp][64]; kp = 576 except in mode 1.
+ * d_status: a device int that a timed-out wait sets. Bit-identical to im2col + wg_gemm_bf16_dev + the
+ * elementwise calls above. */
+int wg_pc_conv(int mode, const void* d_act_bf16, int batch, int h, int w, int dil, const void* d_wgt_bf16, int kp,
+               const float* d_add, const void* d_mask_bf16, float* d_out32, void* d_out16, int* d_status,
+               void* stream);
+/* Split partials [splits][576][64] of the convolution's transposed weight gradient from its input
+ * activations and dL/dy [pixels][64] bf16; columns > 0: the input is a matrix [pixels][columns] and a
+ * partial has `columns` rows. batch h w must be a multiple of 64. */
+int wg_pc_conv_wgrad(const void* d_act_bf16, int columns, const void* d_dy_bf16, int batch, int h, int w, int dil,
+                     int splits, float* d_partial, int* d_status, void* stream);
+/* Data gradient of a 64 -> 1 convolution: dh [pixels][64] and its bf16 copy from dL/dy [pixels] and
+ * column 0 of the transposed weights [576][64]; dout16[pixel][0] = bf16(dL/dy). */
+int wg_pc_out_dgrad(const float* d_dout, const void* d_wt_bf16, int batch, int h, int w, float* d_dh, void* d_dh16,
+                    void* d_dout16, void* stream);
+
 /* render_residual (python/wgnet/render.py:86-109): activated slot parameters [B][1225][6] ->
  * residual field [B][70][70] in km/s; and its vector-Jacobian product: cotangent [B][70][70] ->
  * parameter gradient [B][1225][6]. Device pointers. */

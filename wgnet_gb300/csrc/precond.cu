@@ -161,17 +161,22 @@ __global__ void mse_kernel(const float* __restrict__ out, int ld, const float* _
   if (threadIdx.x == 0) atomicAdd(loss, red[0] / static_cast<double>(M));
 }
 
-// Adam on FP32 master weights w32 [N][Kp]; the gradient is the sum of the split-K partials of the
-// transposed weight gradient [S][Kp][N]. Writes the BF16 weights [N][Kp] and their transpose.
+// Adam on FP32 master weights w32 [N][Kp]; the gradient is the sum, in split order, of the partials
+// of the transposed weight gradient [S][Kp][N]. Writes the BF16 weights [N][Kp] and their transpose.
+// Reading the partials bounds it (9.3 MB for 63 splits of a 64 -> 64 layer), so a warp takes 32
+// neighbouring n of one k: 128-byte lines of the partials, against which the strided accesses to the
+// four weight-sized arrays are few (with neighbouring k per warp it read eight times the bytes).
 __global__ void adam_kernel(const float* __restrict__ partial, int S, int N, int Kp, float* __restrict__ w32,
                             float* __restrict__ m1, float* __restrict__ m2, float lr, float b1, float b2, float eps,
                             float c1, float c2, __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt) {
-  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (i >= static_cast<long>(N) * Kp) return;
-  const int n = static_cast<int>(i / Kp), k = static_cast<int>(i % Kp);
+  const long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (t >= static_cast<long>(N) * Kp) return;
+  const int n = static_cast<int>(t % N), k = static_cast<int>(t / N);
+  const long i = static_cast<long>(n) * Kp + k;
   float g = 0.0f;
   if (partial) {
-    for (int s = 0; s < S; ++s) g += partial[(static_cast<long>(s) * Kp + k) * N + n];
+#pragma unroll 8
+    for (int s = 0; s < S; ++s) g += partial[static_cast<long>(s) * Kp * N + t];
     const float a = b1 * m1[i] + (1.0f - b1) * g;
     const float v = b2 * m2[i] + (1.0f - b2) * g * g;
     m1[i] = a;
@@ -180,7 +185,7 @@ __global__ void adam_kernel(const float* __restrict__ partial, int S, int N, int
   }
   const __nv_bfloat16 q = __float2bfloat16(w32[i]);
   w[i] = q;
-  wt[static_cast<long>(k) * N + n] = q;
+  wt[t] = q;
 }
 
 inline unsigned blocks(long n, int t) { return static_cast<unsigned>((n + t - 1) / t); }

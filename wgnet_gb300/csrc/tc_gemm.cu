@@ -15,89 +15,13 @@
 // owns TMEM lanes 32w..32w+31 = rows of the tile) and store it. Every wait is bounded: on time-out
 // the CTA records an error in the status word, waits (bounded) for its own work in flight, frees
 // its tensor memory and returns.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-#include <cuda_runtime.h>
-
-#include <cstdint>
-#include <string>
-
-#include "wave_launch.h"
-#include "wgnet_gb300.h"
+#include "tc_common.cuh"
 
 namespace wg {
 namespace {
 
 constexpr int BM = 128, BN = 64, BK = 64, STAGES = 4, NTHR = 128;
 constexpr unsigned kStageA = BM * BK * 2, kStageB = BN * BK * 2;  // bytes
-constexpr long kGemmWaitLimit = 1L << 22;
-
-__device__ __forceinline__ unsigned su32(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void bar_init(uint64_t* b, unsigned n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned parity) {
-  const unsigned a = su32(b);
-  for (long i = 0; i < kGemmWaitLimit; ++i) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tma2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* b) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-          "r"(su32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(su32(b))
-      : "memory");
-}
-
-// Shared-memory matrix descriptor, K-major with the 128-byte swizzle: rows of 128 bytes, atoms of
-// 8 rows (sbo = 1024 bytes between atoms along M/N; lbo unused for this layout, encoded as 1). The
-// tile base is 1024-byte aligned, so the base-offset field stays 0.
-__device__ __forceinline__ uint64_t sdesc_sw128(const void* p) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((su32(p) >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>(1) << 16;              // leading byte offset (unused), 16 bytes
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;      // stride byte offset: 8 rows x 128 bytes
-  d |= static_cast<uint64_t>(1) << 46;              // descriptor version for the 5th-generation tensor cores
-  d |= static_cast<uint64_t>(2) << 61;              // layout: 128-byte swizzle
-  return d;
-}
-
-// Instruction descriptor of kind::f16: BF16 A and B, FP32 D, both K-major, M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-  return (1u << 4)                                 // D format F32
-         | (1u << 7)                               // A format BF16
-         | (1u << 10)                              // B format BF16
-         | (static_cast<uint32_t>(n >> 3) << 17)   // N / 8
-         | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* b) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(b)) : "memory");
-}
 
 struct GemmArgs {
   int M, N, K;          // D is M x N; K a multiple of BK
@@ -245,34 +169,6 @@ __global__ void __launch_bounds__(NTHR, 1) gemm_bf16_kernel(const __grid_constan
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }
-  return fn;
-}
-
-// 2-D map over a row-major [rows][K] bf16 matrix, boxes of 64 elements (128 bytes) x box_rows,
-// written to shared memory with the 128-byte swizzle.
-int map_bf16(CUtensorMap* m, const void* base, long rows, long K, int box_rows) {
-  auto fn = encode();
-  if (!fn) return report_error(WG_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-  const cuuint32_t box[2] = {BK, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t es[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return report_error(WG_ERR_CUDA, ("cuTensorMapEncodeTiled(bf16) failed: " + std::to_string(r)).c_str());
-  return WG_OK;
 }
 
 constexpr size_t kGemmSmem = STAGES * (kStageA + kStageB) + (2 * STAGES + 1) * 8 + 16 + 1024;

@@ -9,10 +9,11 @@ proposed model update in km/s. It is a dilated residual convolution network, ~0.
     6 residual blocks, dilations 1, 2, 4, 8, 4, 2:  h = h + conv3x3_d1(ReLU(conv3x3_d(h)))
     conv3x3 64 -> 1 (x 0.25 km/s)
 
-Weights are BF16 with FP32 master copies; every convolution runs as a tensor-core GEMM
-(`wg_gemm_bf16_dev`, FP32 accumulation) on im2col columns, forward, data gradient and weight
-gradient alike; the glue (im2col/col2im, ReLU, residual adds, features, loss, Adam) is the
-library's own kernels. PyTorch only holds the buffers.
+Weights are BF16 with FP32 master copies; every convolution, its data gradient and its weight gradient
+run on the tensor cores with FP32 accumulation (`wg_pc_conv`, `wg_pc_conv_wgrad`), which read the
+activations' shifted pixels directly and finish ReLU, residual adds, masks and bf16 casts in their
+epilogues; only the 8-channel input goes through im2col columns. Features, loss and Adam are the
+library's own kernels too. PyTorch only holds the buffers.
 """
 
 from __future__ import annotations
@@ -31,6 +32,8 @@ CH = 64
 DILATIONS = (1, 2, 4, 8, 4, 2)
 OUT_SCALE = 0.25
 BANDS = (6.0, 9.0, 12.0, None)
+# epilogues of wg_pc_conv
+FWD_RELU, FWD_FIRST, FWD_RESIDUAL, FWD_OUT, DGRAD_MASK, DGRAD_ADD, DGRAD_ADD_MASK = range(7)
 
 
 def band_index(band_hz) -> int:
@@ -140,40 +143,24 @@ class UpdateNet:
             self._bufs[key] = b
         return b
 
-    def _conv(self, L: Layer, x_bf16, B, H, W, out):
+    def _conv(self, mode, L: Layer, x, shape, out16=None, out32=None, add=None, mask=None):
+        """One fused convolution (modes of wg_pc_conv); the data-gradient modes take L's transposed
+        weights."""
+        B, H, W = shape
+        ptr = lambda t: None if t is None else _p(t)  # noqa: E731
+        check(self._lib.wg_pc_conv(mode, _p(x), B, H, W, L.dil, _p(L.wt if mode >= DGRAD_MASK else L.w), L.kp, ptr(add),
+                                   ptr(mask), ptr(out32), ptr(out16), _p(self._status), _stream()), "conv")
+
+    def _wgrad(self, L: Layer, x, dy16, shape, splits, columns=0):
+        """Weight gradient partials of L from its input (or the input's columns) and the bf16 dL/dy."""
         import torch
 
-        M = B * H * W
-        col = self._buf(f"col{L.kp}", (M, L.kp), torch.bfloat16)
-        check(self._lib.wg_pc_im2col(_p(x_bf16), B, H, W, L.cin, L.dil, L.kp, _p(col), _stream()), "im2col")
-        check(self._lib.wg_gemm_bf16_dev(_p(col), _p(L.w), _p(out), M, L.n, L.kp, 1, _p(self._status), _stream()),
-              "gemm")
-        return out
-
-    def _backward_conv(self, L: Layer, x_bf16, dy, B, H, W, splits, need_dx, dx=None, accumulate=0):
-        """Weight gradient partials of L (returned) and, if need_dx, dx (+)= the data gradient."""
-        import torch
-
-        M = B * H * W
-        dy16 = self._buf("dy16", (M, L.n), torch.bfloat16)
-        check(self._lib.wg_pc_cast_bf16(_p(dy), M, L.n, L.n, 0, _p(dy16), _stream()))
-        col = self._buf(f"col{L.kp}", (M, L.kp), torch.bfloat16)
-        check(self._lib.wg_pc_im2col(_p(x_bf16), B, H, W, L.cin, L.dil, L.kp, _p(col), _stream()))
-        colT = self._buf(f"colT{L.kp}", (L.kp, M), torch.bfloat16)
-        check(self._lib.wg_pc_transpose_bf16(_p(col), M, L.kp, _p(colT), _stream()))
-        dyT = self._buf("dyT", (L.n, M), torch.bfloat16)
-        check(self._lib.wg_pc_transpose_bf16(_p(dy16), M, L.n, _p(dyT), _stream()))
-        kt = M // 64
-        per = -(-kt // splits)
-        nz = -(-kt // per)
+        B, H, W = shape
+        kt = B * H * W // 64
+        nz = -(-kt // -(-kt // splits)) if kt else 1
         part = torch.empty((nz, L.kp, L.n), device=self.device, dtype=torch.float32)
-        check(self._lib.wg_gemm_bf16_dev(_p(colT), _p(dyT), _p(part), L.kp, L.n, M, splits, _p(self._status),
+        check(self._lib.wg_pc_conv_wgrad(_p(x), columns, _p(dy16), B, H, W, L.dil, splits, _p(part), _p(self._status),
                                          _stream()), "gemm wgrad")
-        if need_dx:
-            dcol = self._buf(f"dcol{L.kp}", (M, L.kp), torch.float32)
-            check(self._lib.wg_gemm_bf16_dev(_p(dy16), _p(L.wt), _p(dcol), M, L.kp, L.n, 1, _p(self._status),
-                                             _stream()), "gemm dgrad")
-            check(self._lib.wg_pc_col2im(_p(dcol), B, H, W, L.cin, L.dil, L.kp, _p(dx), accumulate, _stream()))
         return part
 
     # -- forward / training -----------------------------------------------------------------------
@@ -188,41 +175,47 @@ class UpdateNet:
             self._status = torch.zeros(4, device=self.device, dtype=torch.int32)
         B, H, W = vel_km.shape
         M = B * H * W
+        shape = (B, H, W)
+
+        def bf16(cols):
+            return torch.empty((M, cols), device=self.device, dtype=torch.bfloat16)
+
+        def f32():
+            return torch.empty((M, CH), device=self.device, dtype=torch.float32)
+
         rms = self._buf("rms", (B,), torch.float32)
-        x0 = torch.empty((M, CIN), device=self.device, dtype=torch.bfloat16)
+        x0 = bf16(CIN)
         check(self._lib.wg_pc_features(_p(vel_km.contiguous()), _p(grad.contiguous()), _p(band.contiguous()), B, H,
                                        W, _p(rms), _p(x0), _stream()), "features")
-        saved = {"x0": x0, "shape": (B, H, W)}
         L = self.layers[0]
-        y = self._buf("y", (M, CH), torch.float32)
-        self._conv(L, x0, B, H, W, y)
-        h16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
-        check(self._lib.wg_pc_cast_bf16(_p(y), M, CH, CH, 1, _p(h16), _stream()))
-        h = torch.empty((M, CH), device=self.device, dtype=torch.float32)
-        check(self._lib.wg_pc_relu_grad(_p(y), _p(h16), M * CH, _p(h), _stream()))
-        saved["h0"] = h16
+        col = bf16(L.kp)
+        check(self._lib.wg_pc_im2col(_p(x0), B, H, W, L.cin, L.dil, L.kp, _p(col), _stream()), "im2col")
+        h16, h = bf16(CH), f32()
+        self._conv(FWD_FIRST, L, col, shape, out16=h16, out32=h)
+        saved = {"x0": x0, "shape": shape, "h0": h16, "col0": col}
         blocks = []
+        a16 = None
         for i in range(len(DILATIONS)):
             La, Lb = self.layers[1 + 2 * i], self.layers[2 + 2 * i]
-            self._conv(La, h16, B, H, W, y)
-            a16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
-            check(self._lib.wg_pc_cast_bf16(_p(y), M, CH, CH, 1, _p(a16), _stream()))
-            self._conv(Lb, a16, B, H, W, y)
-            hn = torch.empty((M, CH), device=self.device, dtype=torch.float32)
-            hn16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
-            check(self._lib.wg_pc_add(_p(h), _p(y), M * CH, _p(hn), _p(hn16), _stream()))
+            if a16 is None or keep:
+                a16 = bf16(CH)
+            self._conv(FWD_RELU, La, h16, shape, out16=a16)
+            # the block's output; without `keep` it takes its input's place (the second convolution
+            # reads a16 only)
+            hn, hn16 = (f32(), bf16(CH)) if keep else (h, h16)
+            self._conv(FWD_RESIDUAL, Lb, a16, shape, out16=hn16, out32=hn, add=h)
             blocks.append((h16, a16, h))
             h, h16 = hn, hn16
-        saved["blocks"] = blocks
-        saved["hlast"] = h16
-        saved["hlast32"] = h
-        out = torch.empty((M, CH), device=self.device, dtype=torch.float32)
-        self._conv(self.layers[-1], h16, B, H, W, out)
+        out = torch.empty(M, device=self.device, dtype=torch.float32)
+        self._conv(FWD_OUT, self.layers[-1], h16, shape, out32=out)
         if keep:
+            saved["blocks"] = blocks
+            saved["hlast"] = h16
+            saved["hlast32"] = h
             self._saved = saved
             self._out = out
             self.last_activations = saved
-        return (out[:, 0] * OUT_SCALE).view(B, H, W)
+        return (out * OUT_SCALE).view(B, H, W)
 
     def train_step(self, vel_km, grad, band, target_km, lr: float = 1e-3, splits: int = 64) -> float:
         """One Adam step on the mean squared error between the proposed update and `target_km`
@@ -232,26 +225,33 @@ class UpdateNet:
 
         self.forward(vel_km, grad, band, keep=True)
         s = self._saved
-        B, H, W = s["shape"]
+        shape = s["shape"]
+        B, H, W = shape
         M = B * H * W
-        out = self._out
-        dout = torch.zeros((M, CH), device=self.device, dtype=torch.float32)
+        dout = torch.empty(M, device=self.device, dtype=torch.float32)
         loss = torch.zeros(1, device=self.device, dtype=torch.float64)
-        check(self._lib.wg_pc_mse(_p(out), CH, _p(target_km.contiguous()), OUT_SCALE, M, _p(loss), _p(dout),
+        check(self._lib.wg_pc_mse(_p(self._out), 1, _p(target_km.contiguous()), OUT_SCALE, M, _p(loss), _p(dout),
                                   _stream()), "mse")
         parts = {}
+        Lo = self.layers[-1]
         dh = torch.empty((M, CH), device=self.device, dtype=torch.float32)
-        parts["out"] = self._backward_conv(self.layers[-1], s["hlast"], dout, B, H, W, splits, True, dh, 0)
-        tmp = torch.empty((M, CH), device=self.device, dtype=torch.float32)
+        dh16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
+        dout16 = torch.zeros((M, CH), device=self.device, dtype=torch.bfloat16)
+        check(self._lib.wg_pc_out_dgrad(_p(dout), _p(Lo.wt), B, H, W, _p(dh), _p(dh16), _p(dout16), _stream()), "out dgrad")
+        parts["out"] = self._wgrad(Lo, s["hlast"], dout16, shape, splits)
+        t16 = dout16  # read for the last time above
         for i in reversed(range(len(DILATIONS))):
             La, Lb = self.layers[1 + 2 * i], self.layers[2 + 2 * i]
             h16, a16, _ = s["blocks"][i]
-            da = torch.empty((M, CH), device=self.device, dtype=torch.float32)
-            parts[Lb.name] = self._backward_conv(Lb, a16, dh, B, H, W, splits, True, da, 0)
-            check(self._lib.wg_pc_relu_grad(_p(da), _p(a16), M * CH, _p(tmp), _stream()))
-            parts[La.name] = self._backward_conv(La, h16, tmp, B, H, W, splits, True, dh, 1)
-        check(self._lib.wg_pc_relu_grad(_p(dh), _p(s["h0"]), M * CH, _p(tmp), _stream()))
-        parts["in"] = self._backward_conv(self.layers[0], s["x0"], tmp, B, H, W, splits, False)
+            parts[Lb.name] = self._wgrad(Lb, a16, dh16, shape, splits)
+            self._conv(DGRAD_MASK, Lb, dh16, shape, out16=t16, mask=a16)
+            parts[La.name] = self._wgrad(La, h16, t16, shape, splits)
+            if i:
+                self._conv(DGRAD_ADD, La, t16, shape, out16=dh16, out32=dh, add=dh)
+            else:
+                self._conv(DGRAD_ADD_MASK, La, t16, shape, out16=dh16, add=dh, mask=s["h0"])
+        Li = self.layers[0]
+        parts["in"] = self._wgrad(Li, s["col0"], dh16, shape, splits, columns=Li.kp)
         self.step += 1
         for L in self.layers:
             p = parts[L.name]
