@@ -171,6 +171,70 @@ __device__ __forceinline__ void st_peer_v2(const float* local_ptr, unsigned peer
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(a), "f"(b));
 }
 
+// Halo exchange of the forward kernels that store gradient terms.
+//
+// The two boundary rows of a CTA go to the neighbouring CTA's halo rows as asynchronous DSMEM stores
+// that complete on an mbarrier of the receiver, and only the warps whose rows read a halo wait for
+// it, at the start of the next step. The other kernels send them with plain DSMEM stores, a
+// cluster-scope fence in the sending warps and a cluster barrier per step. With stored terms in
+// flight that fence also waits for them to reach L2, and the whole cluster waits for the fence:
+// without it the storing pass over 320 units x 100 steps takes 1.33 against 1.50 ms on the 70 x 70
+// grid, and 8 % less on the 100 x 100 and 140 x 140 grids. Where nothing is stored the barrier is the
+// cheaper one (1.49 against 1.54 ms; 12 % on the 100 x 100 grid), and the adjoint hides its loads
+// between the barrier's arrive and wait (4.84 against 5.16 ms), so those keep it.
+//
+// Buffers and mbarriers alternate: what a step writes into buffer q = 0 / 1 arrives on mbarrier q.
+// A CTA cannot be two exchanges ahead of a neighbour (its next step's halo waits for all of the
+// neighbour's rows), so at most one phase of each mbarrier is in flight; and a row is sent after
+// its own stencil reads, so once all of a neighbour's rows have arrived it has read its halo of the
+// other buffer, which may be overwritten.
+struct HaloLink {
+  unsigned bar;    // shared-memory address of this CTA's two mbarriers
+  unsigned bytes;  // bytes per exchange this CTA receives
+  bool dead;       // a wait ran out: record it and stop waiting
+
+  __device__ __forceinline__ void init(float* smem_bar, unsigned n, int tid) {
+    bar = static_cast<unsigned>(__cvta_generic_to_shared(smem_bar));
+    bytes = n;
+    dead = false;
+    if (tid == 0) {
+      for (int q = 0; q < 2; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * q) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+  }
+  // One thread, once per exchange, before this CTA can be sent the next one.
+  __device__ __forceinline__ void expect(int q) const {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * q), "r"(bytes) : "memory");
+  }
+  // Bounded wait for the exchange into buffer q; `use`: how many exchanges into q came before it.
+  __device__ __forceinline__ void wait(int q, int use, int* status) {
+    if (dead) return;
+    const unsigned a = bar + 8 * q, parity = use & 1;
+    for (int i = 0; i < (1 << 20); ++i) {
+      unsigned ok;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok)
+          : "r"(a), "r"(parity)
+          : "memory");
+      if (ok) return;
+    }
+    dead = true;
+    if (status) atomicCAS(status, 0, static_cast<int>(ST_CUDA));
+  }
+  // A pair of values into the peer CTA's copy of `local_ptr`, arriving on the peer's mbarrier q.
+  __device__ __forceinline__ void send(const float* local_ptr, unsigned peer, int q, float x, float y) const {
+    const unsigned la = static_cast<unsigned>(__cvta_generic_to_shared(local_ptr));
+    unsigned ra, rb;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(peer));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar + 8 * q), "r"(peer));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(ra), "f"(x),
+                 "f"(y), "r"(rb));
+  }
+};
+
 // ------------------------------------------------------------------------------------------------
 // Forward (splatForward.wgsl:48-121)
 // ------------------------------------------------------------------------------------------------
@@ -183,6 +247,7 @@ enum : int { LAY_RUNTIME = 0, LAY_EVEN = 1, LAY_SQUARE = 2 };
 template <int NX, int PMLP, int C, int S, int NSEG, int NI, int LAY, bool TRACES, bool STORE, bool FA = false>
 __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __grid_constant__ FwdArgs p) {
   using CL = Cols3<NX, PMLP>;
+  constexpr bool LINK = C > 1 && STORE;  // halos by HaloLink; otherwise a cluster barrier per step
   constexpr int SW = CL::SW;
   constexpr int NT = NSEG * 32 * (1 + NI);
   extern __shared__ __align__(16) float sm[];
@@ -239,7 +304,10 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   const int zb = r0 + seg * S;
   const int ltid = light_tid<NSEG, NI, C>(tid, rank);
   const int nrows = CL::active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
-  const bool pusher = (C > 1) && nrows > 0 && ((rank > 0 && zb < r0 + FD_PAD) || (rank < C - 1 && zb + nrows > r1 - FD_PAD));
+  // warps with rows that read a halo (and are sent to the neighbour)
+  const bool edge = (C > 1) && ((rank > 0 && zb < r0 + FD_PAD) || (rank < C - 1 && zb + S > r1 - FD_PAD));
+  HaloLink link;
+  if constexpr (LINK) link.init(sm + L.off_bar, ((rank > 0) + (rank < C - 1)) * FD_PAD * (NX - 2 * FD_PAD) * 4, tid);
   const int ubase = (zb - zl0) * NX + x;                 // row 0 of the segment in U
   const int abase = (zb - r0) * 2 * SW + CL::strip(x);   // row 0 in APX / ZX (PML warp)
   const int zsh = (zb < nz / 2) ? 0 : (nz - sw - bot_off);
@@ -341,6 +409,11 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 
   auto step = [&](int t, float2 (&uc)[S], float2 (&un)[S]) {
     const int par = (t - p.t0) & 1;
+    const bool last = t + 1 == p.t1;
+    if constexpr (LINK) {
+      if (tid == 0 && !last) link.expect(1 - par);
+      if (edge && t > p.t0) link.wait(par, (t - p.t0 - 1) >> 1, p.status);
+    }
     const float* Uc = U + par * ustride + ubase;
     float* Un = U + (1 - par) * ustride + ubase;
     const float* APXc = APX + par * xstride + abase;
@@ -520,9 +593,15 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
           un[i] = make_float2(n0, n1);
           sts2(uw + i * NX, n0, n1);
           if constexpr (C > 1) {
-            if (rank > 0 && z < r0 + FD_PAD) st_peer_v2(U + (1 - par) * ustride + (z - pr_lo) * NX + x, rank - 1, n0, n1);
-            if (rank < C - 1 && z >= r1 - FD_PAD)
-              st_peer_v2(U + (1 - par) * ustride + (z - (r1 - FD_PAD)) * NX + x, rank + 1, n0, n1);
+            float* up = U + (1 - par) * ustride + (z - pr_lo) * NX + x;
+            float* dn = U + (1 - par) * ustride + (z - (r1 - FD_PAD)) * NX + x;
+            if constexpr (LINK) {
+              if (rank > 0 && z < r0 + FD_PAD && !last) link.send(up, rank - 1, 1 - par, n0, n1);
+              if (rank < C - 1 && z >= r1 - FD_PAD && !last) link.send(dn, rank + 1, 1 - par, n0, n1);
+            } else {
+              if (rank > 0 && z < r0 + FD_PAD) st_peer_v2(up, rank - 1, n0, n1);
+              if (rank < C - 1 && z >= r1 - FD_PAD) st_peer_v2(dn, rank + 1, n0, n1);
+            }
           }
         }
       }
@@ -530,7 +609,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
     rows(Un, APXn, ZXo, APZn, ZZo, st);
     if (TRACES) {
       // receivers at time t, recorded after this thread's update by the threads with the least
-      // work per step: nothing writes buffer `par` before this step's barrier
+      // work per step: nothing writes this CTA's rows of buffer `par` before this step's barrier
+      // (the receivers, one cell below the C-PML's rows, lie inside the first CTA's)
       const float* Ucb = U + par * ustride;
       for (int r = ltid; r < nrec; r += NT) {
         if (sRecOk[r]) {
@@ -546,13 +626,14 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
       const int u = t - p.t0;
       if (u >= H && u % H == 0) wavelet_ring_fill(sW, g.wavelet, u + H, u + 2 * H, wsteps, ltid, H, wtime);
     }
-    if constexpr (C > 1) {
-      if (pusher) fence_cluster();
+    if constexpr (C > 1 && !LINK) {
+      if (edge) fence_cluster();
       __syncthreads();
       cluster_arrive_relaxed();
+      cluster_wait_acquire();
+    } else {
+      __syncthreads();
     }
-    if constexpr (C > 1) cluster_wait_acquire();
-    else __syncthreads();
   };
 
   int t = p.t0;
@@ -561,6 +642,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
     step(t + 1, uB, uA);
   }
   if (t < p.t1) step(t, uA, uB);
+  if constexpr (LINK) cluster_barrier();  // no CTA leaves while a neighbour may still store to it
 }
 
 // ------------------------------------------------------------------------------------------------

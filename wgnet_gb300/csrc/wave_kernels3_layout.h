@@ -15,7 +15,7 @@ constexpr int G3_WAV_STEPS = 128;
 
 struct F3Layout {
   int maxrows, lr, zs;
-  int off_u, off_apx, off_zx, off_apz, off_zz, off_v2, off_c2, off_prof, off_rec, off_src, total;
+  int off_u, off_apx, off_zx, off_apz, off_zz, off_v2, off_c2, off_prof, off_rec, off_src, off_bar, total;
 };
 
 __host__ __device__ inline F3Layout f3_layout_rt(int NX, int pmlp, int nz, int sw, int C, int nrec) {
@@ -34,7 +34,8 @@ __host__ __device__ inline F3Layout f3_layout_rt(int NX, int pmlp, int nz, int s
   L.off_prof = L.off_c2 + L.maxrows * NX;
   L.off_rec = L.off_prof + 3 * (NX + nz);
   L.off_src = (L.off_rec + 9 * nrec + 3) & ~3;  // source corners: 4 cells (int), 4 factors, wavelet ring
-  L.total = L.off_src + 8 + G3_WAV_STEPS;
+  L.off_bar = L.off_src + 8 + G3_WAV_STEPS;  // two mbarriers (halo rows arrived), 8-byte aligned
+  L.total = L.off_bar + 4;
   return L;
 }
 
