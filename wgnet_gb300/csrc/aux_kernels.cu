@@ -12,8 +12,6 @@ namespace wg {
 
 namespace {
 
-constexpr int kRedThreads = 512;
-
 // Block-wide f64 sum with a fixed tree (deterministic for a fixed blockDim).
 __device__ double block_sum(double v, double* sh) {
   const int tid = threadIdx.x;
@@ -44,17 +42,41 @@ __global__ void pad_kernel(const float* __restrict__ vis, int nx_vis, int nz_vis
   }
 }
 
-__global__ void energy_kernel(const float* __restrict__ obs, size_t per_model, double* __restrict__ energy,
-                              float* __restrict__ scale, int* __restrict__ status) {
+// The two f64 reductions over a model's traces. FP64 issues at 2 lanes per clock and SM, which bounds
+// them, so a model's traces are split over up to kRedParts blocks (one block per model took 0.77 ms
+// for 5 shots x 2001 x 70 and left the other SMs idle), and the square is one fused f64 operation
+// (the product of two f32 is exact in f64, so nothing else rounds). A second launch adds a model's
+// partial sums in a fixed order.
+constexpr int kRedThreads = 256;
+constexpr size_t kRedChunk = 8192;  // least values per block
+
+inline int red_parts(size_t per_model) {
+  return static_cast<int>(std::min<size_t>(kRedParts, (per_model + kRedChunk - 1) / kRedChunk));
+}
+
+__global__ void __launch_bounds__(kRedThreads) energy_kernel(const float* __restrict__ obs, size_t per_model,
+                                                             double* __restrict__ part) {
   __shared__ double sh[32];
-  const int model = blockIdx.x;
+  const int model = blockIdx.y, parts = gridDim.x;
+  const size_t chunk = (per_model + parts - 1) / parts;
+  const size_t i0 = blockIdx.x * chunk, i1 = i0 + chunk < per_model ? i0 + chunk : per_model;
   const float* o = obs + static_cast<size_t>(model) * per_model;
   double acc = 0.0;
-  for (size_t i = threadIdx.x; i < per_model; i += blockDim.x) {
+#pragma unroll 4
+  for (size_t i = i0 + threadIdx.x; i < i1; i += kRedThreads) {
     const double d = static_cast<double>(o[i]);
-    acc += d * d;
+    acc = __fma_rn(d, d, acc);
   }
   const double e = block_sum(acc, sh);
+  if (threadIdx.x == 0) part[static_cast<size_t>(model) * kRedParts + blockIdx.x] = e;
+}
+
+__global__ void __launch_bounds__(kRedThreads) energy_final_kernel(const double* __restrict__ part, int parts,
+                                                                   double* __restrict__ energy, float* __restrict__ scale,
+                                                                   int* __restrict__ status) {
+  __shared__ double sh[32];
+  const int model = blockIdx.x;
+  const double e = block_sum(threadIdx.x < parts ? part[static_cast<size_t>(model) * kRedParts + threadIdx.x] : 0.0, sh);
   if (threadIdx.x == 0) {
     energy[model] = e;
     scale[model] = static_cast<float>(1.0 / e);
@@ -63,46 +85,97 @@ __global__ void energy_kernel(const float* __restrict__ obs, size_t per_model, d
 }
 
 // wave_wgpu.rs:13-54: d = p - obs; r = d * scale; e = 0.5 * d * d * scale (f32), summed in f64.
-__global__ void residual_kernel(const float* pred, const float* __restrict__ obs, const float* __restrict__ scale,
-                                size_t per_model, float* res, double* __restrict__ loss) {
+__global__ void __launch_bounds__(kRedThreads) residual_kernel(const float* pred, const float* __restrict__ obs,
+                                                               const float* __restrict__ scale, size_t per_model, float* res,
+                                                               double* __restrict__ part) {
   __shared__ double sh[32];
-  const int model = blockIdx.x;
+  const int model = blockIdx.y, parts = gridDim.x;
+  const size_t chunk = (per_model + parts - 1) / parts;
   const size_t base = static_cast<size_t>(model) * per_model;
+  const size_t i0 = base + blockIdx.x * chunk, end = base + per_model, i1 = i0 + chunk < end ? i0 + chunk : end;
   const float sc = scale[model];
   double acc = 0.0;
-  for (size_t i = threadIdx.x; i < per_model; i += blockDim.x) {
-    const float d = pred[base + i] - obs[base + i];
-    res[base + i] = d * sc;
-    acc += static_cast<double>(((0.5f * d) * d) * sc);
+  // batches of four: pred and res may be one array, so the loads are issued ahead of the stores by hand
+  for (size_t i = i0 + threadIdx.x; i < i1; i += 4 * kRedThreads) {
+    float d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const size_t k = i + q * kRedThreads;
+      d[q] = k < i1 ? pred[k] - obs[k] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const size_t k = i + q * kRedThreads;
+      if (k < i1) {
+        res[k] = d[q] * sc;
+        acc += static_cast<double>(((0.5f * d[q]) * d[q]) * sc);
+      }
+    }
   }
   const double e = block_sum(acc, sh);
+  if (threadIdx.x == 0) part[static_cast<size_t>(model) * kRedParts + blockIdx.x] = e;
+}
+
+__global__ void __launch_bounds__(kRedThreads) loss_final_kernel(const double* __restrict__ part, int parts,
+                                                                 double* __restrict__ loss) {
+  __shared__ double sh[32];
+  const int model = blockIdx.x;
+  const double e = block_sum(threadIdx.x < parts ? part[static_cast<size_t>(model) * kRedParts + threadIdx.x] : 0.0, sh);
   if (threadIdx.x == 0) loss[model] = e;
 }
 
-// wave_wgpu.rs:974-1005. One thread per visible node; the padded cells that fold onto it are
-// visited row-major (the reference's accumulation order), summed in f64.
-__global__ void fold_kernel(const float* __restrict__ gacc, const float* __restrict__ mask, int shots, int nx,
-                            int nz, int pad, int nx_vis, int nz_vis, float* __restrict__ grad) {
+// wave_wgpu.rs:974-1005: the padded cells that fold onto a visible node, row-major (the reference's
+// accumulation order), summed in f64. A node inside the grid has one cell and one thread; a node on
+// the border has pad + 1 cells, a corner (pad + 1)^2, and gets a warp: the lanes load and shot-sum 32
+// cells at a time, then the f64 sum runs over them in order. (A corner's 529 cells x 5 shots in one
+// thread took 0.18 ms, all of it load latency.)
+constexpr int kFoldThreads = 256;
+
+__global__ void __launch_bounds__(kFoldThreads) fold_kernel(const float* __restrict__ gacc, const float* __restrict__ mask,
+                                                            int shots, int nx, int nz, int pad, int nx_vis, int nz_vis,
+                                                            int inner_blocks, float* __restrict__ grad) {
   const int model = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nx_vis * nz_vis) return;
-  const int vz = i / nx_vis, vx = i % nx_vis;
   const size_t cells = static_cast<size_t>(nx) * nz;
-  const int z_lo = (vz == 0) ? 0 : vz + pad;
-  const int z_hi = (vz == nz_vis - 1) ? nz : vz + pad + 1;
-  const int x_lo = (vx == 0) ? 0 : vx + pad;
-  const int x_hi = (vx == nx_vis - 1) ? nx : vx + pad + 1;
   const float* gm = gacc + static_cast<size_t>(model) * shots * cells;
   const float* mk = mask + static_cast<size_t>(model) * cells;
-  double acc = 0.0;
-  for (int z = z_lo; z < z_hi; ++z)
-    for (int x = x_lo; x < x_hi; ++x) {
-      const size_t c = static_cast<size_t>(z) * nx + x;
-      float s = 0.0f;
-      for (int k = 0; k < shots; ++k) s = s + gm[k * cells + c];
-      acc += static_cast<double>(s * mk[c]);
-    }
-  grad[static_cast<size_t>(model) * nx_vis * nz_vis + i] = static_cast<float>(acc);
+  float* out = grad + static_cast<size_t>(model) * nx_vis * nz_vis;
+  auto cell_value = [&](size_t c) {
+    float s = 0.0f;
+    for (int k = 0; k < shots; ++k) s = s + gm[k * cells + c];
+    return static_cast<double>(s * mk[c]);
+  };
+  if (static_cast<int>(blockIdx.x) < inner_blocks) {
+    const int i = blockIdx.x * kFoldThreads + threadIdx.x;
+    if (i >= nx_vis * nz_vis) return;
+    const int vz = i / nx_vis, vx = i % nx_vis;
+    if (vz == 0 || vz == nz_vis - 1 || vx == 0 || vx == nx_vis - 1) return;
+    out[i] = static_cast<float>(0.0 + cell_value(static_cast<size_t>(vz + pad) * nx + vx + pad));
+    return;
+  }
+  // border node b: the top row, the bottom row, then the two ends of each row in between
+  const int lane = threadIdx.x & 31;
+  const int b = (blockIdx.x - inner_blocks) * (kFoldThreads / 32) + (threadIdx.x >> 5);
+  if (b >= 2 * nx_vis + 2 * (nz_vis - 2)) return;
+  int vz, vx;
+  if (b < 2 * nx_vis) {
+    vz = b < nx_vis ? 0 : nz_vis - 1;
+    vx = b % nx_vis;
+  } else {
+    vz = 1 + (b - 2 * nx_vis) / 2;
+    vx = (b & 1) == 0 ? 0 : nx_vis - 1;
+  }
+  const int z_lo = (vz == 0) ? 0 : vz + pad, z_hi = (vz == nz_vis - 1) ? nz : vz + pad + 1;
+  const int x_lo = (vx == 0) ? 0 : vx + pad, x_hi = (vx == nx_vis - 1) ? nx : vx + pad + 1;
+  const int w = x_hi - x_lo, n = (z_hi - z_lo) * w;
+  auto load = [&](int i) { return i < n ? cell_value(static_cast<size_t>(z_lo + i / w) * nx + x_lo + i % w) : 0.0; };
+  double acc = 0.0, v = load(lane);
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const double next = load(i0 + 32 + lane);
+    const int m = n - i0 < 32 ? n - i0 : 32;
+    for (int l = 0; l < m; ++l) acc += __shfl_sync(0xffffffffu, v, l);
+    v = next;
+  }
+  if (lane == 0) out[vz * nx_vis + vx] = static_cast<float>(acc);
 }
 
 // Causal FIR along time of [series][nt][nrec] traces: out[t] = sum over k, in order, of ker[k]
@@ -204,21 +277,29 @@ cudaError_t launch_pad_velocity(const float* vis, int models, int nx_vis, int nz
 }
 
 cudaError_t launch_energy(const float* observed, int models, size_t per_model, double* energy, float* scale,
-                          int* status, cudaStream_t s) {
-  energy_kernel<<<models, kRedThreads, 0, s>>>(observed, per_model, energy, scale, status);
+                          int* status, double* scratch, cudaStream_t s) {
+  const int parts = red_parts(per_model);
+  energy_kernel<<<dim3(parts, models), kRedThreads, 0, s>>>(observed, per_model, scratch);
+  energy_final_kernel<<<models, kRedThreads, 0, s>>>(scratch, parts, energy, scale, status);
+  note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_residual(const float* pred, const float* observed, const float* scale, int models,
-                            size_t per_model, float* residual, double* loss, cudaStream_t s) {
-  residual_kernel<<<models, kRedThreads, 0, s>>>(pred, observed, scale, per_model, residual, loss);
+                            size_t per_model, float* residual, double* loss, double* scratch, cudaStream_t s) {
+  const int parts = red_parts(per_model);
+  residual_kernel<<<dim3(parts, models), kRedThreads, 0, s>>>(pred, observed, scale, per_model, residual, scratch);
+  loss_final_kernel<<<models, kRedThreads, 0, s>>>(scratch, parts, loss);
+  note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_fold(const float* gacc, const float* mask, int models, int shots, int nx, int nz, int pad,
                         int nx_vis, int nz_vis, float* grad, cudaStream_t s) {
-  dim3 grid((nx_vis * nz_vis + 255) / 256, models);
-  fold_kernel<<<grid, 256, 0, s>>>(gacc, mask, shots, nx, nz, pad, nx_vis, nz_vis, grad);
+  const int inner = (nx_vis * nz_vis + kFoldThreads - 1) / kFoldThreads;
+  const int border = 2 * nx_vis + 2 * (nz_vis - 2), warps = kFoldThreads / 32;
+  const dim3 grid(inner + (border + warps - 1) / warps, models);
+  fold_kernel<<<grid, kFoldThreads, 0, s>>>(gacc, mask, shots, nx, nz, pad, nx_vis, nz_vis, inner, grad);
   return cudaGetLastError();
 }
 

@@ -560,6 +560,8 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
   WG_TRY(e->w_scale.ensure(M * 4));
   if (slots > 0) WG_TRY(e->w_ckpt.ensure(M * S * slots * ckf * 4));
   WG_TRY(e->w_stored.ensure(M * S * seg * cells * 4));
+  // adjoint state; until the first adjoint pass it is scratch of the misfit's reductions (kRedParts
+  // doubles per model: an adjoint state is at least 4 KB even without a C-PML)
   WG_TRY(e->w_adj.ensure(M * S * asf * 4));
   WG_TRY(e->w_gacc.ensure(M * S * cells * 4));
   for (int m0 = 0; m0 < models; m0 += M) {
@@ -603,9 +605,9 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
     }
     if (obs_ready && m0 == 0) WG_CK(cudaStreamWaitEvent(st, obs_ready, 0));
     WG_LAUNCH(wg::launch_energy(obs, mc, S * tr, e->w_energy.as<double>(), e->w_scale.as<float>(),
-                                e->d_status.as<int>(), st));
+                                e->d_status.as<int>(), e->w_adj.as<double>(), st));
     WG_LAUNCH(wg::launch_residual(e->w_traces.as<float>(), obs, e->w_scale.as<float>(), mc, S * tr,
-                                  e->w_traces.as<float>(), d_loss + m0, st));
+                                  e->w_traces.as<float>(), d_loss + m0, e->w_adj.as<double>(), st));
     WG_CK(cudaMemsetAsync(e->w_gacc.p, 0, static_cast<size_t>(units) * cells * 4, st));
     wg::AdjArgs a{};
     a.g = e->grid();

@@ -165,7 +165,8 @@ extern "C" int wg_evaluate_adjoint_noalloc(wg_engine* eng, const float* d_vel_mp
     if (e != cudaSuccess) return wg::report_error(WG_ERR_CUDA, cudaGetErrorString(e));
   }
   NA_LAUNCH(wg::launch_pad_velocity(d_vel_mps, models, v.nx_vis, v.nz_vis, v.pad, v.vmin, v.vmax, vpad, mask, st));
-  NA_LAUNCH(wg::launch_energy(d_observed, models, per_model, energy, scale, v.d_status, st));
+  NA_LAUNCH(wg::launch_energy(d_observed, models, per_model, energy, scale, v.d_status,
+                              reinterpret_cast<double*>(adj), st));
   wg::FwdArgs f{};
   f.g = v.grid;
   f.st = v.stations;
@@ -198,7 +199,8 @@ extern "C" int wg_evaluate_adjoint_noalloc(wg_engine* eng, const float* d_vel_mp
     l.stored = stored;
     NA_LAUNCH(wg::launch_fwd(v.fshape, true, true, l, st));
   }
-  NA_LAUNCH(wg::launch_residual(traces, d_observed, scale, models, per_model, traces, d_loss, st));
+  NA_LAUNCH(wg::launch_residual(traces, d_observed, scale, models, per_model, traces, d_loss,
+                                reinterpret_cast<double*>(adj), st));
   // The accumulator's frame cells are never written by the kernels; the array keeps the previous
   // call's contents, so clear it.
   {

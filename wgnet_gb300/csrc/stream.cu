@@ -1070,7 +1070,7 @@ int wait_timeout_selftest(int* d_status, long long polls, cudaStream_t st) {
 }
 
 struct StreamWork {
-  Buf vpad, mask, traces, energy, scale, stored, ckpt, gacc;
+  Buf vpad, mask, traces, energy, scale, part, stored, ckpt, gacc;
   Buf W, PX, ZX, PZ, ZZ;        // forward state
   Buf Wtb, PXtb, ZXtb, PZtb, ZZtb;  // temporally blocked forward: two state sets
   Buf L, LPX, LZX, LPZ, LZZ;    // adjoint state
@@ -1363,11 +1363,13 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   SW_CK(w->traces.ensure(units * tr * 4));
   SW_CK(w->energy.ensure(models * 8));
   SW_CK(w->scale.ensure(models * 4));
+  SW_CK(w->part.ensure(static_cast<size_t>(models) * kRedParts * 8));
   SW_CK(w->gacc.ensure(units * cells * 4));
   note_launch();
   SW_CK(launch_pad_velocity(d_vis, models, v.nx_vis, v.nz_vis, v.pad, v.vmin, v.vmax, w->vpad.f(), w->mask.f(), st));
   note_launch();
-  SW_CK(launch_energy(d_obs, models, v.shots * tr, static_cast<double*>(w->energy.p), w->scale.f(), v.d_status, st));
+  SW_CK(launch_energy(d_obs, models, v.shots * tr, static_cast<double*>(w->energy.p), w->scale.f(), v.d_status,
+                      static_cast<double*>(w->part.p), st));
   if ((rc = alloc_forward(w, v, units, st)) != WG_OK) return rc;
 
   // Segment length: store every step's gradient terms when they fit in 70% of the free memory,
@@ -1432,7 +1434,8 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   }
   timer.mark(0, false, st);
   note_launch();
-  SW_CK(launch_residual(w->traces.f(), d_obs, w->scale.f(), models, v.shots * tr, w->traces.f(), d_loss, st));
+  SW_CK(launch_residual(w->traces.f(), d_obs, w->scale.f(), models, v.shots * tr, w->traces.f(), d_loss,
+                        static_cast<double*>(w->part.p), st));
 
   // adjoint state
   const size_t xsf = xs_floats(v), zsf = zs_floats(v);

@@ -46,14 +46,17 @@ cudaError_t launch_adj(const Shape& s, const AdjArgs& a, cudaStream_t stream);
 cudaError_t launch_pad_velocity(const float* vis, int models, int nx_vis, int nz_vis, int pad, float vmin, float vmax,
                                 float* padded, float* mask, cudaStream_t s);
 
+// Partial sums per model of the two reductions below, and the scratch they need: models * kRedParts doubles.
+constexpr int kRedParts = 256;
+
 // Per-model observed energy sum d^2 in f64 and scale = f32(1 / energy); status on energy <= 0.
 cudaError_t launch_energy(const float* observed, int models, size_t per_model, double* energy, float* scale,
-                          int* status, cudaStream_t s);
+                          int* status, double* scratch, cudaStream_t s);
 
 // residual[i] = (pred[i] - obs[i]) * scale[model]; loss[model] = sum 0.5 (p-d)^2 scale (f64).
 // pred and residual may alias.
 cudaError_t launch_residual(const float* pred, const float* observed, const float* scale, int models,
-                            size_t per_model, float* residual, double* loss, cudaStream_t s);
+                            size_t per_model, float* residual, double* loss, double* scratch, cudaStream_t s);
 
 // grad[m][vz][vx] = sum over padded cells folding onto (vz, vx) of
 //   (sum_s gacc[m][s][cell]) * mask[m][cell]       (f32 shot-sum, f64 fold), wave_wgpu.rs:974-1005.
