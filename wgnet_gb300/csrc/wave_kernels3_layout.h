@@ -69,7 +69,8 @@ __host__ __device__ inline A3Layout a3_layout_rt(int NX, int pmlp, int nz, int s
   L.off_v2 = L.off_lzz + sz;              // V2[maxrows][NX]     v^2 dt^2 (owner only)
   L.off_ga = L.off_v2 + L.maxrows * NX;   // GA[maxrows][NX]     gradient accumulator (owner only)
   L.off_prof = L.off_ga + L.maxrows * NX; // ax bx dbx az bz dbz
-  L.off_opb = L.off_prof + 3 * (NX + nz); // 1 + bx, per column
+  // 1 + bx, per column, read in pairs: on an even offset whatever nz is
+  L.off_opb = (L.off_prof + 3 * (NX + nz) + 1) & ~1;
   L.off_src = (L.off_opb + NX + 3) & ~3;  // source corners: 4 cells (int), 4 factors, then the
                                           // wavelet samples of the launch's steps
   L.rcap = (nrec + 3) & ~3;
