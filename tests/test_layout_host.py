@@ -9,6 +9,7 @@ from conftest import ROOT
 
 SOURCE = r"""
 #include <cstddef>
+#include <initializer_list>
 #define __host__
 #define __device__
 #define __forceinline__ inline
