@@ -297,39 +297,47 @@ int set_receivers_impl(wg_engine* e) {
   return WG_OK;
 }
 
-// Compiled shape with this (cluster, threads, cells-per-thread) triple.
-bool find_shape(int which, int cluster, int threads, int cpt, wg::Shape* out) {
+bool shape_fits(const wg_engine* e, int which, const wg::Shape& s) {
+  return which == 0 ? wg::fwd_shape_fits(s, e->nx, e->nz, e->sw, e->nrec) : wg::adj_shape_fits(s, e->nx, e->nz, e->swa, e->nrec);
+}
+
+// Compiled shape with this (cluster, threads, cells-per-thread) triple: 0 none, 1 one that does not fit
+// the engine's grid, 2 one that does (several shapes, of different grid widths, may share a triple).
+int find_shape(const wg_engine* e, int which, int cluster, int threads, int cpt, wg::Shape* out) {
   const int n = which == 0 ? wg::fwd_shape_count() : wg::adj_shape_count();
+  int found = 0;
   for (int i = 0; i < n; ++i) {
     const wg::Shape k = which == 0 ? wg::fwd_shape(i) : wg::adj_shape(i);
-    if (k.cluster == cluster && k.threads == threads && k.cpt == cpt) {
+    if (k.cluster != cluster || k.threads != threads || k.cpt != cpt) continue;
+    found = 1;
+    if (shape_fits(e, which, k)) {
       *out = k;
-      return true;
+      return 2;
     }
   }
-  return false;
+  return found;
 }
 
 bool pick_shapes(wg_engine* e) {
   // Preference order; the first compiled shape that fits the grid is the default (the autotuner
   // can choose another among wg_shape_candidates).
-  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 896, 4}, {4, 448, 8}, {1, 1024, 12},
+  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 896, 4}, {4, 448, 8}, {4, 448, 10}, {1, 1024, 12},
                                  {2, 1024, 6}, {2, 512, 12}, {2, 1024, 10}, {4, 1024, 8}, {2, 1024, 16},
                                  {4, 512, 16}};
-  static const int apref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {2, 1024, 6}, {4, 896, 4}, {4, 448, 8},
+  static const int apref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 448, 10}, {2, 1024, 6}, {4, 896, 4}, {4, 448, 8},
                                  {2, 512, 12}, {4, 1024, 4}, {4, 1024, 8}, {4, 512, 16}};
   e->fshape = wg::Shape{0, 0, 0};
   e->ashape = wg::Shape{0, 0, 0};
   for (const auto& t : fpref) {
     wg::Shape s;
-    if (find_shape(0, t[0], t[1], t[2], &s) && wg::fwd_shape_fits(s, e->nx, e->nz, e->sw, e->nrec)) {
+    if (find_shape(e, 0, t[0], t[1], t[2], &s) == 2) {
       e->fshape = s;
       break;
     }
   }
   for (const auto& t : apref) {
     wg::Shape s;
-    if (find_shape(1, t[0], t[1], t[2], &s) && wg::adj_shape_fits(s, e->nx, e->nz, e->swa, e->nrec)) {
+    if (find_shape(e, 1, t[0], t[1], t[2], &s) == 2) {
       e->ashape = s;
       break;
     }
@@ -928,16 +936,12 @@ int wg_get_option(const wg_engine* e, const char* key, int* value) {
 int wg_set_launch_shape(wg_engine* e, int which, int cluster, int threads, int cpt) {
   if (!e) return fail(WG_ERR_ARG, "null engine");
   if (which != 0 && which != 1) return fail(WG_ERR_ARG, "which must be 0 (forward) or 1 (adjoint)");
-  wg::Shape s;
-  if (!find_shape(which, cluster, threads, cpt, &s)) return fail(WG_ERR_ARG, "launch shape not compiled");
   std::lock_guard<std::mutex> lk(e->mu);
-  if (which == 0) {
-    if (!wg::fwd_shape_fits(s, e->nx, e->nz, e->sw, e->nrec)) return fail(WG_ERR_ARG, "forward shape does not fit this grid");
-    e->fshape = s;
-  } else {
-    if (!wg::adj_shape_fits(s, e->nx, e->nz, e->swa, e->nrec)) return fail(WG_ERR_ARG, "adjoint shape does not fit this grid");
-    e->ashape = s;
-  }
+  wg::Shape s;
+  const int found = find_shape(e, which, cluster, threads, cpt, &s);
+  if (found == 0) return fail(WG_ERR_ARG, "launch shape not compiled");
+  if (found == 1) return fail(WG_ERR_ARG, which == 0 ? "forward shape does not fit this grid" : "adjoint shape does not fit this grid");
+  (which == 0 ? e->fshape : e->ashape) = s;
   return WG_OK;
 }
 

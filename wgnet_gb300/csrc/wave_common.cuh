@@ -124,6 +124,7 @@ struct Shape {
   int kind = 1, seg_rows = 0, nseg = 0, ni = 0;
   int nxc = 0, pmlp = 0;  // generation 3: compile-time grid width and PML column pairs per side
   int fast = 0;           // generation 3: fast-arithmetic forward compiled for this shape
+  int rag = 0;            // generation 3: any width up to nxc (row stride nxc in shared memory)
 };
 
 }  // namespace wg

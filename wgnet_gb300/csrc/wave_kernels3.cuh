@@ -29,21 +29,60 @@ namespace wg {
 // PMLP both halves of the row ran into the same banks (the last left pair and the first right pair
 // of a 114-wide row, and the packed strips' left and right columns), replaying a wavefront on
 // every access of the PML warp. Each half-warp now reads one contiguous run of columns.
-template <int NX, int PMLP>
+//
+// RAG: NX is only the row stride of the shared arrays; the grid's width `nx` is any width up to it,
+// odd ones included. The pairs still start at x = 2, so on an odd width the last pair's second
+// column is the grid's frame (`Pairs::half`): its values stay zero and it is left out of global
+// reads and writes. The right strip then starts one pair further in (PMLP + 1 pairs).
+template <int NX, int PMLP, bool RAG = false>
 struct Cols3 {
-  static_assert(PMLP <= 16, "the PML warp holds at most 16 column pairs per side");
-  static constexpr int PCOLS = 2 * PMLP;          // PML columns per side, starting at x = 2
-  static constexpr int SW = PCOLS + 4;            // packed strip width per side (reads reach x+3); = g3_sw
+  static_assert(PMLP + (RAG ? 1 : 0) <= 16, "the PML warp holds at most 16 column pairs per side");
+  static constexpr int PCOLS = 2 * PMLP;              // PML columns per side, starting at x = 2
+  static constexpr int SW = g3_xsw(PMLP, RAG);        // packed strip width per side (reads reach x+3)
   static constexpr int IPAIRS = (NX - 4 - 2 * PCOLS) / 2;
-  __device__ static int x_of(int wk, int lane) {
-    if (wk == 0) return lane < 16 ? FD_PAD + 2 * lane : (NX - FD_PAD - PCOLS) + 2 * (lane - 16);
+  int nx, right, pairs;  // first right pair's index and number of pairs
+  __device__ explicit Cols3(int nx_)
+      : nx(RAG ? nx_ : NX), right((nx - 2 * FD_PAD - PCOLS) / 2), pairs((nx - 2 * FD_PAD + 1) / 2) {}
+  __device__ int x_of(int wk, int lane) const {
+    if (wk == 0) return lane < 16 ? FD_PAD + 2 * lane : FD_PAD + 2 * (right + lane - 16);
     return FD_PAD + PCOLS + 2 * ((wk - 1) * 32 + lane);
   }
-  __device__ static bool active(int wk, int lane) {
-    if (wk == 0) return (lane & 15) < PMLP;
-    return (wk - 1) * 32 + lane < IPAIRS;
+  __device__ bool active(int wk, int lane) const {
+    if (!RAG) return wk == 0 ? (lane & 15) < PMLP : (wk - 1) * 32 + lane < IPAIRS;
+    if (wk == 0) return lane < 16 ? lane < PMLP : right + lane - 16 < pairs;
+    return PMLP + (wk - 1) * 32 + lane < right;
   }
-  __host__ __device__ static int strip(int x) { return x < SW ? x : x - (NX - 2 * SW); }
+  __device__ bool half(int x) const { return RAG && x + 1 >= nx - FD_PAD; }
+  // column of x in the packed x strips: the right strip follows the left one from x = right pair - 2 on
+  __device__ int strip(int x) const { return x < SW ? x : x - (RAG ? FD_PAD + 2 * right - 2 : NX - SW) + SW; }
+};
+
+// A row's column pair in global memory: one 64-bit access on even widths (rows are then 8-byte
+// aligned), two 32-bit ones on odd widths; of a half pair only the first column, the other reads 0.
+template <bool RAG>
+struct PairIo {
+  bool even, half;
+  __device__ __forceinline__ float2 load(const float* p) const {
+    if (!RAG || even) return __ldg(reinterpret_cast<const float2*>(p));
+    return make_float2(__ldg(p), half ? 0.0f : __ldg(p + 1));
+  }
+  __device__ __forceinline__ float2 load_stream(const float* p) const {
+    if (!RAG || even) return __ldcs(reinterpret_cast<const float2*>(p));
+    return make_float2(__ldcs(p), half ? 0.0f : __ldcs(p + 1));
+  }
+  __device__ __forceinline__ void store(float* p, float2 v) const {
+    if (!RAG || even) {
+      *reinterpret_cast<float2*>(p) = v;
+    } else {
+      p[0] = v.x;
+      if (!half) p[1] = v.y;
+    }
+  }
+  // v with the frame column's value set to zero
+  __device__ __forceinline__ float2 mask(float2 v) const {
+    if (RAG && half) v.y = 0.0f;
+    return v;
+  }
 };
 
 // Role of warp `warp` within its segment (0: the PML warp). Warp w issues from scheduler w % 4; with
@@ -240,13 +279,15 @@ struct HaloLink {
 // ------------------------------------------------------------------------------------------------
 // Row layouts (LAY): LAY_RUNTIME, any nz; LAY_EVEN, the rows split evenly into the segments (every
 // segment has exactly S rows); LAY_SQUARE, a square grid (nz = NX), so nz and every shared-memory
-// offset are compile-time constants (and the rows split evenly when C S NSEG = NX - 4).
-enum : int { LAY_RUNTIME = 0, LAY_EVEN = 1, LAY_SQUARE = 2 };
+// offset are compile-time constants (and the rows split evenly when C S NSEG = NX - 4); LAY_RAGGED,
+// any nz and any width up to NX.
+enum : int { LAY_RUNTIME = 0, LAY_EVEN = 1, LAY_SQUARE = 2, LAY_RAGGED = 3 };
 
 // FA: fast arithmetic (see FastCoef); otherwise the reference's operation order, unfused.
 template <int NX, int PMLP, int C, int S, int NSEG, int NI, int LAY, bool TRACES, bool STORE, bool FA = false>
 __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __grid_constant__ FwdArgs p) {
-  using CL = Cols3<NX, PMLP>;
+  constexpr bool RAG = LAY == LAY_RAGGED;
+  using CL = Cols3<NX, PMLP, RAG>;
   constexpr bool LINK = C > 1 && STORE;  // halos by HaloLink; otherwise a cluster barrier per step
   constexpr int SW = CL::SW;
   constexpr int NT = NSEG * 32 * (1 + NI);
@@ -255,8 +296,11 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   constexpr bool SQ = LAY == LAY_SQUARE;
   constexpr bool FULL = LAY == LAY_EVEN || (SQ && NX - 2 * FD_PAD == C * S * NSEG);
   const int nz = SQ ? NX : g.nz;
+  const CL cl(g.nx);
+  const int nx = cl.nx;  // width of the grid and row stride in global memory; NX: row stride in shared memory
   const int sw = g.sw, region = g.region, nrec = p.st.nrec;
   const float rh = g.rh, dt2 = g.dt2, d2a = g.d2a, d2b = g.d2b;
+  static_assert(!(FA && RAG), "no fast arithmetic on ragged widths");
   const FastCoef fc = FastCoef::make(rh);
   const Pk pk{make_float2(g.nz2[0], g.nz2[1])};
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -265,8 +309,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   const int unit = blockIdx.x / C;
   const int shot = unit % p.st.shots;
   const int model = unit / p.st.shots;
-  const size_t cells = static_cast<size_t>(NX) * nz;
-  const F3Layout L = f3_layout_rt(NX, PMLP, nz, sw, C, nrec);
+  const size_t cells = static_cast<size_t>(nx) * nz;
+  const F3Layout L = f3_layout_rt(NX, PMLP, nz, sw, C, nrec, RAG);
   const int r0 = split_row(nz, C, rank), r1 = split_row(nz, C, rank + 1);
   const int zl0 = r0 - FD_PAD;
   const int bot_off = (C == 1) ? sw : 0;
@@ -285,43 +329,44 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 
   for (int i = tid; i < L.total; i += NT) sm[i] = 0.0f;
   __syncthreads();
-  for (int i = tid; i < 3 * (NX + nz); i += NT) sm[L.off_prof + i] = g.prof[i];
+  for (int i = tid; i < 3 * nz; i += NT) sAZ[i] = g.prof[3 * nx + i];
   if (TRACES) {
     for (int r = tid; r < nrec; r += NT) {
-      const int z0 = p.st.rec_cell[4 * r] / NX;
+      const int z0 = p.st.rec_cell[4 * r] / nx;
       const bool ok = (z0 >= r0 || rank == 0) && (z0 < r1 || rank == C - 1);
       sRecOk[r] = ok ? 1 : 0;
       for (int k = 0; k < 4; ++k) {
         const int cell = p.st.rec_cell[4 * r + k];
-        sRecCell[4 * r + k] = ok ? (cell / NX - zl0) * NX + cell % NX : 0;
+        sRecCell[4 * r + k] = ok ? (cell / nx - zl0) * NX + cell % nx : 0;
         sRecW[4 * r + k] = p.st.rec_w[4 * r + k];
       }
     }
   }
 
   const bool pml = (wk == 0);
-  const int x = CL::x_of(wk, lane);
+  const int x = cl.x_of(wk, lane);
   const int zb = r0 + seg * S;
   const int ltid = light_tid<NSEG, NI, C>(tid, rank);
-  const int nrows = CL::active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
+  const int nrows = cl.active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
+  const PairIo<RAG> io{(nx & 1) == 0, cl.half(x)};
   // warps with rows that read a halo (and are sent to the neighbour)
   const bool edge = (C > 1) && ((rank > 0 && zb < r0 + FD_PAD) || (rank < C - 1 && zb + S > r1 - FD_PAD));
   HaloLink link;
-  if constexpr (LINK) link.init(sm + L.off_bar, ((rank > 0) + (rank < C - 1)) * FD_PAD * (NX - 2 * FD_PAD) * 4, tid);
+  if constexpr (LINK) link.init(sm + L.off_bar, ((rank > 0) + (rank < C - 1)) * FD_PAD * cl.pairs * 8, tid);
   const int ubase = (zb - zl0) * NX + x;                 // row 0 of the segment in U
-  const int abase = (zb - r0) * 2 * SW + CL::strip(x);   // row 0 in APX / ZX (PML warp)
+  const int abase = (zb - r0) * 2 * SW + cl.strip(x);   // row 0 in APX / ZX (PML warp)
   const int zsh = (zb < nz / 2) ? 0 : (nz - sw - bot_off);
   const int zbase = (zb - zsh) * NX + x;                 // row 0 in APZ / ZZ (z-strip rows)
-  const int gbase = zb * NX + x;                         // row 0 in a global [nz][NX] field
+  const int gbase = zb * nx + x;                         // row 0 in a global [nz][nx] field
 
   float ax0 = 0.f, ax1 = 0.f, bx0 = 0.f, bx1 = 0.f, dbx0 = 0.f, dbx1 = 0.f;
   if (pml) {
     ax0 = g.prof[x];
     ax1 = g.prof[x + 1];
-    bx0 = g.prof[NX + x];
-    bx1 = g.prof[NX + x + 1];
-    dbx0 = g.prof[2 * NX + x];
-    dbx1 = g.prof[2 * NX + x + 1];
+    bx0 = g.prof[nx + x];
+    bx1 = g.prof[nx + x + 1];
+    dbx0 = g.prof[2 * nx + x];
+    dbx1 = g.prof[2 * nx + x + 1];
   }
   const float opbx0 = 1.0f + bx0, opbx1 = 1.0f + bx1;
   const float2 ax = make_float2(ax0, ax1), bx = make_float2(bx0, bx1), dbx = make_float2(dbx0, dbx1),
@@ -352,30 +397,30 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   for (int i = 0; i < S; ++i) {
     uA[i] = uB[i] = make_float2(0.f, 0.f);
     if (i < nrows) {
-      const float2 v = __ldg(reinterpret_cast<const float2*>(vel + i * NX));
+      const float2 v = io.load(vel + i * nx);
       sts2(V2o + i * NX, v.x * v.x * dt2, v.y * v.y * dt2);
       if (STORE) sts2(C2o + i * NX, (2.0f * v.x) * dt2, (2.0f * v.y) * dt2);
-      const int cell = gbase + i * NX;
+      const int cell = gbase + i * nx;
       if (cell == sc[0] || cell == sc[1] || cell == sc[2] || cell == sc[3]) srcmask |= 1u << (2 * i);
       if (cell + 1 == sc[0] || cell + 1 == sc[1] || cell + 1 == sc[2] || cell + 1 == sc[3])
         srcmask |= 1u << (2 * i + 1);
     }
   }
 
-  const size_t ckf = ckpt_floats(NX, nz, sw);
+  const size_t ckf = ckpt_floats(nx, nz, sw);
   if (p.ck_in) {
     const float* ck = p.ck_in + (static_cast<size_t>(unit) * p.ck_slots + p.ck_in_slot) * ckf;
     const float* cU = ck;
     const float* cP = ck + cells;
     const float* cAX = ck + 2 * cells;
     const float* cAZ = cAX + static_cast<size_t>(nz) * 2 * sw;
-    const float* cZX = cAZ + static_cast<size_t>(2) * sw * NX;
+    const float* cZX = cAZ + static_cast<size_t>(2) * sw * nx;
     const float* cZZ = cZX + static_cast<size_t>(nz) * 2 * sw;
-    constexpr int W = NX - 2 * FD_PAD;
+    const int W = nx - 2 * FD_PAD;
     const int ra = max(r0 - FD_PAD, FD_PAD), rb = min(r1 + FD_PAD, nz - FD_PAD);
     for (int i = tid; i < (rb - ra) * W; i += NT) {
       const int z = ra + i / W, xx = FD_PAD + i % W;
-      U[(z - zl0) * NX + xx] = cU[z * NX + xx];
+      U[(z - zl0) * NX + xx] = cU[z * nx + xx];
     }
 #pragma unroll
     for (int i = 0; i < S; ++i) {
@@ -384,17 +429,18 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int xx = x + j;
-          (j ? uA[i].y : uA[i].x) = cU[z * NX + xx];
-          (j ? uB[i].y : uB[i].x) = cP[z * NX + xx];
-          if (xx < sw || xx >= NX - sw) {
-            const int xc = strip_col(xx, NX, sw);
+          if (j && io.half) break;
+          (j ? uA[i].y : uA[i].x) = cU[z * nx + xx];
+          (j ? uB[i].y : uB[i].x) = cP[z * nx + xx];
+          if (xx < sw || xx >= nx - sw) {
+            const int xc = strip_col(xx, nx, sw);
             APX[abase + i * 2 * SW + j] = cAX[z * 2 * sw + xc];
             ZX[abase + i * 2 * SW + j] = cZX[z * 2 * sw + xc];
           }
           if (z < sw || z >= nz - sw) {
             const int zc = strip_col(z, nz, sw);
-            APZ[zbase + i * NX + j] = cAZ[zc * NX + xx];
-            ZZ[zbase + i * NX + j] = cZZ[zc * NX + xx];
+            APZ[zbase + i * NX + j] = cAZ[zc * nx + xx];
+            ZZ[zbase + i * NX + j] = cZZ[zc * nx + xx];
           }
         }
       }
@@ -427,7 +473,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
       float* ck = p.ck_out + (static_cast<size_t>(unit) * p.ck_slots + (t / p.ck_every - 1)) * ckf;
       float* cAX = ck + 2 * cells;
       float* cAZ = cAX + static_cast<size_t>(nz) * 2 * sw;
-      float* cZX = cAZ + static_cast<size_t>(2) * sw * NX;
+      float* cZX = cAZ + static_cast<size_t>(2) * sw * nx;
       float* cZZ = cZX + static_cast<size_t>(nz) * 2 * sw;
 #pragma unroll
       for (int i = 0; i < S; ++i) {
@@ -436,17 +482,18 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             const int xx = x + j;
-            ck[z * NX + xx] = j ? uc[i].y : uc[i].x;
-            ck[cells + z * NX + xx] = j ? un[i].y : un[i].x;
-            if (xx < sw || xx >= NX - sw) {
-              const int xc = strip_col(xx, NX, sw);
+            if (j && io.half) break;
+            ck[z * nx + xx] = j ? uc[i].y : uc[i].x;
+            ck[cells + z * nx + xx] = j ? un[i].y : un[i].x;
+            if (xx < sw || xx >= nx - sw) {
+              const int xc = strip_col(xx, nx, sw);
               cAX[z * 2 * sw + xc] = APXc[i * 2 * SW + j];
               cZX[z * 2 * sw + xc] = ZXo[i * 2 * SW + j];
             }
             if (z < sw || z >= nz - sw) {
               const int zc = strip_col(z, nz, sw);
-              cAZ[zc * NX + xx] = APZc[i * NX + j];
-              cZZ[zc * NX + xx] = ZZo[i * NX + j];
+              cAZ[zc * nx + xx] = APZc[i * NX + j];
+              cZZ[zc * nx + xx] = ZZo[i * NX + j];
             }
           }
         }
@@ -534,7 +581,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
             const float2 vv = lds2(V2o + i * NX);
             if (STORE) {
               const float2 cc = lds2(C2o + i * NX);
-              *reinterpret_cast<float2*>(stg + i * NX) = make_float2(cc.x * w0, cc.y * w1);
+              io.store(stg + i * nx, make_float2(cc.x * w0, cc.y * w1));
             }
             n0 = fmaf(vv.x, w0, fmaf(2.0f, u0, -un[i].x));
             n1 = fmaf(vv.y, w1, fmaf(2.0f, u1, -un[i].y));
@@ -550,8 +597,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               const float2 tmp = add2(add2(pk.mul(opbx, w), pk.mul(dbx, d1)), da);
               const float2 az = pk.mul(ax, Z);
               w = add2(pk.mul(opbx, tmp), az);
-              sts2(zxo + i * 2 * SW, add2(pk.mul(bx, tmp), az));
-              sts2(apxn + i * 2 * SW, mul2(ax, add2(pk.mul(bx, d1), P1)));
+              sts2(zxo + i * 2 * SW, io.mask(add2(pk.mul(bx, tmp), az)));
+              sts2(apxn + i * 2 * SW, io.mask(mul2(ax, add2(pk.mul(bx, d1), P1))));
             }
             const float2 d2z = pk.second(u, add2(zp1, zm1), add2(zp2, zm2), d2a, d2b);
             if (z < region || z >= nz - region) {
@@ -574,13 +621,13 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               w = add2(w, d2z);
             }
             // written as the row is updated: holding them for after the barrier spilled registers
-            if (STORE) *reinterpret_cast<float2*>(stg + i * NX) = mul2(lds2(C2o + i * NX), w);
+            if (STORE) io.store(stg + i * nx, mul2(lds2(C2o + i * NX), w));
             const float2 n = sub2(add2(pk.mul(lds2(V2o + i * NX), w), add2(u, u)), un[i]);
             n0 = n.x;
             n1 = n.y;
           }
           if (wsrc & (3u << (2 * i))) {
-            const int cell = gbase + i * NX;
+            const int cell = gbase + i * nx;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int c = sSrcCell[k];
@@ -590,6 +637,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
               n1 = (cell + 1 == c) ? a1 : n1;
             }
           }
+          if (RAG && io.half) n1 = 0.0f;
           un[i] = make_float2(n0, n1);
           sts2(uw + i * NX, n0, n1);
           if constexpr (C > 1) {
@@ -652,7 +700,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
 // registers per thread) instead of loading each row's terms when the row is processed.
 template <int NX, int PMLP, int C, int S, int NSEG, int NI, int LAY, bool PREF>
 __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __grid_constant__ AdjArgs p) {
-  using CL = Cols3<NX, PMLP>;
+  constexpr bool RAG = LAY == LAY_RAGGED;
+  using CL = Cols3<NX, PMLP, RAG>;
   constexpr int SW = CL::SW;
   constexpr int NT = NSEG * 32 * (1 + NI);
   extern __shared__ __align__(16) float sm[];
@@ -660,6 +709,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   constexpr bool SQ = LAY == LAY_SQUARE;
   constexpr bool FULL = LAY == LAY_EVEN || (SQ && NX - 2 * FD_PAD == C * S * NSEG);  // S rows per segment
   const int nz = SQ ? NX : g.nz;                                                     // compile-time if square
+  const CL cl(g.nx);
+  const int nx = cl.nx;  // width of the grid and row stride in global memory; NX: row stride in shared memory
   const int swa = g.swa, region = g.region_adj, nrec = p.st.nrec, nt = g.nt;
   const float rh = g.rh, dt2 = g.dt2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -668,8 +719,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   const int unit = blockIdx.x / C;
   const int shot = unit % p.st.shots;
   const int model = unit / p.st.shots;
-  const size_t cells = static_cast<size_t>(NX) * nz;
-  const A3Layout L = a3_layout_rt(NX, PMLP, nz, swa, C, nrec);
+  const size_t cells = static_cast<size_t>(nx) * nz;
+  const A3Layout L = a3_layout_rt(NX, PMLP, nz, swa, C, nrec, RAG);
   const int r0 = split_row(nz, C, rank), r1 = split_row(nz, C, rank + 1);
   const int zl0 = r0 - FD_PAD;
   const int bot_off = (C == 1) ? swa : 0;
@@ -683,12 +734,14 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
 
   for (int i = tid; i < L.total; i += NT) sm[i] = 0.0f;
   __syncthreads();
-  for (int i = tid; i < 3 * (NX + nz); i += NT) sAX[i] = g.prof[i];
+  for (int i = tid; i < 3 * nx; i += NT) sAX[(i / nx) * NX + i % nx] = g.prof[i];
+  for (int i = tid; i < 3 * nz; i += NT) sAZ[i] = g.prof[3 * nx + i];
 
   const bool pml = (wk == 0);
-  const int x = CL::x_of(wk, lane);
+  const int x = cl.x_of(wk, lane);
   const int zb = r0 + seg * S;
-  const int nrows = CL::active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
+  const int nrows = cl.active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
+  const PairIo<RAG> io{(nx & 1) == 0, cl.half(x)};
   const bool pusher = (C > 1) && nrows > 0 && ((rank > 0 && zb < r0 + FD_PAD) || (rank < C - 1 && zb + nrows > r1 - FD_PAD));
   // The PML warp's stencil reaches two columns past its own on the interior side: the pair next to
   // the interior on the left strip reads x + 2, x + 3, the one on the right strip x - 2, x - 1.
@@ -696,12 +749,12 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   // (T = 1 VS + 0 zeta differs from VS at most in the sign of a zero): those two lanes read VS
   // instead, so only the PML warp derives strip terms for the x strips.
   const bool edge_r = pml && (x + 2 == FD_PAD + CL::PCOLS);
-  const bool edge_l = pml && (x == NX - FD_PAD - CL::PCOLS);
+  const bool edge_l = pml && (x == FD_PAD + 2 * cl.right);
   const int vbase = (zb - zl0) * NX + x;
-  const int abase = (zb - r0) * 2 * SW + CL::strip(x);
+  const int abase = (zb - r0) * 2 * SW + cl.strip(x);
   const int zsh = (zb < nz / 2) ? 0 : (nz - swa - bot_off);
   const int zbase = (zb - zsh) * NX + x;
-  const int gbase = zb * NX + x;
+  const int gbase = zb * nx + x;
   float* LPX = sm + L.off_lpx + abase;
   float* LZX = sm + L.off_lzx + abase;
   float* LPZ = sm + L.off_lpz + zbase;
@@ -715,7 +768,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
 
   // per-column constants live in shared memory: (1 + b) in sOPB, a, b, db in the profiles
   float* sOPB = sm + L.off_opb;
-  for (int i = tid; i < NX; i += NT) sOPB[i] = 1.0f + g.prof[NX + i];
+  for (int i = tid; i < nx; i += NT) sOPB[i] = 1.0f + g.prof[nx + i];
   // Source corners: cell and the step-invariant factor ((-2 v) dt^2) w of the shader's
   // ((((-2 v) dt^2) w) f) (left to right, so the product with f rounds identically).
   int* sSrcCell = reinterpret_cast<int*>(sm + L.off_src);
@@ -741,8 +794,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   int* sER = reinterpret_cast<int*>(sm + L.off_er);
   float* sP = sm + L.off_res;
   const int crows = r1 - r0;
-  const int E0 = p.st.csr[r0 * NX];
-  const int ecnt = p.st.csr[r1 * NX] - E0;
+  const int E0 = p.st.csr[r0 * nx];
+  const int ecnt = p.st.csr[r1 * nx] - E0;
   const bool stage = ecnt <= L.pcap && ecnt <= NT;
   const int ltid = light_tid<NSEG, NI, C>(tid, rank);
   const float* resu = p.residual + static_cast<size_t>(unit) * nt * nrec;
@@ -759,7 +812,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
     int used = 0;
     for (int c0 = 0; c0 < crows; c0 += 32) {
       const int r = c0 + lane;
-      const bool has = r < crows && p.st.csr[(r0 + r) * NX] < p.st.csr[(r0 + r + 1) * NX];
+      const bool has = r < crows && p.st.csr[(r0 + r) * nx] < p.st.csr[(r0 + r + 1) * nx];
       const unsigned b = __ballot_sync(0xffffffffu, has);
       const int slot = used + __popc(b & ((1u << lane) - 1u));
       if (r < crows) sRRow[r] = (has && stage && slot < G3_REC_ROWS) ? slot : -1;
@@ -771,19 +824,19 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   unsigned srcmask = 0, recmask = 0;
   const int* sc = p.st.src_cell + 4 * shot;
   const float* vel = p.vel + static_cast<size_t>(model) * cells + gbase;
-  const size_t asf = adjstate_floats(NX, nz, swa);
+  const size_t asf = adjstate_floats(nx, nz, swa);
   float* stt = p.state + static_cast<size_t>(unit) * asf;
   float* sLc = stt;
   float* sLp = stt + cells;
   float* sPX = stt + 2 * cells;
   float* sZX = sPX + static_cast<size_t>(nz) * 2 * swa;
   float* sPZ = sZX + static_cast<size_t>(nz) * 2 * swa;
-  float* sZZ = sPZ + static_cast<size_t>(2) * swa * NX;
+  float* sZZ = sPZ + static_cast<size_t>(2) * swa * nx;
   float* gacc = p.gacc + static_cast<size_t>(unit) * cells + gbase;
   __syncthreads();
-  for (int i = tid; i < crows * (NX + 1); i += NT) {
-    const int r = i / (NX + 1), xx = i - r * (NX + 1), slot = sRRow[r];
-    if (slot >= 0) sROff[slot * (NX + 4) + xx] = p.st.csr[(r0 + r) * NX + xx] - E0;
+  for (int i = tid; i < crows * (nx + 1); i += NT) {
+    const int r = i / (nx + 1), xx = i - r * (nx + 1), slot = sRRow[r];
+    if (slot >= 0) sROff[slot * (NX + 4) + xx] = p.st.csr[(r0 + r) * nx + xx] - E0;
   }
   unsigned recslots = 0;  // per own row: 3 bits, the row's slot or 7 (global CSR)
 #pragma unroll
@@ -797,29 +850,30 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
     if (i < nrows) {
       const int z = zb + i;
       {
-        const float2 v = __ldg(reinterpret_cast<const float2*>(vel + i * NX));
+        const float2 v = io.load(vel + i * nx);
         sts2(V2o + i * NX, v.x * v.x * dt2, v.y * v.y * dt2);
         sts2(GAo + i * NX, 0.0f, 0.0f);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int cell = gbase + i * NX + j;
+        const int cell = gbase + i * nx + j;
+        if (j && io.half) break;
         if (cell == sc[0] || cell == sc[1] || cell == sc[2] || cell == sc[3]) srcmask |= 1u << (2 * i + j);
         if (p.st.csr[cell] < p.st.csr[cell + 1]) recmask |= 1u << (2 * i + j);
         if (!p.first) {
           lA[i][j] = sLc[cell];
           lB[i][j] = sLp[cell];
-          GAo[i * NX + j] = gacc[i * NX + j];
+          GAo[i * NX + j] = gacc[i * nx + j];
           const int xx = x + j;
-          if (xx < swa || xx >= NX - swa) {
-            const int xc = strip_col(xx, NX, swa);
+          if (xx < swa || xx >= nx - swa) {
+            const int xc = strip_col(xx, nx, swa);
             LPX[i * 2 * SW + j] = sPX[z * 2 * swa + xc];
             LZX[i * 2 * SW + j] = sZX[z * 2 * swa + xc];
           }
           if (z < swa || z >= nz - swa) {
             const int zc = strip_col(z, nz, swa);
-            LPZ[i * NX + j] = sPZ[zc * NX + xx];
-            LZZ[i * NX + j] = sZZ[zc * NX + xx];
+            LPZ[i * NX + j] = sPZ[zc * nx + xx];
+            LZZ[i * NX + j] = sZZ[zc * nx + xx];
           }
         }
       }
@@ -905,7 +959,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
     const float* st0 = p.stored + (static_cast<size_t>(unit) * segn + (p.t_hi - 1 - p.t_lo)) * cells + gbase;
 #pragma unroll
     for (int i = 0; i < S; ++i)
-      stv[i] = (i < nrows) ? __ldcs(reinterpret_cast<const float2*>(st0 + i * NX)) : make_float2(0.f, 0.f);
+      stv[i] = (i < nrows) ? io.load_stream(st0 + i * nx) : make_float2(0.f, 0.f);
   }
   // One reverse step at time t: `lc` holds lambda at t, `lp` holds the previous one and receives
   // the next.
@@ -948,7 +1002,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
           const float2 P = lds2(LPX + i * 2 * SW);
           const float2 Z = lds2(LZX + i * 2 * SW);
           const float2 a = lds2(sAX + x);
-          sts2(LPX + i * 2 * SW, ((-a.x) * dt0) + (a.x * P.x), ((-a.y) * dt1) + (a.y * P.y));
+          sts2(LPX + i * 2 * SW, io.mask(make_float2(((-a.x) * dt0) + (a.x * P.x), ((-a.y) * dt1) + (a.y * P.y))));
           sts2(LZX + i * 2 * SW, (a.x * Vb.x) + (a.x * Z.x), (a.y * Vb.y) + (a.y * Z.y));
         } else {
           const float2 Va = lds2(VSd + i * NX - 2), Vc = lds2(VSd + i * NX + 2);
@@ -985,7 +1039,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
         }
         float n0 = (w0 + (2.0f * lc[i][0])) - lp[i][0];
         float n1 = (w1 + (2.0f * lc[i][1])) - lp[i][1];
-        const float2 sv = PREF ? stv[PREF ? i : 0] : __ldcs(reinterpret_cast<const float2*>(st_t + i * NX));
+        const float2 sv = PREF ? stv[PREF ? i : 0] : io.load_stream(st_t + i * nx);
         // the shader starts the per-step gradient at +0; starting from the product itself differs
         // only in the sign of an exact zero
         float g0 = (lc[i][0] * sv.x) * 1.0f;
@@ -999,15 +1053,19 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
             for (int e = e0; e < e1; ++e) n0 = n0 + P[e];
             for (int e = e1; e < e2; ++e) n1 = n1 + P[e];
           } else {
-            const int cell = gbase + i * NX;
+            const int cell = gbase + i * nx;
             const int e1 = p.st.csr[cell + 1], e2 = p.st.csr[cell + 2];
             for (int e = p.st.csr[cell]; e < e1; ++e) n0 = n0 + (p.st.ent_w[e] * res_t[p.st.ent_rec[e]]);
             for (int e = e1; e < e2; ++e) n1 = n1 + (p.st.ent_w[e] * res_t[p.st.ent_rec[e]]);
           }
         }
+        if (RAG && io.half) {
+          n1 = 0.0f;
+          g1 = 0.0f;
+        }
         if (t > p.t_lo) put_vs(1 - par, i, n0, n1);  // VS of the new lambda for step t - 1
         if (wsrc & (3u << (2 * i))) {
-          const int cell = gbase + i * NX;
+          const int cell = gbase + i * nx;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const int c = sSrcCell[k];
@@ -1043,7 +1101,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
       const float* stn = p.stored + (static_cast<size_t>(unit) * segn + (t - 1 - p.t_lo)) * cells + gbase;
 #pragma unroll
       for (int i = 0; i < S; ++i)
-        if (i < nrows) stv[PREF ? i : 0] = __ldcs(reinterpret_cast<const float2*>(stn + i * NX));
+        if (i < nrows) stv[PREF ? i : 0] = io.load_stream(stn + i * nx);
     }
     if constexpr (C > 1) cluster_wait_acquire();
     else __syncthreads();
@@ -1066,20 +1124,21 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
       const int z = zb + i;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int cell = gbase + i * NX + j;
+        const int cell = gbase + i * nx + j;
+        if (j && io.half) break;
         sLc[cell] = flips ? lB[i][j] : lA[i][j];
         sLp[cell] = flips ? lA[i][j] : lB[i][j];
-        gacc[i * NX + j] = GAo[i * NX + j];
+        gacc[i * nx + j] = GAo[i * NX + j];
         const int xx = x + j;
-        if (xx < swa || xx >= NX - swa) {
-          const int xc = strip_col(xx, NX, swa);
+        if (xx < swa || xx >= nx - swa) {
+          const int xc = strip_col(xx, nx, swa);
           sPX[z * 2 * swa + xc] = LPX[i * 2 * SW + j];
           sZX[z * 2 * swa + xc] = LZX[i * 2 * SW + j];
         }
         if (z < swa || z >= nz - swa) {
           const int zc = strip_col(z, nz, swa);
-          sPZ[zc * NX + xx] = LPZ[i * NX + j];
-          sZZ[zc * NX + xx] = LZZ[i * NX + j];
+          sPZ[zc * nx + xx] = LPZ[i * NX + j];
+          sZZ[zc * nx + xx] = LZZ[i * NX + j];
         }
       }
     }
@@ -1138,6 +1197,18 @@ template <int NX, int PMLP, int C, int S, int NSEG, int NI>
 cudaError_t adj3_dispatch_impl_pref(const AdjArgs& a, size_t smem, cudaStream_t s) {
   if (a.prefetch) return adj3_dispatch_impl<NX, PMLP, C, S, NSEG, NI, true>(a, smem, s);
   return adj3_dispatch_impl<NX, PMLP, C, S, NSEG, NI, false>(a, smem, s);
+}
+
+// Grids of any width up to NX (LAY_RAGGED).
+template <int NX, int PMLP, int C, int S, int NSEG, int NI>
+cudaError_t fwd3r_dispatch_impl(bool traces, bool store, const FwdArgs& a, size_t smem, cudaStream_t s) {
+  return fwd3_launch<NX, PMLP, C, S, NSEG, NI, LAY_RAGGED, false>(traces, store, a, smem, s);
+}
+template <int NX, int PMLP, int C, int S, int NSEG, int NI>
+cudaError_t adj3r_dispatch_impl(const AdjArgs& a, size_t smem, cudaStream_t s) {
+  constexpr int NT = NSEG * 32 * (1 + NI);
+  if (a.prefetch) return launch_cluster(adj3_kernel<NX, PMLP, C, S, NSEG, NI, LAY_RAGGED, true>, C, NT, a.units, smem, s, a);
+  return launch_cluster(adj3_kernel<NX, PMLP, C, S, NSEG, NI, LAY_RAGGED, false>, C, NT, a.units, smem, s, a);
 }
 
 }  // namespace wg

@@ -8,7 +8,9 @@
 
 namespace wg {
 
-__host__ __device__ inline int g3_sw(int pmlp) { return 2 * pmlp + 4; }  // packed strip width per side
+__host__ __device__ constexpr int g3_sw(int pmlp) { return 2 * pmlp + 4; }  // packed strip width per side
+// of the x strips: on ragged widths the right strip may hold a column more, rounded to a pair
+__host__ __device__ constexpr int g3_xsw(int pmlp, bool rag) { return g3_sw(pmlp) + (rag ? 2 : 0); }
 
 // Wavelet samples kept in shared memory: a ring over the launch's steps, refilled half at a time.
 constexpr int G3_WAV_STEPS = 128;
@@ -18,16 +20,17 @@ struct F3Layout {
   int off_u, off_apx, off_zx, off_apz, off_zz, off_v2, off_c2, off_prof, off_rec, off_src, off_bar, total;
 };
 
-__host__ __device__ inline F3Layout f3_layout_rt(int NX, int pmlp, int nz, int sw, int C, int nrec) {
-  const int SW = g3_sw(pmlp);
+__host__ __device__ inline F3Layout f3_layout_rt(int NX, int pmlp, int nz, int sw, int C, int nrec,
+                                                  bool rag = false) {
+  const int SW = g3_sw(pmlp), XSW = g3_xsw(pmlp, rag);
   F3Layout L;
   L.maxrows = max_rows(nz, C);
   L.lr = L.maxrows + 2 * FD_PAD;
   L.zs = (C == 1 ? 2 : 1) * SW;
   L.off_u = 0;                                    // U[2][lr][NX]
   L.off_apx = L.off_u + 2 * L.lr * NX;            // APX[2][maxrows][2 SW]   a * psi_x
-  L.off_zx = L.off_apx + 2 * L.maxrows * 2 * SW;  // ZX[maxrows][2 SW]      zeta_x (owner only)
-  L.off_apz = L.off_zx + L.maxrows * 2 * SW;      // APZ[2][zs][NX]          a * psi_z
+  L.off_zx = L.off_apx + 2 * L.maxrows * 2 * XSW;  // ZX[maxrows][2 SW]      zeta_x (owner only)
+  L.off_apz = L.off_zx + L.maxrows * 2 * XSW;      // APZ[2][zs][NX]          a * psi_z
   L.off_zz = L.off_apz + 2 * L.zs * NX;           // ZZ[zs][NX]              zeta_z (owner only)
   L.off_v2 = L.off_zz + L.zs * NX;                // V2[maxrows][NX]         v^2 dt^2 (owner only)
   L.off_c2 = L.off_v2 + L.maxrows * NX;           // C2[maxrows][NX]         2 v dt^2 (owner only)
@@ -50,13 +53,14 @@ struct A3Layout {
 
 // VS is exchanged with the peer CTA and double-buffered; the x- and z-strip derived terms are read
 // only inside the CTA and are single-buffered (a CTA barrier separates their reads and writes).
-__host__ __device__ inline A3Layout a3_layout_rt(int NX, int pmlp, int nz, int swa, int C, int nrec) {
-  const int SW = g3_sw(pmlp);
+__host__ __device__ inline A3Layout a3_layout_rt(int NX, int pmlp, int nz, int swa, int C, int nrec,
+                                                  bool rag = false) {
+  const int SW = g3_sw(pmlp), XSW = g3_xsw(pmlp, rag);
   A3Layout L;
   L.maxrows = max_rows(nz, C);
   L.lr = L.maxrows + 2 * FD_PAD;
   L.zs = (C == 1 ? 2 : 1) * SW;
-  const int sx = L.maxrows * 2 * SW, sz = L.zs * NX;
+  const int sx = L.maxrows * 2 * XSW, sz = L.zs * NX;
   L.off_vs = 0;                           // VS[2][lr][NX]   v^2 dt^2 lambda
   L.off_tx = L.off_vs + 2 * L.lr * NX;    // TX[maxrows][2 SW]
   L.off_u1x = L.off_tx + sx;              // U1X[maxrows][2 SW]

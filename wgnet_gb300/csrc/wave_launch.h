@@ -31,6 +31,11 @@ template <int NX, int PMLP, int C, int S, int NSEG, int NI>
 cudaError_t fwd3_dispatch(bool traces, bool store, const FwdArgs& a, size_t smem, cudaStream_t s);
 template <int NX, int PMLP, int C, int S, int NSEG, int NI>
 cudaError_t adj3_dispatch(const AdjArgs& a, size_t smem, cudaStream_t s);
+// any grid width up to NX, compiled for the shapes of WG_G3_RAGGED_SHAPES (wave_table.cu)
+template <int NX, int PMLP, int C, int S, int NSEG, int NI>
+cudaError_t fwd3r_dispatch(bool traces, bool store, const FwdArgs& a, size_t smem, cudaStream_t s);
+template <int NX, int PMLP, int C, int S, int NSEG, int NI>
+cudaError_t adj3r_dispatch(const AdjArgs& a, size_t smem, cudaStream_t s);
 // fast-arithmetic forward, compiled for the shapes of WG_G3_FAST_SHAPES (wave_table.cu)
 template <int NX, int PMLP, int C, int S, int NSEG, int NI>
 cudaError_t fwd3f_dispatch(bool traces, bool store, const FwdArgs& a, size_t smem, cudaStream_t s);

@@ -38,6 +38,13 @@ namespace wg {
   X(144, 12, 4, 5, 7, 2)        \
   X(184, 12, 6, 6, 5, 3)
 
+// generation-3 shapes for any width up to NX (one instantiation file each), for the grids whose width
+// none of the above was compiled for
+#define WG_G3_RAGGED_SHAPES(X)  \
+  X(116, 12, 4, 5, 7, 1)        \
+  X(144, 12, 4, 5, 7, 2)        \
+  X(184, 12, 6, 6, 5, 3)
+
 #define WG_ADJ_SHAPES(X) \
   X(2, 1024, 6)          \
   X(2, 512, 12)          \
@@ -50,15 +57,18 @@ namespace wg {
 // CTA's rows and its shared-memory layout fits the 227 KB per-CTA limit.
 #define WG_LIST(Cc, NTt, CPTt) Shape{Cc, NTt, CPTt, 1, 0, 0, 0},
 #define WG_LIST3(NXs, PMLPs, Cc, Ss, NSEGs, NIs) Shape{Cc, NSEGs * 32 * (1 + NIs), 2 * Ss, 3, Ss, NSEGs, NIs, NXs, PMLPs},
-static const Shape kFwdShapes[] = {WG_G3_SHAPES(WG_LIST3) WG_SHAPES(WG_LIST)};
-static const Shape kAdjShapes[] = {WG_G3_SHAPES(WG_LIST3) WG_ADJ_SHAPES(WG_LIST)};
+#define WG_LIST3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs) \
+  Shape{Cc, NSEGs * 32 * (1 + NIs), 2 * Ss, 3, Ss, NSEGs, NIs, NXs, PMLPs, 0, 1},
+static const Shape kFwdShapes[] = {WG_G3_SHAPES(WG_LIST3) WG_G3_RAGGED_SHAPES(WG_LIST3R) WG_SHAPES(WG_LIST)};
+static const Shape kAdjShapes[] = {WG_G3_SHAPES(WG_LIST3) WG_G3_RAGGED_SHAPES(WG_LIST3R) WG_ADJ_SHAPES(WG_LIST)};
+#undef WG_LIST3R
 #undef WG_LIST
 #undef WG_LIST3
 
 // Whether the fast-arithmetic kernels exist for a generation-3 shape.
 static bool g3_has_fast(const Shape& s) {
 #define WG_HASF(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                  \
-  if (s.kind == 3 && s.nxc == NXs && s.pmlp == PMLPs && s.cluster == Cc && s.seg_rows == Ss && s.nseg == NSEGs && \
+  if (s.kind == 3 && !s.rag && s.nxc == NXs && s.pmlp == PMLPs && s.cluster == Cc && s.seg_rows == Ss && s.nseg == NSEGs && \
       s.ni == NIs)                                                                                                 \
     return true;
   WG_G3_FAST_SHAPES(WG_HASF)
@@ -77,24 +87,37 @@ Shape fwd_shape(int i) { return with_fast(kFwdShapes[i]); }
 Shape adj_shape(int i) { return with_fast(kAdjShapes[i]); }
 
 size_t fwd_smem_bytes(const Shape& s, int nx, int nz, int sw, int nrec) {
-  if (s.kind == 3) return static_cast<size_t>(f3_layout_rt(s.nxc, s.pmlp, nz, sw, s.cluster, nrec).total) * sizeof(float);
+  if (s.kind == 3) return static_cast<size_t>(f3_layout_rt(s.nxc, s.pmlp, nz, sw, s.cluster, nrec, s.rag != 0).total) * sizeof(float);
   return static_cast<size_t>(fwd_layout(nx, nz, sw, s.cluster, nrec).total) * sizeof(float);
 }
 size_t adj_smem_bytes(const Shape& s, int nx, int nz, int swa, int nrec) {
   if (s.kind == 3)
-    return static_cast<size_t>(a3_layout_rt(s.nxc, s.pmlp, nz, swa, s.cluster, nrec).total) * sizeof(float);
+    return static_cast<size_t>(a3_layout_rt(s.nxc, s.pmlp, nz, swa, s.cluster, nrec, s.rag != 0).total) * sizeof(float);
   return static_cast<size_t>(adj_layout(nx, nz, swa, s.cluster).total) * sizeof(float);
 }
 
-// A generation-3 shape fits when the grid width equals its compile-time width, its PML warp covers
-// the adjoint's C-PML columns [2, region_adj) (which contain the forward's), its interior warps
-// cover the columns in between and its segments cover the CTA's rows.
+// A generation-3 shape fits when the grid width equals its compile-time width (a ragged one: is at
+// most that, odd or even, and no other shape was compiled for it), its PML warp covers the adjoint's
+// C-PML columns [2, region_adj) (which contain the forward's), its interior warps cover the columns in
+// between and its segments cover the CTA's rows.
+static bool g3_exact_width(int nx) {
+  bool found = false;
+#define WG_WIDTH(NXs, PMLPs, Cc, Ss, NSEGs, NIs) found = found || nx == NXs;
+  WG_G3_SHAPES(WG_WIDTH)
+#undef WG_WIDTH
+  return found;
+}
 static bool g3_fits(const Shape& s, int nx, int nz, int rows, int region_adj) {
-  if (nx != s.nxc || (nx & 1)) return false;
   if (FD_PAD + 2 * s.pmlp < region_adj) return false;
+  if (rows > s.seg_rows * s.nseg || nz < 2 * g3_sw(s.pmlp)) return false;
+  if (s.rag) {
+    // pairs left of the right strip, without the left strip's; two at least keep the packed strips apart
+    const int ipairs = (nx - 2 * FD_PAD - 2 * s.pmlp) / 2 - s.pmlp;
+    return nx <= s.nxc && !g3_exact_width(nx) && ipairs >= 2 && ipairs <= 32 * s.ni;
+  }
+  if (nx != s.nxc || (nx & 1)) return false;
   const int ipairs = (nx - 2 * FD_PAD - 4 * s.pmlp) / 2;
-  if (ipairs < 1 || ipairs > 32 * s.ni) return false;
-  return rows <= s.seg_rows * s.nseg && nz >= 2 * g3_sw(s.pmlp);
+  return ipairs >= 1 && ipairs <= 32 * s.ni;
 }
 
 bool fwd_shape_fits(const Shape& s, int nx, int nz, int sw, int nrec) {
@@ -130,6 +153,14 @@ bool adj_shape_fits(const Shape& s, int nx, int nz, int swa, int nrec) {
 
 cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a, cudaStream_t stream) {
   const size_t smem = fwd_smem_bytes(s, a.g.nx, a.g.nz, a.g.sw, a.st.nrec);
+  if (s.kind == 3 && s.rag) {
+#define WG_FWD3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
+  if (s.nxc == NXs && s.pmlp == PMLPs && s.cluster == Cc && s.seg_rows == Ss && s.nseg == NSEGs && s.ni == NIs) \
+    return fwd3r_dispatch<NXs, PMLPs, Cc, Ss, NSEGs, NIs>(traces, store, a, smem, stream);
+    WG_G3_RAGGED_SHAPES(WG_FWD3R)
+#undef WG_FWD3R
+    return cudaErrorInvalidValue;
+  }
   if (s.kind == 3) {
     if (a.fast) {  // shapes without fast-arithmetic kernels run the unfused ones
 #define WG_FWD3F(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
@@ -154,6 +185,14 @@ cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a
 
 cudaError_t launch_adj(const Shape& s, const AdjArgs& a, cudaStream_t stream) {
   const size_t smem = adj_smem_bytes(s, a.g.nx, a.g.nz, a.g.swa, a.st.nrec);
+  if (s.kind == 3 && s.rag) {
+#define WG_ADJ3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
+  if (s.nxc == NXs && s.pmlp == PMLPs && s.cluster == Cc && s.seg_rows == Ss && s.nseg == NSEGs && s.ni == NIs) \
+    return adj3r_dispatch<NXs, PMLPs, Cc, Ss, NSEGs, NIs>(a, smem, stream);
+    WG_G3_RAGGED_SHAPES(WG_ADJ3R)
+#undef WG_ADJ3R
+    return cudaErrorInvalidValue;
+  }
   if (s.kind == 3) {
 #define WG_ADJ3(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                  \
   if (s.nxc == NXs && s.pmlp == PMLPs && s.cluster == Cc && s.seg_rows == Ss && s.nseg == NSEGs && s.ni == NIs) \
