@@ -65,3 +65,26 @@ def test_a_nan_cell_on_an_odd_width(cuda_lib):
     obs = o.forward(sv, np.nan_to_num(cur, nan=2000.0), src, wav)
     np.testing.assert_array_equal(eng.simulate(cur), o.forward(sv, cur, src, wav))
     np.testing.assert_array_equal(eng.evaluate_adjoint(cur, obs)[1], o.evaluate_adjoint(sv, cur, src, wav, obs)[1])
+
+
+@pytest.mark.parametrize("models,shots", [(1, 5), (2, 2), (18, 2), (8, 5), (23, 2), (24, 2), (16, 5)])
+def test_small_batches_take_other_shapes_and_no_checkpoints_with_equal_results(cuda_lib, models, shots):
+    """Up to 36 units fit the chip in clusters of four, 46 of three, 76 of two (and 80 to 92 take two
+    waves of three), so the default shapes differ; an engine with default checkpointing keeps every
+    term of a small batch."""
+    sv = o.Survey(shots=shots, nt=130, dt=0.001)
+    rng = np.random.default_rng(models)
+    cur = (1700.0 + 2500.0 * rng.random((models, 70, 70))).astype(np.float32)
+    src = sv.default_sources()
+    eng, fixed = _engine(sv, src), _engine(sv, src, checkpoint_every=50)
+    fixed.set_launch_shape("forward", (2, 704, 10))
+    fixed.set_launch_shape("adjoint", (2, 704, 10))
+    obs = fixed.simulate(cur[::-1].copy())
+    np.testing.assert_array_equal(eng.simulate(cur[::-1].copy()), obs)
+    l0, g0 = eng.evaluate_adjoint(cur, obs)
+    l1, g1 = fixed.evaluate_adjoint(cur, obs)
+    np.testing.assert_array_equal(g0, g1)
+    np.testing.assert_array_equal(l0, l1)
+    k = min(models, 2)
+    np.testing.assert_array_equal(g0[:k], o.evaluate_adjoint(sv, cur[:k], src, eng.wavelet(), obs[:k])[1])
+    assert eng.checkpoint_every == 50

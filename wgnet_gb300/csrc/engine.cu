@@ -143,7 +143,16 @@ struct wg_engine {
   cudaStream_t stream = nullptr;
   DevBuf d_prof, d_wavelet, d_src_cell, d_src_w, d_rec_cell, d_rec_w, d_csr, d_ent_rec, d_ent_w, d_status;
   wg::Shape fshape{0, 0, 0}, ashape{0, 0, 0};
+  // shapes to choose from by the number of units (unused once a launch shape has been set)
+  struct Choice {
+    wg::Shape s;
+    float cost;  // time of a step
+    int slots;   // clusters the chip holds at once
+  };
+  std::vector<Choice> fchoice, achoice;
+  bool fshape_set = false, ashape_set = false;
   int ck_every = 50;
+  bool ck_set = false;  // an interval was set: it is kept to whatever memory is free
   int adj_prefetch = 1;
   int fast = 0;      // 1: fast-arithmetic resident kernels (option "arith")
   int tblock = 0;    // streamed path: temporally blocked forward (option "temporal_block")
@@ -321,7 +330,8 @@ int find_shape(const wg_engine* e, int which, int cluster, int threads, int cpt,
 bool pick_shapes(wg_engine* e) {
   // Preference order; the first compiled shape that fits the grid is the default (the autotuner
   // can choose another among wg_shape_candidates).
-  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 896, 4}, {4, 448, 8}, {4, 448, 10}, {1, 1024, 12},
+  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 896, 4}, {4, 448, 8},
+                                 {4, 448, 10}, {1, 1024, 12},
                                  {2, 1024, 6}, {2, 512, 12}, {2, 1024, 10}, {4, 1024, 8}, {2, 1024, 16},
                                  {4, 512, 16}};
   static const int apref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 448, 10}, {2, 1024, 6}, {4, 896, 4}, {4, 448, 8},
@@ -342,7 +352,51 @@ bool pick_shapes(wg_engine* e) {
       break;
     }
   }
+  // What a step costs in each shape (us, one wave of clusters, nt 200; forward: mean of recording
+  // traces and storing terms), measured on the 70 x 70 (stride 114), 100 x 100 (144), 72 x 100 (ragged
+  // 116) and 93 x 77 (ragged 144) grids. Only ratios between shapes of one grid are used.
+  static const struct {
+    int nxc, rag, cluster, threads, cpt;
+    float fwd, adj;
+  } costs[] = {{114, 0, 2, 704, 10, 2.69f, 4.67f}, {114, 0, 3, 832, 6, 2.16f, 4.00f}, {114, 0, 3, 640, 8, 2.22f, 3.79f},
+               {114, 0, 4, 448, 8, 1.85f, 3.37f},  {114, 0, 4, 896, 4, 1.86f, 3.25f}, {144, 0, 4, 672, 10, 2.68f, 4.95f},
+               {144, 0, 3, 768, 12, 3.42f, 0.0f},  {116, 1, 4, 448, 10, 2.40f, 5.19f}, {116, 1, 3, 768, 8, 2.74f, 5.07f},
+               {144, 1, 4, 672, 10, 3.02f, 5.32f}, {144, 1, 3, 768, 10, 3.30f, 5.64f}, {144, 1, 3, 768, 12, 4.06f, 7.33f}};
+  for (int which = 0; which < 2; ++which) {
+    const int n = which == 0 ? wg::fwd_shape_count() : wg::adj_shape_count();
+    for (int i = 0; i < n; ++i) {
+      const wg::Shape s = which == 0 ? wg::fwd_shape(i) : wg::adj_shape(i);
+      if (s.kind != 3 || !shape_fits(e, which, s)) continue;
+      for (const auto& c : costs) {
+        const float cost = which == 0 ? c.fwd : c.adj;
+        if (c.nxc == s.nxc && c.rag == s.rag && c.cluster == s.cluster && c.threads == s.threads && c.cpt == s.cpt && cost > 0)
+          (which == 0 ? e->fchoice : e->achoice).push_back({s, cost, wg::resident_clusters(s.cluster)});
+      }
+    }
+  }
   return e->fshape.cluster > 0;
+}
+
+// Launch shape of a pass over `units`: the one whose waves of clusters take the least time. Few CTAs per
+// unit use the SMs best (the C-PML's rows sit in the outer CTAs, the inner ones of wide clusters wait
+// for them), many finish a step soonest: on the 70 x 70 grid 5 units x 2001 steps take 3.74 ms in four
+// CTAs per unit against 5.24 in two, and 40 units, one too many for a wave of four, take 2.2 us a step in
+// three against 2.7 in two and 3.7 in two waves of four. With fast arithmetic, only shapes that have it.
+wg::Shape shape_for(const wg_engine* e, int which, int units) {
+  const wg::Shape def = which == 0 ? e->fshape : e->ashape;
+  if (which == 0 ? e->fshape_set : e->ashape_set) return def;
+  wg::Shape best = def;
+  float least = 0.0f;
+  for (const auto& c : which == 0 ? e->fchoice : e->achoice) {
+    if (which == 0 && e->fast && def.fast && !c.s.fast) continue;
+    if (c.slots < 1) continue;
+    const float t = static_cast<float>((units + c.slots - 1) / c.slots) * c.cost;
+    if (least == 0.0f || t < least) {
+      least = t;
+      best = c.s;
+    }
+  }
+  return best;
 }
 
 int create_impl(const wg_config* c, bool cpu_d2, wg_engine** out) {
@@ -535,13 +589,33 @@ int simulate_dev_impl(wg_engine* e, const float* d_vis, int models, float* d_tra
     a.traces = d_traces + static_cast<size_t>(m0) * e->shots * e->nt * e->nrec;
     a.status = e->d_status.as<int>();
     a.fast = e->fast;
-    WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(e->fshape, true, false, a, st); }));
+    const wg::Shape fs = shape_for(e, 0, a.units);
+    WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, false, a, st); }));
   }
   return WG_OK;
 }
 
 // obs_ready (optional): an event the observed data's arrival is recorded on; nothing reads them
 // before the first forward pass has been launched, so their host->device copy can overlap it.
+// An engine whose checkpoint interval was never set keeps every step's gradient term (no recompute:
+// the gradient is the same bit for bit) when the batch's terms are small beside the memory: at most
+// kStoreBytes and an eighth of what is free, and the allocation succeeds; the buffer then stays with
+// the engine, as its other workspaces do. One default-engine gradient (5 shots, nt 2001, 0.5 GB of
+// terms): 1 x 2001 steps of forward saved, 3.7 of 14 ms.
+constexpr size_t kStoreBytes = size_t(4) << 30;
+bool store_by_default(wg_engine* e, int models) {
+  if (e->ck_set) return false;
+  const size_t need = static_cast<size_t>(models) * e->shots * e->nt * e->cells * 4;
+  if (need > kStoreBytes) return false;
+  if (need <= e->w_stored.bytes) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return need <= free_b / 8 && e->w_stored.ensure(need) == WG_OK;
+}
+
 int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int models, double* d_loss, float* d_grad,
                       cudaStream_t st, cudaEvent_t obs_ready = nullptr) {
   if (models < 1) return fail(WG_ERR_ARG, "models must be >= 1");
@@ -552,7 +626,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
                                timer_of(e));
   }
   if (e->ashape.cluster == 0) return fail(WG_ERR_UNSUPPORTED, "grid does not fit the resident adjoint kernel");
-  const bool store_all = e->ck_every <= 0 || e->ck_every >= e->nt;
+  const bool store_all = e->ck_every <= 0 || e->ck_every >= e->nt || store_by_default(e, models);
   const int k = store_all ? e->nt : e->ck_every;
   const int J = store_all ? 1 : (e->nt + k - 1) / k;
   const int slots = J - 1;
@@ -575,6 +649,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
   for (int m0 = 0; m0 < models; m0 += M) {
     const int mc = std::min(M, models - m0);
     const int units = mc * e->shots;
+    const wg::Shape fs = shape_for(e, 0, units), as = shape_for(e, 1, units);
     const float* obs = d_obs + static_cast<size_t>(m0) * S * tr;
     WG_LAUNCH(wg::launch_pad_velocity(d_vis + static_cast<size_t>(m0) * e->nx_vis * e->nz_vis, mc, e->nx_vis,
                                       e->nz_vis, e->pad, e->cfg.vmin, e->cfg.vmax, e->w_vpad.as<float>(),
@@ -591,7 +666,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
     f.fast = e->fast;
     if (store_all) {
       f.stored = e->w_stored.as<float>();
-      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(e->fshape, true, true, f, st); }));
+      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, true, f, st); }));
     } else {
       // Steps [0, (J-1) k] with receivers and checkpoints (the last checkpoint is written at the
       // start of step (J-1) k, which is computed once more below), then the last segment from
@@ -601,7 +676,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
       f.ck_every = k;
       f.ck_slots = slots;
       f.t1 = (J - 1) * k + 1;
-      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(e->fshape, true, false, f, st); }));
+      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, false, f, st); }));
       wg::FwdArgs l = f;
       l.t0 = (J - 1) * k;
       l.t1 = e->nt;
@@ -609,7 +684,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
       l.ck_in = e->w_ckpt.as<float>();
       l.ck_in_slot = J - 2;
       l.stored = e->w_stored.as<float>();
-      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(e->fshape, true, true, l, st); }));
+      WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, true, l, st); }));
     }
     if (obs_ready && m0 == 0) WG_CK(cudaStreamWaitEvent(st, obs_ready, 0));
     WG_LAUNCH(wg::launch_energy(obs, mc, S * tr, e->w_energy.as<double>(), e->w_scale.as<float>(),
@@ -632,7 +707,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
       a.t_hi = e->nt;
       a.t_lo = 0;
       a.first = 1;
-      WG_LAUNCH(timed(e, K_ADJ, st, [&] { return wg::launch_adj(e->ashape, a, st); }));
+      WG_LAUNCH(timed(e, K_ADJ, st, [&] { return wg::launch_adj(as, a, st); }));
     } else {
       for (int j = J - 1; j >= 0; --j) {
         const int t0 = j * k, t1 = std::min(t0 + k, e->nt);
@@ -651,11 +726,11 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
         r.status = e->d_status.as<int>();
         r.fast = e->fast;
         if (j < J - 1)  // the last segment's terms are already stored by the first pass
-          WG_LAUNCH(timed(e, K_RECOMPUTE, st, [&] { return wg::launch_fwd(e->fshape, false, true, r, st); }));
+          WG_LAUNCH(timed(e, K_RECOMPUTE, st, [&] { return wg::launch_fwd(fs, false, true, r, st); }));
         a.t_hi = t1;
         a.t_lo = t0;
         a.first = (j == J - 1) ? 1 : 0;
-        WG_LAUNCH(timed(e, K_ADJ, st, [&] { return wg::launch_adj(e->ashape, a, st); }));
+        WG_LAUNCH(timed(e, K_ADJ, st, [&] { return wg::launch_adj(as, a, st); }));
       }
     }
     WG_LAUNCH(wg::launch_fold(e->w_gacc.as<float>(), e->w_mask.as<float>(), mc, e->shots, e->nx, e->nz, e->pad,
@@ -882,6 +957,7 @@ int wg_set_checkpoint_interval(wg_engine* e, int k) {
   if (!e) return fail(WG_ERR_ARG, "null engine");
   std::lock_guard<std::mutex> lk(e->mu);
   e->ck_every = k;
+  e->ck_set = true;
   return WG_OK;
 }
 
@@ -893,6 +969,7 @@ int wg_set_option(wg_engine* e, const char* key, int value) {
   const std::string k(key);
   if (k == "checkpoint_every") {
     e->ck_every = value;
+    e->ck_set = true;
   } else if (k == "adjoint_prefetch") {
     e->adj_prefetch = value ? 1 : 0;
   } else if (k == "arith") {
@@ -942,6 +1019,7 @@ int wg_set_launch_shape(wg_engine* e, int which, int cluster, int threads, int c
   if (found == 0) return fail(WG_ERR_ARG, "launch shape not compiled");
   if (found == 1) return fail(WG_ERR_ARG, which == 0 ? "forward shape does not fit this grid" : "adjoint shape does not fit this grid");
   (which == 0 ? e->fshape : e->ashape) = s;
+  (which == 0 ? e->fshape_set : e->ashape_set) = true;
   return WG_OK;
 }
 

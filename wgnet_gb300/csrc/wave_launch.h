@@ -22,6 +22,10 @@ size_t adj_smem_bytes(const Shape& s, int nx, int nz, int swa, int nrec);
 bool fwd_shape_fits(const Shape& s, int nx, int nz, int sw, int nrec);
 bool adj_shape_fits(const Shape& s, int nx, int nz, int swa, int nrec);
 
+// How many clusters of `cluster` CTAs, one CTA per SM, the current device holds at once (clusters lie
+// within a GPC, so fewer than SMs / cluster).
+int resident_clusters(int cluster);
+
 // Per-shape launchers, specialised in the wave_inst_*.cu files.
 template <int C, int NT, int CPT>
 cudaError_t fwd_dispatch(bool traces, bool store, const FwdArgs& a, size_t smem, cudaStream_t s);

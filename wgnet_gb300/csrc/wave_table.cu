@@ -1,5 +1,7 @@
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "wave_device.cuh"
 #include "wave_kernels3_layout.h"
 #include "wave_launch.h"
@@ -26,8 +28,11 @@ namespace wg {
   X(114, 12, 4, 4, 7, 1)        \
   X(114, 12, 4, 2, 14, 1)       \
   X(114, 12, 1, 8, 14, 1)       \
+  X(114, 12, 3, 3, 13, 1)       \
+  X(114, 12, 3, 4, 10, 1)       \
   X(144, 12, 4, 5, 7, 2)        \
   X(144, 12, 4, 7, 5, 2)        \
+  X(144, 12, 3, 6, 8, 2)        \
   X(184, 12, 6, 6, 5, 3)        \
   X(184, 12, 6, 10, 3, 3)
 
@@ -42,7 +47,10 @@ namespace wg {
 // none of the above was compiled for
 #define WG_G3_RAGGED_SHAPES(X)  \
   X(116, 12, 4, 5, 7, 1)        \
+  X(116, 12, 3, 4, 12, 1)       \
   X(144, 12, 4, 5, 7, 2)        \
+  X(144, 12, 3, 5, 8, 2)        \
+  X(144, 12, 3, 6, 8, 2)        \
   X(184, 12, 6, 6, 5, 3)
 
 #define WG_ADJ_SHAPES(X) \
@@ -149,6 +157,41 @@ bool adj_shape_fits(const Shape& s, int nx, int nz, int swa, int nrec) {
     if (split_row(nz, s.cluster, 1) < swa || split_row(nz, s.cluster, s.cluster - 1) > nz - swa) return false;
   }
   return nx < 65536 && nz < 32768;
+}
+
+// Stands for a resident kernel in the occupancy query: its shared memory allows one CTA per SM.
+static __global__ void one_per_sm_kernel() {
+  extern __shared__ float sm[];
+  sm[threadIdx.x] = 0.0f;
+}
+
+int resident_clusters(int cluster) {
+  constexpr int kMost = 17;
+  constexpr size_t kSmem = 150 * 1024;
+  static std::mutex mu;
+  static int known[64][kMost] = {};
+  int dev = 0;
+  if (cluster < 1 || cluster >= kMost || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (known[dev][cluster]) return known[dev][cluster];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(32);
+  cfg.dynamicSmemBytes = kSmem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(one_per_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
+      (cluster > 8 && cudaFuncSetAttribute(one_per_sm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, one_per_sm_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return known[dev][cluster] = n;
 }
 
 cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a, cudaStream_t stream) {
