@@ -156,6 +156,7 @@ struct wg_engine {
   int adj_prefetch = 1;
   int fast = 0;      // 1: fast-arithmetic resident kernels (option "arith")
   int tblock = 0;    // streamed path: temporally blocked forward (option "temporal_block")
+  bool tblock_set = false;
   int streamed = 0;  // 1: wavefields in HBM, one launch per step (grids beyond the resident kernels)
   cudaStream_t copy_stream = nullptr;  // host->device copy of observed data, overlapping the forward
   cudaEvent_t obs_ready = nullptr;
@@ -226,7 +227,7 @@ wg::EngineView view_of(const wg_engine* e) {
   v.d_status = e->d_status.as<int>();
   v.adj_prefetch = e->adj_prefetch;
   v.fast = e->fast;
-  v.tblock = e->tblock;
+  v.tblock = e->tblock_set ? e->tblock : -1;
   return v;
 }
 
@@ -977,6 +978,7 @@ int wg_set_option(wg_engine* e, const char* key, int value) {
     e->fast = value;
   } else if (k == "temporal_block") {
     e->tblock = value ? 1 : 0;
+    e->tblock_set = true;
   } else if (k == "streamed") {
     if (value) {
       std::string why;

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "wave_launch.h"
+#include "wave_packed.cuh"
 #include "wgnet_gb300.h"
 
 namespace wg {
@@ -64,12 +65,15 @@ struct SArgs {
   int seg;
   const float* residual; // [units][nt][nrec]
   float* gacc;           // [units][nz][nx]
+  alignas(8) float nz2[2];  // -0, for packed products (wave_packed.cuh)
 };
 
 __device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 ldg2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+
+__device__ __forceinline__ void put2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -111,36 +115,7 @@ __device__ __forceinline__ void tma_load(float* dst, const CUtensorMap* map, int
 
 __device__ __forceinline__ int xstrip(int x, int nx, int ssw) { return x < ssw ? x : x - (nx - 2 * ssw); }
 
-struct Pipe {
-  uint64_t* bar;
-  float* stage;  // [2][BZ * BX]
-};
-
-// Issue the tile load of job `job` (buffer `buf` of the wavefield) into stage s.
-__device__ __forceinline__ void issue(const SArgs& a, const CUtensorMap* map, Pipe& p, int job, int s, int buf) {
-  const int tiles = a.tiles_x * a.tiles_z;
-  const int unit = job / tiles, tile = job % tiles;
-  const int tz = tile / a.tiles_x, tx = tile % a.tiles_x;
-  mbar_expect_tx(&p.bar[s], kTileBytes);
-  tma_load(p.stage + s * BZ * BX, map, tx * TX_ - HX, tz * TZ_ - HZ, buf * a.units + unit, &p.bar[s]);
-}
-
 __device__ __forceinline__ void report(int* status) { atomicCAS(status, 0, ST_CUDA); }
-
-// A tile (with its halo) clear of the PML strips, the grid frame, the receivers' rows and this
-// unit's source corners: every pair of every row takes the interior formulas.
-__device__ __forceinline__ bool interior_tile(const SArgs& a, int x0, int z0, const int* sc) {
-  const int m = a.ssw;
-  if (x0 - HX < m || x0 + TX_ + HX > a.nx - m || z0 - HZ < m || z0 + TZ_ + HZ > a.nz - m) return false;
-  if (z0 + TZ_ > a.rec_z0 && z0 <= a.rec_z1) return false;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int c = __ldg(&sc[k]);
-    const int cz = c / a.nx, cx = c % a.nx;
-    if (cz >= z0 && cz < z0 + TZ_ && cx >= x0 && cx < x0 + TX_) return false;
-  }
-  return true;
-}
 
 // ------------------------------------------------------------------------------------------------
 // Forward step t: u_next = v^2 dt^2 w + 2 u - u_prev over every unit, receivers read before the
@@ -155,22 +130,91 @@ constexpr int FST = 3;                                        // forward pipelin
 constexpr int FSTAGE_F = BZ * BX + 2 * TZ_ * TX_;             // floats per stage: U | P | V
 constexpr size_t kFwdSmem = FST * FSTAGE_F * 4 + 128 + 16 * FST;
 
-// Issue the three copies of job `job` into stage buffer `st` with barrier `bar`.
-__device__ __forceinline__ void issue_fwd(const SArgs& a, const FwdMaps& m, float* st, uint64_t* bar, int job,
-                                          int par) {
-  const int tiles = a.tiles_x * a.tiles_z;
-  const int unit = job / tiles, tile = job % tiles;
-  const int tz = tile / a.tiles_x, tx = tile % a.tiles_x;
-  mbar_expect_tx(bar, FSTAGE_F * 4);
-  tma_load(st, &m.u, tx * TX_ - HX, tz * TZ_ - HZ, par * a.units + unit, bar);
-  tma_load(st + BZ * BX, &m.p, tx * TX_, tz * TZ_, (1 - par) * a.units + unit, bar);
-  tma_load(st + BZ * BX + TZ_ * TX_, &m.v, tx * TX_, tz * TZ_, unit / a.shots, bar);
-}
-
 constexpr int FWD_THREADS = NTH + 32;  // 8 consumer warps + 1 producer warp
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// One tile of a step's work, decoded once per CTA (by the thread that issues its copies) instead of by
+// every thread: the divisions and the look-up of the shot's source were a third of an interior tile's
+// instructions.
+struct Job {
+  int unit, tile, x0, z0;
+  int shot, inner, src, model;  // inner: interior formulas only; src: the source's corners touch the tile
+};
+
+// Walks the jobs blockIdx.x, blockIdx.x + gridDim.x, ... of a step.
+struct JobWalk {
+  int unit, tile, du, dt;
+  __device__ __forceinline__ explicit JobWalk(const SArgs& a) {
+    const int tiles = a.tiles_x * a.tiles_z, first = blockIdx.x, step = gridDim.x;
+    unit = first / tiles;
+    tile = first - unit * tiles;
+    du = step / tiles;
+    dt = step - du * tiles;
+  }
+  __device__ __forceinline__ void advance(const SArgs& a) {
+    const int tiles = a.tiles_x * a.tiles_z;
+    unit += du;
+    tile += dt;
+    if (tile >= tiles) {
+      tile -= tiles;
+      ++unit;
+    }
+  }
+  // A tile (with its halo) clear of the PML strips, the grid frame, the receivers' rows and this
+  // unit's source corners is an inner one: every pair of every row takes the interior formulas.
+  __device__ __forceinline__ Job decode(const SArgs& a) const {
+    Job j;
+    const int tz = tile / a.tiles_x;
+    j.unit = unit;
+    j.tile = tile;
+    j.x0 = (tile - tz * a.tiles_x) * TX_;
+    j.z0 = tz * TZ_;
+    j.model = unit / a.shots;
+    j.shot = unit - j.model * a.shots;
+    const int c = __ldg(&a.st.src_cell[4 * j.shot]);  // the first of the 2 x 2 corner cells
+    const int cz = c / a.nx, cx = c - cz * a.nx;
+    j.src = cz + 1 >= j.z0 && cz < j.z0 + TZ_ && cx + 1 >= j.x0 && cx < j.x0 + TX_;
+    const int m = a.ssw;
+    j.inner = !j.src && j.x0 - HX >= m && j.x0 + TX_ + HX <= a.nx - m && j.z0 - HZ >= m && j.z0 + TZ_ + HZ <= a.nz - m &&
+              !(j.z0 + TZ_ > a.rec_z0 && j.z0 <= a.rec_z1);
+    return j;
+  }
+};
+
+// Programmatic dependent launch: the next step's kernel may be scheduled as soon as this one's CTAs leave,
+// and waits here, after its prologue, for this one's results.
+__device__ __forceinline__ void wait_for_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_step_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* m) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
+}
+
+// Bit 2 r + j: cell (zr + r, x + j) is a corner of the source.
+__device__ __forceinline__ unsigned source_bits(const SArgs& a, int shot, int zr, int x) {
+  unsigned m = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int d = __ldg(&a.st.src_cell[4 * shot + k]) - (zr * a.nx + x);
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+      const unsigned o = static_cast<unsigned>(d - r * a.nx);
+      if (o < 2u) m |= 1u << (2 * r + o);
+    }
+  }
+  return m;
+}
+
+// Issue the three copies of a job into stage buffer `st` with barrier `bar`.
+__device__ __forceinline__ void issue_fwd(const SArgs& a, const FwdMaps& m, float* st, uint64_t* bar, const Job& j,
+                                          int par) {
+  mbar_expect_tx(bar, FSTAGE_F * 4);
+  tma_load(st, &m.u, j.x0 - HX, j.z0 - HZ, par * a.units + j.unit, bar);
+  tma_load(st + BZ * BX, &m.p, j.x0, j.z0, (1 - par) * a.units + j.unit, bar);
+  tma_load(st + BZ * BX + TZ_ * TX_, &m.v, j.x0, j.z0, j.model, bar);
 }
 
 // Warp-specialised: warp 8 (one lane) streams the jobs' tiles into FST stages (waiting on each
@@ -178,6 +222,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // with one arrival per warp. No CTA-wide barrier per tile: consumer warps run up to FST tiles
 // apart. Every wait is bounded; a consumer that gives up records the error and leaves; the
 // producer that gives up records it and waits (bounded) for the copies it issued.
+// Decoding a job once per CTA, packed arithmetic (wave_packed.cuh) and the overlapped launch took a step of
+// 16 shots of the 844 x 344 grid from 38.5 to 31.5 us (storing terms) and from 36.2 to 30.9 (not). What
+// is left is latency: the C-PML tiles (43 % of them) wait on their strips' values in L2. Loading them
+// for all four rows ahead spills at 96 registers and measured slower (44 us).
 template <bool TRACES, bool STORE>
 __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid_constant__ FwdMaps maps,
                                                                     const __grid_constant__ SArgs a) {
@@ -185,12 +233,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
   float* stage = fsm_raw + ((128 - (smem_u32(fsm_raw) & 127)) & 127) / 4;  // [FST][U | P | V]
   uint64_t* full = reinterpret_cast<uint64_t*>(stage + FST * FSTAGE_F);
   uint64_t* empty = full + FST;
+  __shared__ Job info[FST];
   const int tid = threadIdx.x;
-  const int tiles = a.tiles_x * a.tiles_z;
-  const int jobs = a.units * tiles;
+  const int jobs = a.units * a.tiles_x * a.tiles_z;
   const int par = a.t & 1;
   const int nx = a.nx, nz = a.nz, ssw = a.ssw, region = a.region;
   const size_t cells = static_cast<size_t>(nx) * nz;
+  const Pk pk{make_float2(a.nz2[0], a.nz2[1])};
   if (tid == 0) {
     for (int k = 0; k < FST; ++k) {
       mbar_init(&full[k], 1);
@@ -198,11 +247,19 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (tid == NTH) {
+    prefetch_map(&maps.u);
+    prefetch_map(&maps.p);
+    prefetch_map(&maps.v);
+  }
   __syncthreads();
+  wait_for_previous_step();
+  let_next_step_launch();
   if (tid >= NTH) {  // producer warp
     if (tid == NTH) {
       int issued = 0;
-      for (int job = blockIdx.x; job < jobs; job += gridDim.x, ++issued) {
+      JobWalk walk(a);
+      for (int job = blockIdx.x; job < jobs; job += gridDim.x, ++issued, walk.advance(a)) {
         const int s = issued % FST;
         if (issued >= FST && !mbar_wait(&empty[s], (issued / FST - 1) & 1)) {
           report(a.status);
@@ -211,13 +268,18 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
           return;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        issue_fwd(a, maps, stage + s * FSTAGE_F, &full[s], job, par);
+        const Job j = walk.decode(a);
+        info[s] = j;  // released to the consumers by the arrival on the full barrier
+        issue_fwd(a, maps, stage + s * FSTAGE_F, &full[s], j, par);
       }
     }
     return;
   }
   const float f = __ldg(&a.wavelet[a.t]);
   const int pc = tid & 31, grp = tid >> 5;
+  const size_t xs_unit = static_cast<size_t>(nz) * 2 * ssw;  // floats per unit of an x strip array
+  const size_t zs_unit = static_cast<size_t>(2) * ssw * nx;
+  const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
   int job = blockIdx.x;
   for (int i = 0; job < jobs; ++i, job += gridDim.x) {
     const int s = i % FST;
@@ -225,52 +287,30 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
       report(a.status);
       return;
     }
-    const int unit = job / tiles, tile = job % tiles;
-    const int tzi = tile / a.tiles_x, txi = tile % a.tiles_x;
-    const int x0 = txi * TX_, z0 = tzi * TZ_;
-    const int shot = unit % a.shots;
-    const int x = x0 + 2 * pc;
-    const int zr = z0 + RPT * grp;
-    const bool xok = x >= FD_PAD && x + 1 < nx - FD_PAD;
-    const bool xpml = x < region || x + 1 >= nx - region;
-    float* Wn = a.W + (static_cast<size_t>(1 - par) * a.units + unit) * cells;
-    const float* Pt = stage + s * FSTAGE_F + BZ * BX;
-    const float* Vt = Pt + TZ_ * TX_;
-    float2 pv[RPT], vv[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      pv[r] = lds2(Pt + (RPT * grp + r) * TX_ + 2 * pc);
-      vv[r] = lds2(Vt + (RPT * grp + r) * TX_ + 2 * pc);
-    }
+    const Job j = info[s];
+    const int x = j.x0 + 2 * pc;
+    const int zr = j.z0 + RPT * grp;
+    float* Wn = a.W + (static_cast<size_t>(1 - par) * a.units + j.unit) * cells;
     const float* T = stage + s * FSTAGE_F;
-
-    if (interior_tile(a, x0, z0, a.st.src_cell + 4 * shot)) {
-      // interior tile: no frame, PML, receivers or sources
-      const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
-      float2 col[RPT + 4];
+    const float* Pt = T + BZ * BX + RPT * grp * TX_ + 2 * pc;
+    const float* Vt = Pt + TZ_ * TX_;
+    float* stp = STORE ? a.stored + (static_cast<size_t>(j.unit) * a.seg + (a.t - a.seg_t0)) * cells : nullptr;
+    float2 col[RPT + 4];
 #pragma unroll
-      for (int k = 0; k < RPT + 4; ++k) col[k] = lds2(T + (sz - 2 + k) * BX + sx);
-      float* stp = STORE ? a.stored + (static_cast<size_t>(unit) * a.seg + (a.t - a.seg_t0)) * cells : nullptr;
+    for (int k = 0; k < RPT + 4; ++k) col[k] = lds2(T + (sz - 2 + k) * BX + sx);
+
+    if (j.inner) {
+      // interior tile: no frame, PML, receivers or sources
 #pragma unroll
       for (int r = 0; r < RPT; ++r) {
         const int cell = (zr + r) * nx + x;
-        const float2 A = lds2(T + (sz + r) * BX + sx - 2);
-        const float2 B = lds2(T + (sz + r) * BX + sx + 2);
-        const float u0 = col[r + 2].x, u1 = col[r + 2].y;
-        const float2 zm2 = col[r], zm1 = col[r + 1], zp1 = col[r + 3], zp2 = col[r + 4];
-        const float d2x0 = (((F_D2A * u0 + F_D2B * (u1 + A.y)) - F_D2C * (B.x + A.x)) * a.d2a) * a.d2b;
-        const float d2x1 = (((F_D2A * u1 + F_D2B * (B.x + u0)) - F_D2C * (B.y + A.y)) * a.d2a) * a.d2b;
-        const float d2z0 = (((F_D2A * u0 + F_D2B * (zp1.x + zm1.x)) - F_D2C * (zp2.x + zm2.x)) * a.d2a) * a.d2b;
-        const float d2z1 = (((F_D2A * u1 + F_D2B * (zp1.y + zm1.y)) - F_D2C * (zp2.y + zm2.y)) * a.d2a) * a.d2b;
-        const float w0 = d2x0 + d2z0, w1 = d2x1 + d2z1;
-        const float2 v = vv[r];
-        const float v20 = (v.x * v.x) * a.dt2, v21 = (v.y * v.y) * a.dt2;
-        const float n0 = ((v20 * w0) + (2.0f * u0)) - pv[r].x;
-        const float n1 = ((v21 * w1) + (2.0f * u1)) - pv[r].y;
-        if (STORE)
-          __stcs(reinterpret_cast<float2*>(stp + cell),
-                 make_float2(((2.0f * v.x) * a.dt2) * w0, ((2.0f * v.y) * a.dt2) * w1));
-        st2(Wn + cell, n0, n1);
+        const float2 A = lds2(T + (sz + r) * BX + sx - 2), B = lds2(T + (sz + r) * BX + sx + 2), u = col[r + 2];
+        const float2 w = add2(pk.second(u, side_sum(A, u, B), add2(B, A), a.d2a, a.d2b),
+                              pk.second(u, add2(col[r + 3], col[r + 1]), add2(col[r + 4], col[r]), a.d2a, a.d2b));
+        const float2 v = lds2(Vt + r * TX_);
+        const float2 n = sub2(add2(pk.mul(scale2(a.dt2, mul2(v, v)), w), add2(u, u)), lds2(Pt + r * TX_));
+        if (STORE) __stcs(reinterpret_cast<float2*>(stp + cell), mul2(scale2(a.dt2, add2(v, v)), w));
+        *reinterpret_cast<float2*>(Wn + cell) = n;
       }
       __syncwarp();
       if (pc == 0) mbar_arrive(&empty[s]);
@@ -278,132 +318,96 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
     }
 
     if (TRACES) {
-      const int r0 = a.tile_rec_start[tile], r1 = a.tile_rec_start[tile + 1];
+      const int r0 = a.tile_rec_start[j.tile], r1 = a.tile_rec_start[j.tile + 1];
       for (int k = r0 + tid; k < r1; k += NTH) {
         const int r = a.tile_rec[k];
         float acc = 0.0f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int cell = a.st.rec_cell[4 * r + c];
-          const int cz = cell / nx - (z0 - HZ), cx = cell % nx - (x0 - HX);
+          const int cz = cell / nx - (j.z0 - HZ), cx = cell % nx - (j.x0 - HX);
           acc = acc + a.st.rec_w[4 * r + c] * T[cz * BX + cx];
         }
-        a.traces[(static_cast<size_t>(unit) * a.nt + a.t) * a.st.nrec + r] = acc;
+        a.traces[(static_cast<size_t>(j.unit) * a.nt + a.t) * a.st.nrec + r] = acc;
       }
     }
 
-    const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
-    float2 col[RPT + 4];
-#pragma unroll
-    for (int k = 0; k < RPT + 4; ++k) col[k] = lds2(T + (sz - 2 + k) * BX + sx);
-    const int* sc = a.st.src_cell + 4 * shot;
-    // bit 2 r + j: cell (zr + r, x + j) is a corner of this unit's source
-    unsigned srcm = 0;
-    {
-      const int base = zr * nx + x;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int d = __ldg(&sc[k]) - base;
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-          const unsigned o = static_cast<unsigned>(d - r * nx);
-          if (o < 2u) srcm |= 1u << (2 * r + o);
-        }
-      }
-    }
-    float* stp = STORE ? a.stored + (static_cast<size_t>(unit) * a.seg + (a.t - a.seg_t0)) * cells : nullptr;
-    float ax0 = 0.f, ax1 = 0.f, bx0 = 0.f, bx1 = 0.f, dbx0 = 0.f, dbx1 = 0.f;
+    const bool xok = x >= FD_PAD && x + 1 < nx - FD_PAD;
+    const bool xpml = x < region || x + 1 >= nx - region;
+    const unsigned srcm = j.src ? source_bits(a, j.shot, zr, x) : 0u;
+    float2 ax = make_float2(0.f, 0.f), bx = ax, dbx = ax;
     if (xok && xpml) {
-      const float2 pa = ldg2(a.prof + x), pb = ldg2(a.prof + nx + x), pd = ldg2(a.prof + 2 * nx + x);
-      ax0 = pa.x, ax1 = pa.y, bx0 = pb.x, bx1 = pb.y, dbx0 = pd.x, dbx1 = pd.y;
+      ax = ldg2(a.prof + x);
+      bx = ldg2(a.prof + nx + x);
+      dbx = ldg2(a.prof + 2 * nx + x);
     }
-    const float opbx0 = 1.0f + bx0, opbx1 = 1.0f + bx1;
-    const size_t xs_unit = static_cast<size_t>(nz) * 2 * ssw;  // floats per unit of an x strip array
-    const size_t zs_unit = static_cast<size_t>(2) * ssw * nx;
-    const float* PXc = a.PX + (static_cast<size_t>(par) * a.units + unit) * xs_unit;
-    float* PXn = a.PX + (static_cast<size_t>(1 - par) * a.units + unit) * xs_unit;
-    float* ZXo = a.ZX + static_cast<size_t>(unit) * xs_unit;
-    const float* PZc = a.PZ + (static_cast<size_t>(par) * a.units + unit) * zs_unit;
-    float* PZn = a.PZ + (static_cast<size_t>(1 - par) * a.units + unit) * zs_unit;
-    float* ZZo = a.ZZ + static_cast<size_t>(unit) * zs_unit;
+    const float2 opbx = make_float2(1.0f + bx.x, 1.0f + bx.y);
+    const float* PXc = a.PX + (static_cast<size_t>(par) * a.units + j.unit) * xs_unit;
+    float* PXn = a.PX + (static_cast<size_t>(1 - par) * a.units + j.unit) * xs_unit;
+    float* ZXo = a.ZX + static_cast<size_t>(j.unit) * xs_unit;
+    const float* PZc = a.PZ + (static_cast<size_t>(par) * a.units + j.unit) * zs_unit;
+    float* PZn = a.PZ + (static_cast<size_t>(1 - par) * a.units + j.unit) * zs_unit;
+    float* ZZo = a.ZZ + static_cast<size_t>(j.unit) * zs_unit;
     const int xc = xstrip(x, nx, ssw);
+    // the rows' stores go to other cells than the strips' loads: through restrict-qualified pointers the
+    // loads of a row may be issued ahead of the stores of the row before
+    auto rows = [&](float* __restrict__ wn, float* __restrict__ pxn, float* __restrict__ zxo, float* __restrict__ pzn,
+                    float* __restrict__ zzo, float* __restrict__ sto) {
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int z = zr + r;
-      if (!xok || z < FD_PAD || z >= nz - FD_PAD) continue;
-      const int cell = z * nx + x;
-      const float2 U = col[r + 2];
-      const float2 A = lds2(T + (sz + r) * BX + sx - 2);
-      const float2 B = lds2(T + (sz + r) * BX + sx + 2);
-      const float u0 = U.x, u1 = U.y;
-      const float d2x0 = (((F_D2A * u0 + F_D2B * (u1 + A.y)) - F_D2C * (B.x + A.x)) * a.d2a) * a.d2b;
-      const float d2x1 = (((F_D2A * u1 + F_D2B * (B.x + u0)) - F_D2C * (B.y + A.y)) * a.d2a) * a.d2b;
-      float w0, w1;
-      if (xpml) {
-        const float* row = PXc + z * 2 * ssw + xc;
-        const float2 P0 = ld2(row - 2), P1 = ld2(row), P2 = ld2(row + 2);
-        float* zrow = ZXo + z * 2 * ssw + xc;
-        const float2 Z = ld2(zrow);
-        const float d10 = ((F_D1A * (u1 - A.y)) - F_D1B * (B.x - A.x)) * a.rh;
-        const float d11 = ((F_D1A * (B.x - u0)) - F_D1B * (B.y - A.y)) * a.rh;
-        const float da0 = ((F_D1A * (P1.y - P0.y)) - F_D1B * (P2.x - P0.x)) * a.rh;
-        const float da1 = ((F_D1A * (P2.x - P1.x)) - F_D1B * (P2.y - P0.y)) * a.rh;
-        const float tmp0 = ((opbx0 * d2x0) + (dbx0 * d10)) + da0;
-        const float tmp1 = ((opbx1 * d2x1) + (dbx1 * d11)) + da1;
-        w0 = (opbx0 * tmp0) + (ax0 * Z.x);
-        w1 = (opbx1 * tmp1) + (ax1 * Z.y);
-        const float psi0 = (bx0 * d10) + P1.x;
-        const float psi1 = (bx1 * d11) + P1.y;
-        st2(zrow, (bx0 * tmp0) + (ax0 * Z.x), (bx1 * tmp1) + (ax1 * Z.y));
-        st2(PXn + z * 2 * ssw + xc, ax0 * psi0, ax1 * psi1);
-      } else {
-        w0 = d2x0;
-        w1 = d2x1;
-      }
-      const float2 zm2 = col[r], zm1 = col[r + 1], zp1 = col[r + 3], zp2 = col[r + 4];
-      const float d2z0 = (((F_D2A * u0 + F_D2B * (zp1.x + zm1.x)) - F_D2C * (zp2.x + zm2.x)) * a.d2a) * a.d2b;
-      const float d2z1 = (((F_D2A * u1 + F_D2B * (zp1.y + zm1.y)) - F_D2C * (zp2.y + zm2.y)) * a.d2a) * a.d2b;
-      if (z < region || z >= nz - region) {
-        const int zc = z < ssw ? z : z - (nz - 2 * ssw);
-        const float az = __ldg(&a.prof[3 * nx + z]), bz = __ldg(&a.prof[3 * nx + nz + z]),
-                    dbz = __ldg(&a.prof[3 * nx + 2 * nz + z]);
-        const float opbz = 1.0f + bz;
-        const float* q = PZc + zc * nx + x;
-        const float2 Qm2 = ld2(q - 2 * nx), Qm1 = ld2(q - nx), Q0 = ld2(q), Qp1 = ld2(q + nx), Qp2 = ld2(q + 2 * nx);
-        float* zz = ZZo + zc * nx + x;
-        const float2 Z = ld2(zz);
-        const float d10 = ((F_D1A * (zp1.x - zm1.x)) - F_D1B * (zp2.x - zm2.x)) * a.rh;
-        const float d11 = ((F_D1A * (zp1.y - zm1.y)) - F_D1B * (zp2.y - zm2.y)) * a.rh;
-        const float da0 = ((F_D1A * (Qp1.x - Qm1.x)) - F_D1B * (Qp2.x - Qm2.x)) * a.rh;
-        const float da1 = ((F_D1A * (Qp1.y - Qm1.y)) - F_D1B * (Qp2.y - Qm2.y)) * a.rh;
-        const float tmp0 = ((opbz * d2z0) + (dbz * d10)) + da0;
-        const float tmp1 = ((opbz * d2z1) + (dbz * d11)) + da1;
-        w0 = w0 + ((opbz * tmp0) + (az * Z.x));
-        w1 = w1 + ((opbz * tmp1) + (az * Z.y));
-        const float psi0 = (bz * d10) + Q0.x;
-        const float psi1 = (bz * d11) + Q0.y;
-        st2(zz, (bz * tmp0) + (az * Z.x), (bz * tmp1) + (az * Z.y));
-        st2(PZn + zc * nx + x, az * psi0, az * psi1);
-      } else {
-        w0 = w0 + d2z0;
-        w1 = w1 + d2z1;
-      }
-      const float2 v = vv[r];
-      const float v20 = (v.x * v.x) * a.dt2, v21 = (v.y * v.y) * a.dt2;
-      const float2 prev = pv[r];
-      float n0 = ((v20 * w0) + (2.0f * u0)) - prev.x;
-      float n1 = ((v21 * w1) + (2.0f * u1)) - prev.y;
-      if (STORE)
-        __stcs(reinterpret_cast<float2*>(stp + cell), make_float2(((2.0f * v.x) * a.dt2) * w0, ((2.0f * v.y) * a.dt2) * w1));
-      if (srcm & (3u << (2 * r))) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (cell == sc[k]) n0 = n0 + (((-v20) * a.st.src_w[4 * shot + k]) * f);
-          if (cell + 1 == sc[k]) n1 = n1 + (((-v21) * a.st.src_w[4 * shot + k]) * f);
+      for (int r = 0; r < RPT; ++r) {
+        const int z = zr + r;
+        if (!xok || z < FD_PAD || z >= nz - FD_PAD) continue;
+        const int cell = z * nx + x;
+        const float2 A = lds2(T + (sz + r) * BX + sx - 2), B = lds2(T + (sz + r) * BX + sx + 2), u = col[r + 2];
+        float2 w = pk.second(u, side_sum(A, u, B), add2(B, A), a.d2a, a.d2b);
+        if (xpml) {
+          const float* row = PXc + z * 2 * ssw + xc;
+          const float2 P0 = ld2(row - 2), P1 = ld2(row), P2 = ld2(row + 2);
+          const float2 Z = ld2(zxo + z * 2 * ssw + xc);
+          const float2 d1 = pk.first(side_diff(A, u, B), sub2(B, A), a.rh);
+          const float2 da = pk.first(side_diff(P0, P1, P2), sub2(P2, P0), a.rh);
+          const float2 tmp = add2(add2(pk.mul(opbx, w), pk.mul(dbx, d1)), da);
+          const float2 az = pk.mul(ax, Z);
+          w = add2(pk.mul(opbx, tmp), az);
+          *reinterpret_cast<float2*>(zxo + z * 2 * ssw + xc) = add2(pk.mul(bx, tmp), az);
+          *reinterpret_cast<float2*>(pxn + z * 2 * ssw + xc) = mul2(ax, add2(pk.mul(bx, d1), P1));
         }
+        const float2 zm2 = col[r], zm1 = col[r + 1], zp1 = col[r + 3], zp2 = col[r + 4];
+        const float2 d2z = pk.second(u, add2(zp1, zm1), add2(zp2, zm2), a.d2a, a.d2b);
+        if (z < region || z >= nz - region) {
+          const int zc = z < ssw ? z : z - (nz - 2 * ssw);
+          const float az = __ldg(&a.prof[3 * nx + z]), bz = __ldg(&a.prof[3 * nx + nz + z]),
+                      dbz = __ldg(&a.prof[3 * nx + 2 * nz + z]);
+          const float opbz = 1.0f + bz;
+          const float* q = PZc + zc * nx + x;
+          const float2 Qm2 = ld2(q - 2 * nx), Qm1 = ld2(q - nx), Q0 = ld2(q), Qp1 = ld2(q + nx), Qp2 = ld2(q + 2 * nx);
+          const float2 Z = ld2(zzo + zc * nx + x);
+          const float2 d1 = pk.first(sub2(zp1, zm1), sub2(zp2, zm2), a.rh);
+          const float2 da = pk.first(sub2(Qp1, Qm1), sub2(Qp2, Qm2), a.rh);
+          const float2 tmp = add2(add2(pk.scale(opbz, d2z), pk.scale(dbz, d1)), da);
+          const float2 aZ = pk.scale(az, Z);
+          w = add2(w, add2(pk.scale(opbz, tmp), aZ));
+          *reinterpret_cast<float2*>(zzo + zc * nx + x) = add2(pk.scale(bz, tmp), aZ);
+          *reinterpret_cast<float2*>(pzn + zc * nx + x) = scale2(az, add2(pk.scale(bz, d1), Q0));
+        } else {
+          w = add2(w, d2z);
+        }
+        const float2 v = lds2(Vt + r * TX_);
+        const float2 v2 = scale2(a.dt2, mul2(v, v));
+        float2 n = sub2(add2(pk.mul(v2, w), add2(u, u)), lds2(Pt + r * TX_));
+        if (STORE) __stcs(reinterpret_cast<float2*>(sto + cell), mul2(scale2(a.dt2, add2(v, v)), w));
+        if (srcm & (3u << (2 * r))) {
+          const int* sc = a.st.src_cell + 4 * j.shot;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (cell == sc[k]) n.x = n.x + (((-v2.x) * a.st.src_w[4 * j.shot + k]) * f);
+            if (cell + 1 == sc[k]) n.y = n.y + (((-v2.y) * a.st.src_w[4 * j.shot + k]) * f);
+          }
+        }
+        *reinterpret_cast<float2*>(wn + cell) = n;
       }
-      st2(Wn + cell, n0, n1);
-    }
+    };
+    rows(Wn, PXn, ZXo, PZn, ZZo, stp);
     __syncwarp();
     if (pc == 0) mbar_arrive(&empty[s]);  // this warp is done with the stage
   }
@@ -420,17 +424,16 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
 // bit for bit (sources are injected into halo copies too; receivers are recorded by the tile that
 // holds their first corner). Per step the wavefield crosses HBM once per TB_T steps instead of once
 // per step. The state is read from one set and written to the other (sets alternate per launch),
-// so no CTA overwrites cells a neighbouring CTA still has to read. Off by default (engine option
-// "temporal_block"): the per-step forward is latency-bound rather than bandwidth-bound, so the
-// saved traffic buys nothing, and the redundant halo updates (31 % of the work) make this kernel
-// slower on the 800 x 300 survey.
+// so no CTA overwrites cells a neighbouring CTA still has to read. Faster than one step per launch where a
+// step is mostly latency (see blocked()); on large surveys the redundant halo updates (31 % of the
+// work) make it slower (41 against 31 us a step for 16 shots of the 844 x 344 grid).
 // ------------------------------------------------------------------------------------------------
 constexpr int TB_T = 4;                      // time steps per launch
 constexpr int TB_H = 2 * TB_T;               // halo per side
 constexpr int TB_RX = TX_ + 2 * TB_H;        // 80 region columns (x offset 64 k - 8: 16-byte aligned)
 constexpr int TB_RZ = TZ_ + 2 * TB_H;        // 48 region rows
 constexpr int TB_N = TB_RX * TB_RZ;          // cells of a region
-constexpr int TB_THREADS = 512;
+constexpr int TB_THREADS = 1024;
 constexpr int TB_STAGE = 3 * TB_N;           // floats per stage: u(t) | u(t-1) | v
 constexpr size_t kTbSmem = static_cast<size_t>(2 * TB_STAGE + 6 * TB_N) * 4 + 2 * 8 + 128;
 
@@ -467,12 +470,17 @@ __global__ void __launch_bounds__(TB_THREADS, 1) fwd_tb_kernel(const __grid_cons
   const size_t cells = static_cast<size_t>(nx) * nz;
   const size_t xs_unit = static_cast<size_t>(nz) * 2 * ssw, zs_unit = static_cast<size_t>(2) * ssw * nx;
   const int set_out = 1 - p.set_in;
+  const Pk pk{make_float2(a.nz2[0], a.nz2[1])};
   if (tid == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    prefetch_map(&umap);
+    prefetch_map(&vmap);
   }
   __syncthreads();
+  wait_for_previous_step();
+  let_next_step_launch();
   auto issue = [&](int job, int s) {
     const int unit = job / tiles, tile = job % tiles;
     const int x = (tile % a.tiles_x) * TX_ - TB_H, z = (tile / a.tiles_x) * TZ_ - TB_H;
@@ -512,34 +520,48 @@ __global__ void __launch_bounds__(TB_THREADS, 1) fwd_tb_kernel(const __grid_cons
       const float* ZXi = p.ZX + (static_cast<size_t>(p.set_in) * a.units + unit) * xs_unit;
       const float* PZi = p.PZ + (static_cast<size_t>(p.set_in) * a.units + unit) * zs_unit;
       const float* ZZi = p.ZZ + (static_cast<size_t>(p.set_in) * a.units + unit) * zs_unit;
-      for (int c = tid; c < TB_N; c += TB_THREADS) {
+      // pairs of columns (a pair lies in a strip or outside it: nx and ssw are even), loaded ahead of
+      // their stores
+      constexpr int PER = (TB_N / 2 + TB_THREADS - 1) / TB_THREADS;
+      float2 px[PER], zx[PER], pz[PER], zz[PER];
+#pragma unroll
+      for (int it = 0; it < PER; ++it) {
+        const int c = 2 * (tid + it * TB_THREADS);
         const int z = rz0 + c / TB_RX, x = rx0 + c % TB_RX;
-        float px = 0.f, zx = 0.f, pz = 0.f, zz = 0.f;
-        if (x >= 0 && x < nx && z >= 0 && z < nz) {
+        px[it] = zx[it] = pz[it] = zz[it] = make_float2(0.f, 0.f);
+        if (c < TB_N && x >= 0 && x < nx && z >= 0 && z < nz) {
           if (x < ssw || x >= nx - ssw) {
             const int k = z * 2 * ssw + xstrip(x, nx, ssw);
-            px = PXi[k];
-            zx = ZXi[k];
+            px[it] = ld2(PXi + k);
+            zx[it] = ld2(ZXi + k);
           }
           if (z < ssw || z >= nz - ssw) {
             const int k = (z < ssw ? z : z - (nz - 2 * ssw)) * nx + x;
-            pz = PZi[k];
-            zz = ZZi[k];
+            pz[it] = ld2(PZi + k);
+            zz[it] = ld2(ZZi + k);
           }
         }
+      }
+#pragma unroll
+      for (int it = 0; it < PER; ++it) {
+        const int c = 2 * (tid + it * TB_THREADS);
+        if (c >= TB_N) break;
         // both buffers: a*psi of strip cells outside the C-PML region is never updated
-        PXA[c] = px;
-        PXB[c] = px;
-        ZXr[c] = zx;
-        PZA[c] = pz;
-        PZB[c] = pz;
-        ZZr[c] = zz;
+        put2(PXA + c, px[it]);
+        put2(PXB + c, px[it]);
+        put2(ZXr + c, zx[it]);
+        put2(PZA + c, pz[it]);
+        put2(PZB + c, pz[it]);
+        put2(ZZr + c, zz[it]);
       }
       __syncthreads();
     }
     const int* sc = a.st.src_cell + 4 * shot;
     const float* sw = a.st.src_w + 4 * shot;
     const int sc0 = __ldg(&sc[0]), sc1 = __ldg(&sc[1]), sc2 = __ldg(&sc[2]), sc3 = __ldg(&sc[3]);
+    // the source's 2 x 2 corners against the region
+    const int srz = sc0 / nx - rz0, srx = sc0 % nx - rx0;
+    const bool src_near = srz >= -1 && srz < TB_RZ && srx >= -1 && srx < TB_RX;
     for (int k = 0; k < p.nsub; ++k) {
       const int t = a.t + k;
       const float f = __ldg(&a.wavelet[t]);
@@ -565,87 +587,67 @@ __global__ void __launch_bounds__(TB_THREADS, 1) fwd_tb_kernel(const __grid_cons
       float* stp = STORE ? a.stored + (static_cast<size_t>(unit) * a.seg + (t - a.seg_t0)) * cells : nullptr;
       const int m = 2 * (k + 1);  // region of step k: 2 (k + 1) cells inside the loaded one
       const int pairs = (TB_RX - 2 * m) / 2, rows = TB_RZ - 2 * m;
+      // idx / pairs for idx < pairs rows <= 1672 and 32 <= pairs <= 38: the reciprocal's error, under
+      // pairs / 2^16 per unit, stays below one
+      const int inv = (65536 + pairs - 1) / pairs;
       for (int idx = tid; idx < pairs * rows; idx += TB_THREADS) {
-        const int lz = m + idx / pairs, lx = m + 2 * (idx % pairs);
+        const int qz = (idx * inv) >> 16;
+        const int lz = m + qz, lx = m + 2 * (idx - qz * pairs);
         const int z = rz0 + lz, x = rx0 + lx;
         if (z < FD_PAD || z >= nz - FD_PAD || x < FD_PAD || x + 1 >= nx - FD_PAD) continue;
         const int c = lz * TB_RX + lx;
         const int cell = z * nx + x;
-        const float2 U0 = lds2(Uc + c);
-        const float2 A = lds2(Uc + c - 2);
-        const float2 B = lds2(Uc + c + 2);
-        const float u0 = U0.x, u1 = U0.y;
-        const float d2x0 = (((F_D2A * u0 + F_D2B * (u1 + A.y)) - F_D2C * (B.x + A.x)) * a.d2a) * a.d2b;
-        const float d2x1 = (((F_D2A * u1 + F_D2B * (B.x + u0)) - F_D2C * (B.y + A.y)) * a.d2a) * a.d2b;
-        float w0, w1;
-        if (x < region || x + 1 >= nx - region) {
-          const float2 pa = ldg2(a.prof + x), pb = ldg2(a.prof + nx + x), pd = ldg2(a.prof + 2 * nx + x);
-          const float ax0 = pa.x, ax1 = pa.y, bx0 = pb.x, bx1 = pb.y, dbx0 = pd.x, dbx1 = pd.y;
-          const float opbx0 = 1.0f + bx0, opbx1 = 1.0f + bx1;
+        const float2 u = lds2(Uc + c), A = lds2(Uc + c - 2), B = lds2(Uc + c + 2);
+        float2 w = pk.second(u, side_sum(A, u, B), add2(B, A), a.d2a, a.d2b);
+        if (pml_tile && (x < region || x + 1 >= nx - region)) {
+          const float2 ax = ldg2(a.prof + x), bx = ldg2(a.prof + nx + x), dbx = ldg2(a.prof + 2 * nx + x);
+          const float2 opbx = make_float2(1.0f + bx.x, 1.0f + bx.y);
           const float2 P0 = lds2(Pc + c - 2), P1 = lds2(Pc + c), P2 = lds2(Pc + c + 2);
           const float2 Z = lds2(ZXr + c);
-          const float d10 = ((F_D1A * (u1 - A.y)) - F_D1B * (B.x - A.x)) * a.rh;
-          const float d11 = ((F_D1A * (B.x - u0)) - F_D1B * (B.y - A.y)) * a.rh;
-          const float da0 = ((F_D1A * (P1.y - P0.y)) - F_D1B * (P2.x - P0.x)) * a.rh;
-          const float da1 = ((F_D1A * (P2.x - P1.x)) - F_D1B * (P2.y - P0.y)) * a.rh;
-          const float tmp0 = ((opbx0 * d2x0) + (dbx0 * d10)) + da0;
-          const float tmp1 = ((opbx1 * d2x1) + (dbx1 * d11)) + da1;
-          w0 = (opbx0 * tmp0) + (ax0 * Z.x);
-          w1 = (opbx1 * tmp1) + (ax1 * Z.y);
-          const float psi0 = (bx0 * d10) + P1.x;
-          const float psi1 = (bx1 * d11) + P1.y;
-          st2(ZXr + c, (bx0 * tmp0) + (ax0 * Z.x), (bx1 * tmp1) + (ax1 * Z.y));
-          st2(Pn + c, ax0 * psi0, ax1 * psi1);
-        } else {
-          w0 = d2x0;
-          w1 = d2x1;
+          const float2 d1 = pk.first(side_diff(A, u, B), sub2(B, A), a.rh);
+          const float2 da = pk.first(side_diff(P0, P1, P2), sub2(P2, P0), a.rh);
+          const float2 tmp = add2(add2(pk.mul(opbx, w), pk.mul(dbx, d1)), da);
+          const float2 az = pk.mul(ax, Z);
+          w = add2(pk.mul(opbx, tmp), az);
+          put2(ZXr + c, add2(pk.mul(bx, tmp), az));
+          put2(Pn + c, mul2(ax, add2(pk.mul(bx, d1), P1)));
         }
         const float2 zm2 = lds2(Uc + c - 2 * TB_RX), zm1 = lds2(Uc + c - TB_RX), zp1 = lds2(Uc + c + TB_RX),
                      zp2 = lds2(Uc + c + 2 * TB_RX);
-        const float d2z0 = (((F_D2A * u0 + F_D2B * (zp1.x + zm1.x)) - F_D2C * (zp2.x + zm2.x)) * a.d2a) * a.d2b;
-        const float d2z1 = (((F_D2A * u1 + F_D2B * (zp1.y + zm1.y)) - F_D2C * (zp2.y + zm2.y)) * a.d2a) * a.d2b;
-        if (z < region || z >= nz - region) {
+        const float2 d2z = pk.second(u, add2(zp1, zm1), add2(zp2, zm2), a.d2a, a.d2b);
+        if (pml_tile && (z < region || z >= nz - region)) {
           const float az = __ldg(&a.prof[3 * nx + z]), bz = __ldg(&a.prof[3 * nx + nz + z]),
                       dbz = __ldg(&a.prof[3 * nx + 2 * nz + z]);
           const float opbz = 1.0f + bz;
           const float2 Qm2 = lds2(Qc + c - 2 * TB_RX), Qm1 = lds2(Qc + c - TB_RX), Q0 = lds2(Qc + c),
                        Qp1 = lds2(Qc + c + TB_RX), Qp2 = lds2(Qc + c + 2 * TB_RX);
           const float2 Z = lds2(ZZr + c);
-          const float d10 = ((F_D1A * (zp1.x - zm1.x)) - F_D1B * (zp2.x - zm2.x)) * a.rh;
-          const float d11 = ((F_D1A * (zp1.y - zm1.y)) - F_D1B * (zp2.y - zm2.y)) * a.rh;
-          const float da0 = ((F_D1A * (Qp1.x - Qm1.x)) - F_D1B * (Qp2.x - Qm2.x)) * a.rh;
-          const float da1 = ((F_D1A * (Qp1.y - Qm1.y)) - F_D1B * (Qp2.y - Qm2.y)) * a.rh;
-          const float tmp0 = ((opbz * d2z0) + (dbz * d10)) + da0;
-          const float tmp1 = ((opbz * d2z1) + (dbz * d11)) + da1;
-          w0 = w0 + ((opbz * tmp0) + (az * Z.x));
-          w1 = w1 + ((opbz * tmp1) + (az * Z.y));
-          const float psi0 = (bz * d10) + Q0.x;
-          const float psi1 = (bz * d11) + Q0.y;
-          st2(ZZr + c, (bz * tmp0) + (az * Z.x), (bz * tmp1) + (az * Z.y));
-          st2(Qn + c, az * psi0, az * psi1);
+          const float2 d1 = pk.first(sub2(zp1, zm1), sub2(zp2, zm2), a.rh);
+          const float2 da = pk.first(sub2(Qp1, Qm1), sub2(Qp2, Qm2), a.rh);
+          const float2 tmp = add2(add2(pk.scale(opbz, d2z), pk.scale(dbz, d1)), da);
+          const float2 aZ = pk.scale(az, Z);
+          w = add2(w, add2(pk.scale(opbz, tmp), aZ));
+          put2(ZZr + c, add2(pk.scale(bz, tmp), aZ));
+          put2(Qn + c, scale2(az, add2(pk.scale(bz, d1), Q0)));
         } else {
-          w0 = w0 + d2z0;
-          w1 = w1 + d2z1;
+          w = add2(w, d2z);
         }
         const float2 v = lds2(V + c);
-        const float v20 = (v.x * v.x) * a.dt2, v21 = (v.y * v.y) * a.dt2;
-        const float2 prev = lds2(Un + c);
-        float n0 = ((v20 * w0) + (2.0f * u0)) - prev.x;
-        float n1 = ((v21 * w1) + (2.0f * u1)) - prev.y;
+        const float2 v2 = scale2(a.dt2, mul2(v, v));
+        float2 n = sub2(add2(pk.mul(v2, w), add2(u, u)), lds2(Un + c));
         if (STORE && lz >= TB_H && lz < TB_H + TZ_ && lx >= TB_H && lx < TB_H + TX_)
-          __stcs(reinterpret_cast<float2*>(stp + cell),
-                 make_float2(((2.0f * v.x) * a.dt2) * w0, ((2.0f * v.y) * a.dt2) * w1));
+          __stcs(reinterpret_cast<float2*>(stp + cell), mul2(scale2(a.dt2, add2(v, v)), w));
         // sources: corners in the halo are injected too, so that halo copies match their owners
-        if (cell == sc0 || cell + 1 == sc0 || cell == sc1 || cell + 1 == sc1 || cell == sc2 || cell + 1 == sc2 ||
-            cell == sc3 || cell + 1 == sc3) {
+        if (src_near && (cell == sc0 || cell + 1 == sc0 || cell == sc1 || cell + 1 == sc1 || cell == sc2 ||
+                         cell + 1 == sc2 || cell == sc3 || cell + 1 == sc3)) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int scq = q == 0 ? sc0 : q == 1 ? sc1 : q == 2 ? sc2 : sc3;
-            if (cell == scq) n0 = n0 + (((-v20) * __ldg(&sw[q])) * f);
-            if (cell + 1 == scq) n1 = n1 + (((-v21) * __ldg(&sw[q])) * f);
+            if (cell == scq) n.x = n.x + (((-v2.x) * __ldg(&sw[q])) * f);
+            if (cell + 1 == scq) n.y = n.y + (((-v2.y) * __ldg(&sw[q])) * f);
           }
         }
-        st2(Un + c, n0, n1);
+        put2(Un + c, n);
       }
       __syncthreads();
     }
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) fwd_tb_kernel(const __grid_cons
 // Derived terms v^2 dt^2 lambda (VS) and, in the PML strips, T = (1+b) VS + b zeta and
 // U1 = db T + b psi are formed once per tile cell (halo included) in shared memory.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__ CUtensorMap map,
+__global__ void __launch_bounds__(NTH, 2) adj_stream_kernel(const __grid_constant__ CUtensorMap map,
                                                          const __grid_constant__ SArgs a) {
   extern __shared__ __align__(128) float dsm_raw[];
   // TMA destinations start on a 128-byte boundary
@@ -710,22 +712,34 @@ __global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__
   float* U1Zs = TZs + BZ * BX;
   uint64_t* bar = reinterpret_cast<uint64_t*>(U1Zs + BZ * BX);
   const int tid = threadIdx.x;
-  const int tiles = a.tiles_x * a.tiles_z;
-  const int jobs = a.units * tiles;
+  __shared__ Job info[2];
+  const int jobs = a.units * a.tiles_x * a.tiles_z;
+  const Pk pk{make_float2(a.nz2[0], a.nz2[1])};
   const int q = a.t & 1;  // lambda(t) in buffer q; lambda(t-1) is written into buffer 1 - q
   const int nx = a.nx, nz = a.nz, ssw = a.ssw, region = a.region;
   const size_t cells = static_cast<size_t>(nx) * nz;
   const size_t xs_unit = static_cast<size_t>(nz) * 2 * ssw;
   const size_t zs_unit = static_cast<size_t>(2) * ssw * nx;
-  Pipe pipe{bar, stage};
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    prefetch_map(&map);
   }
-  __syncthreads();
+  wait_for_previous_step();
+  let_next_step_launch();
+  // thread 0 decodes each job and issues its tile's copy, one job ahead
+  JobWalk walk(a);
+  auto issue = [&](int s) {
+    const Job j = walk.decode(a);
+    info[s] = j;
+    mbar_expect_tx(&bar[s], kTileBytes);
+    tma_load(stage + s * BZ * BX, &map, j.x0 - HX, j.z0 - HZ, q * a.units + j.unit, &bar[s]);
+    walk.advance(a);
+  };
   int job = blockIdx.x;
-  if (tid == 0 && job < jobs) issue(a, &map, pipe, job, 0, q);
+  if (tid == 0 && job < jobs) issue(0);
+  __syncthreads();
   const float f = __ldg(&a.wavelet[a.t]);
   const float* sAX = a.prof;
   const float* sBX = a.prof + nx;
@@ -734,21 +748,22 @@ __global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__
   const float* sBZ = sAZ + nz;
   const float* sDBZ = sBZ + nz;
   const int pc = tid & 31, grp = tid >> 5;
-  constexpr int DER = (BZ * (BX / 2) + NTH - 1) / NTH;  // derive pairs per thread
+  // Halo pair of this thread (192 of the 256 threads): rows 0, 1, 34, 35 of the tile's 32 inner pairs, then
+  // pairs 1 and 34 of its 32 inner rows. The stencils are axis-parallel: no corner is needed, and the
+  // rows need the z strips' terms only, the columns the x strips' only.
+  const bool hrow = tid < 4 * 32, hcol = !hrow && tid < 4 * 32 + 2 * TZ_;
+  const int hk = hrow ? (tid / 32 < 2 ? tid / 32 : BZ - 4 + tid / 32) : HZ + (tid - 4 * 32) / 2;
+  const int hj = hrow ? HX / 2 + tid % 32 : ((tid & 1) ? BX / 2 - 2 : 1);
   for (int i = 0; job < jobs; ++i, job += gridDim.x) {
     const int s = i & 1;
     const int nxt = job + gridDim.x;
     if (tid == 0 && nxt < jobs) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      issue(a, &map, pipe, nxt, s ^ 1, q);
+      issue(s ^ 1);
     }
-    const int unit = job / tiles, tile = job % tiles;
-    const int tzi = tile / a.tiles_x, txi = tile % a.tiles_x;
-    const int x0 = txi * TX_, z0 = tzi * TZ_;
-    const int model = unit / a.shots, shot = unit % a.shots;
+    const Job j = info[s];
+    const int unit = j.unit, x0 = j.x0, z0 = j.z0, model = j.model, shot = j.shot;
     const float* vel = a.vel + static_cast<size_t>(model) * cells;
-    const bool xtile = x0 - 2 < region + 3 || x0 + TX_ + 2 > nx - region - 3;
-    const bool ztile = z0 - 2 < region + 2 || z0 + TZ_ + 2 > nz - region - 2;
     const float* LPXc = a.PX + (static_cast<size_t>(q) * a.units + unit) * xs_unit;
     const float* LZXc = a.ZX + (static_cast<size_t>(q) * a.units + unit) * xs_unit;
     const float* LPZc = a.PZ + (static_cast<size_t>(q) * a.units + unit) * zs_unit;
@@ -759,18 +774,19 @@ __global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__
     float* Ln = a.W + (static_cast<size_t>(1 - q) * a.units + unit) * cells;
     const float* st_t = a.stored + (static_cast<size_t>(unit) * a.seg + (a.t - a.seg_t0)) * cells;
     float* gacc = a.gacc + static_cast<size_t>(unit) * cells;
-    // inputs that do not depend on the tile copy, requested before it is waited for: the
-    // velocity of the derive pairs, and per own cell lambda_prev, the stored term, the gradient
-    float2 vd[DER];
-#pragma unroll
-    for (int d = 0; d < DER; ++d) {
-      const int e = tid + d * NTH;
-      const int k = e / (BX / 2), j = e % (BX / 2);
-      const int z = z0 - HZ + k, xx = x0 - HX + 2 * j;
-      const bool in = e < BZ * (BX / 2) && z >= 0 && z < nz && xx >= 0 && xx < nx;
-      vd[d] = in ? ldg2(vel + static_cast<size_t>(z) * nx + xx) : make_float2(0.f, 0.f);
-    }
-    float2 lpv[RPT], stv[RPT], gav[RPT];
+    const bool inner = j.inner;
+    const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
+
+    // Everything that does not depend on the tile copy is requested before it is waited for: per own
+    // cell the velocity, lambda_prev, the stored term, the gradient and the strips' psi and zeta, and
+    // the halo pair's. (Read between the rows' stores, each strip value cost an L2 latency; with the
+    // overlapped launch, packed arithmetic and one barrier less a step of 16 shots of the 844 x 344
+    // grid went from 62 to 51.6 us, one of 10 shots of 344 x 194 from 18.3 to 14.4.)
+    float2 vv[RPT], lpv[RPT], stv[RPT], gav[RPT], xP[RPT], xZ[RPT], zP[RPT], zZ[RPT];
+    float2 hv = make_float2(0.f, 0.f), hP = hv, hZ = hv;
+    const bool in_x = x < nx;                                     // own pair inside the grid (nx is even)
+    const bool xs = !inner && in_x && (x < ssw || x >= nx - ssw);  // in an x strip
+    const int xc = xstrip(x, nx, ssw);
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int z = zr + r;
@@ -779,150 +795,156 @@ __global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__
       lpv[r] = ld2(Ln + cell);
       stv[r] = __ldcs(reinterpret_cast<const float2*>(st_t + cell));
       gav[r] = ld2(gacc + cell);
+      vv[r] = in_x && z < nz ? ldg2(vel + static_cast<size_t>(z) * nx + x) : make_float2(0.f, 0.f);
+      if (xs && z < nz) {
+        xP[r] = ld2(LPXc + static_cast<size_t>(z) * 2 * ssw + xc);
+        xZ[r] = ld2(LZXc + static_cast<size_t>(z) * 2 * ssw + xc);
+      }
+      if (!inner && in_x && z < nz && (z < ssw || z >= nz - ssw)) {
+        const int zc = z < ssw ? z : z - (nz - 2 * ssw);
+        zP[r] = ld2(LPZc + static_cast<size_t>(zc) * nx + x);
+        zZ[r] = ld2(LZZc + static_cast<size_t>(zc) * nx + x);
+      }
     }
-    // a wait that runs out (the copy never completed) ends the kernel in every thread together,
-    // after thread 0 has waited, again bounded, for the copy it issued for the next tile
-    if (__syncthreads_or(mbar_wait(&bar[s], (i >> 1) & 1) ? 0 : 1)) {
+    const int hz = z0 - HZ + hk, hx = x0 - HX + 2 * hj;
+    const bool hin = (hrow || hcol) && hz >= 0 && hz < nz && hx >= 0 && hx < nx;
+    const bool hxs = !inner && hcol && hin && (hx < ssw || hx >= nx - ssw);
+    const bool hzs = !inner && hrow && hin && (hz < ssw || hz >= nz - ssw);
+    if (hin) hv = ldg2(vel + static_cast<size_t>(hz) * nx + hx);
+    if (hxs) {
+      const size_t o = static_cast<size_t>(hz) * 2 * ssw + xstrip(hx, nx, ssw);
+      hP = ld2(LPXc + o);
+      hZ = ld2(LZXc + o);
+    }
+    if (hzs) {
+      const size_t o = static_cast<size_t>(hz < ssw ? hz : hz - (nz - 2 * ssw)) * nx + hx;
+      hP = ld2(LPZc + o);
+      hZ = ld2(LZZc + o);
+    }
+    // a wait that runs out (the copy never completed) ends the kernel in every thread together, at
+    // the barrier below
+    const bool arrived = mbar_wait(&bar[s], (i >> 1) & 1);
+    const float* L = stage + s * BZ * BX;
+
+    // derived terms of the own cells and of the halo pair
+    const float2 xb = xs ? ldg2(sBX + x) : make_float2(0.f, 0.f), xdb = xs ? ldg2(sDBX + x) : make_float2(0.f, 0.f);
+    const float2 opxb = make_float2(1.0f + xb.x, 1.0f + xb.y);
+    float2 vs[RPT];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+      const int z = zr + r;
+      const int o = (sz + r) * BX + sx;
+      const float2 l = lds2(L + o);
+      const bool in = in_x && z < nz;
+      vs[r] = in ? mul2(scale2(a.dt2, mul2(vv[r], vv[r])), l) : make_float2(0.f, 0.f);
+      put2(VS + o, vs[r]);
+      if (xs && z < nz) {
+        const float2 T = add2(pk.mul(opxb, vs[r]), pk.mul(xb, xZ[r]));
+        put2(TXs + o, T);
+        put2(U1Xs + o, add2(pk.mul(xdb, T), pk.mul(xb, xP[r])));
+      }
+      if (!inner && in && (z < ssw || z >= nz - ssw)) {
+        const float bz = __ldg(&sBZ[z]), dbz = __ldg(&sDBZ[z]);
+        const float2 T = add2(pk.scale(1.0f + bz, vs[r]), pk.scale(bz, zZ[r]));
+        put2(TZs + o, T);
+        put2(U1Zs + o, add2(pk.scale(dbz, T), pk.scale(bz, zP[r])));
+      }
+    }
+    if (hrow || hcol) {
+      const int o = hk * BX + 2 * hj;
+      const float2 l = lds2(L + o);
+      const float v0 = hin ? ((hv.x * hv.x) * a.dt2) * l.x : 0.0f, v1 = hin ? ((hv.y * hv.y) * a.dt2) * l.y : 0.0f;
+      st2(VS + o, v0, v1);
+      if (hxs) {
+        const float2 b = ldg2(sBX + hx), db = ldg2(sDBX + hx);
+        const float T0 = ((1.0f + b.x) * v0) + (b.x * hZ.x);
+        const float T1 = ((1.0f + b.y) * v1) + (b.y * hZ.y);
+        st2(TXs + o, T0, T1);
+        st2(U1Xs + o, (db.x * T0) + (b.x * hP.x), (db.y * T1) + (b.y * hP.y));
+      }
+      if (hzs) {
+        const float bz = __ldg(&sBZ[hz]), dbz = __ldg(&sDBZ[hz]);
+        const float opbz = 1.0f + bz;
+        const float T0 = (opbz * v0) + (bz * hZ.x);
+        const float T1 = (opbz * v1) + (bz * hZ.y);
+        st2(TZs + o, T0, T1);
+        st2(U1Zs + o, (dbz * T0) + (bz * hP.x), (dbz * T1) + (bz * hP.y));
+      }
+    }
+    if (__syncthreads_or(!arrived)) {
       if (tid == 0) {
         report(a.status);
         if (nxt < jobs) mbar_wait(&bar[s ^ 1], ((i + 1) >> 1) & 1);
       }
       return;
     }
-    const float* L = stage + s * BZ * BX;
 
-    if (interior_tile(a, x0, z0, a.st.src_cell + 4 * shot)) {
-      // interior tile: VS over the tile and halo, then the interior update
-#pragma unroll
-      for (int d = 0; d < DER; ++d) {
-        const int e = tid + d * NTH;
-        if (e >= BZ * (BX / 2)) break;
-        const int o = (e / (BX / 2)) * BX + 2 * (e % (BX / 2));
-        const float2 l = lds2(L + o);
-        st2(VS + o, ((vd[d].x * vd[d].x) * a.dt2) * l.x, ((vd[d].y * vd[d].y) * a.dt2) * l.y);
-      }
-      __syncthreads();
-      const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
+    if (inner) {
       float* Lnf = a.W + (static_cast<size_t>(1 - q) * a.units + unit) * cells;
       float* gf = a.gacc + static_cast<size_t>(unit) * cells;
+      // rows around the own four; the own ones are in registers
+      const int so = sz * BX + sx;
+      const float2 up2 = lds2(VS + so - 2 * BX), up1 = lds2(VS + so - BX), dn1 = lds2(VS + so + RPT * BX),
+                   dn2 = lds2(VS + so + (RPT + 1) * BX);
 #pragma unroll
       for (int r = 0; r < RPT; ++r) {
         const int cell = (zr + r) * nx + x;
-        const int so = (sz + r) * BX + sx;
-        const float2 Vb = lds2(VS + so), Va = lds2(VS + so - 2), Vc = lds2(VS + so + 2);
-        const float2 Vm2 = lds2(VS + so - 2 * BX), Vm1 = lds2(VS + so - BX), Vp1 = lds2(VS + so + BX),
-                     Vp2 = lds2(VS + so + 2 * BX);
-        float w0 = ((((F_D2A * Vb.x) + (F_D2B * (Vb.y + Va.y))) + (A_D2C * (Vc.x + Va.x))) * a.rh) * a.rh;
-        float w1 = ((((F_D2A * Vb.y) + (F_D2B * (Vc.x + Vb.x))) + (A_D2C * (Vc.y + Va.y))) * a.rh) * a.rh;
-        w0 = w0 + ((((F_D2A * Vb.x) + (F_D2B * (Vp1.x + Vm1.x))) + (A_D2C * (Vp2.x + Vm2.x))) * a.rh) * a.rh;
-        w1 = w1 + ((((F_D2A * Vb.y) + (F_D2B * (Vp1.y + Vm1.y))) + (A_D2C * (Vp2.y + Vm2.y))) * a.rh) * a.rh;
-        const float2 lc = lds2(L + so);
-        const float n0 = (w0 + (2.0f * lc.x)) - lpv[r].x;
-        const float n1 = (w1 + (2.0f * lc.y)) - lpv[r].y;
-        const float g0 = 0.0f + ((lc.x * stv[r].x) * 1.0f);
-        const float g1 = 0.0f + ((lc.y * stv[r].y) * 1.0f);
-        st2(gf + cell, gav[r].x + g0, gav[r].y + g1);
-        st2(Lnf + cell, n0, n1);
+        const float2 Vb = vs[r], Va = lds2(VS + so + r * BX - 2), Vc = lds2(VS + so + r * BX + 2);
+        const float2 Vm2 = r >= 2 ? vs[r >= 2 ? r - 2 : 0] : (r == 1 ? up1 : up2);
+        const float2 Vm1 = r >= 1 ? vs[r >= 1 ? r - 1 : 0] : up1;
+        const float2 Vp1 = r + 1 < RPT ? vs[r + 1 < RPT ? r + 1 : r] : dn1;
+        const float2 Vp2 = r + 2 < RPT ? vs[r + 2 < RPT ? r + 2 : r] : (r + 2 == RPT ? dn1 : dn2);
+        const float2 w = add2(pk.second(Vb, side_sum(Va, Vb, Vc), add2(Vc, Va), a.rh, a.rh),
+                              pk.second(Vb, add2(Vp1, Vm1), add2(Vp2, Vm2), a.rh, a.rh));
+        const float2 lc = lds2(L + so + r * BX);
+        // the shader starts the per-step gradient at +0; starting from the product itself differs
+        // only in the sign of an exact zero
+        put2(gf + cell, add2(gav[r], pk.mul(lc, stv[r])));
+        put2(Lnf + cell, sub2(add2(w, add2(lc, lc)), lpv[r]));
       }
       __syncthreads();  // stage and VS are reused by the next tile
       continue;
     }
 
-    // derived terms over the tile and its halo (pairs of columns x0-4+2j, rows z0-2+k)
-#pragma unroll
-    for (int d = 0; d < DER; ++d) {
-      const int e = tid + d * NTH;
-      if (e >= BZ * (BX / 2)) break;
-      const int k = e / (BX / 2), j = e % (BX / 2);
-      const int z = z0 - HZ + k, x = x0 - HX + 2 * j;
-      const int o = k * BX + 2 * j;
-      float vs0 = 0.f, vs1 = 0.f;
-      const bool in = z >= 0 && z < nz && x >= 0 && x < nx;
-      if (in) {
-        const float2 v = vd[d];
-        const float2 l = lds2(L + o);
-        vs0 = ((v.x * v.x) * a.dt2) * l.x;
-        vs1 = ((v.y * v.y) * a.dt2) * l.y;
-      }
-      st2(VS + o, vs0, vs1);
-      if (xtile && in && (x < ssw || x >= nx - ssw)) {
-        const int xc = xstrip(x, nx, ssw);
-        const float2 b = ldg2(sBX + x), db = ldg2(sDBX + x);
-        const float2 Z = ld2(LZXc + static_cast<size_t>(z) * 2 * ssw + xc);
-        const float2 P = ld2(LPXc + static_cast<size_t>(z) * 2 * ssw + xc);
-        const float T0 = ((1.0f + b.x) * vs0) + (b.x * Z.x);
-        const float T1 = ((1.0f + b.y) * vs1) + (b.y * Z.y);
-        st2(TXs + o, T0, T1);
-        st2(U1Xs + o, (db.x * T0) + (b.x * P.x), (db.y * T1) + (b.y * P.y));
-      }
-      if (ztile && in && (z < ssw || z >= nz - ssw)) {
-        const int zc = z < ssw ? z : z - (nz - 2 * ssw);
-        const float bz = __ldg(&sBZ[z]), dbz = __ldg(&sDBZ[z]);
-        const float opbz = 1.0f + bz;
-        const float2 Z = ld2(LZZc + static_cast<size_t>(zc) * nx + x);
-        const float2 P = ld2(LPZc + static_cast<size_t>(zc) * nx + x);
-        const float T0 = (opbz * vs0) + (bz * Z.x);
-        const float T1 = (opbz * vs1) + (bz * Z.y);
-        st2(TZs + o, T0, T1);
-        st2(U1Zs + o, (dbz * T0) + (bz * P.x), (dbz * T1) + (bz * P.y));
-      }
-    }
-    __syncthreads();
-
-    const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
     const bool xpml = x < region || x + 1 >= nx - region;
     const int* sc = a.st.src_cell + 4 * shot;
     const float* res_t = a.residual + (static_cast<size_t>(unit) * a.nt + a.t) * a.st.nrec;
     const bool rec_rows = zr + RPT > a.rec_z0 && zr <= a.rec_z1;
-    unsigned srcm = 0;
-    {
-      const int base = zr * nx + x;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int d = __ldg(&sc[k]) - base;
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-          const unsigned o = static_cast<unsigned>(d - r * nx);
-          if (o < 2u) srcm |= 1u << (2 * r + o);
-        }
-      }
-    }
-    const int xc = xstrip(x, nx, ssw);
+    const unsigned srcm = j.src ? source_bits(a, shot, zr, x) : 0u;
     float* LPXn = a.PX + (static_cast<size_t>(1 - q) * a.units + unit) * xs_unit;
     float* LZXn = a.ZX + (static_cast<size_t>(1 - q) * a.units + unit) * xs_unit;
     float* LPZn = a.PZ + (static_cast<size_t>(1 - q) * a.units + unit) * zs_unit;
     float* LZZn = a.ZZ + (static_cast<size_t>(1 - q) * a.units + unit) * zs_unit;
+    float2 Ba = make_float2(0.f, 0.f), Bb = Ba, Bc = Ba, ax = Ba;
+    if (xpml && xok) {
+      Ba = ldg2(sBX + x - 2);
+      Bb = ldg2(sBX + x);
+      Bc = ldg2(sBX + x + 2);
+      ax = ldg2(sAX + x);
+    }
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int z = zr + r;
       if (!xok || z < FD_PAD || z >= nz - FD_PAD) continue;
       const int cell = z * nx + x;
       const int so = (sz + r) * BX + sx;
-      const float2 Vb = lds2(VS + so);
-      float w0, w1;
+      const float2 Vb = vs[r];
+      float2 w;
       if (xpml) {
         const float2 Ta = lds2(TXs + so - 2), Tb = lds2(TXs + so), Tc = lds2(TXs + so + 2);
         const float2 Ua = lds2(U1Xs + so - 2), Ub = lds2(U1Xs + so), Uc = lds2(U1Xs + so + 2);
-        const float2 Ba = ldg2(sBX + x - 2), Bb = ldg2(sBX + x), Bc = ldg2(sBX + x + 2);
-        const float q0 = (1.0f + Ba.x) * Ta.x, q1 = (1.0f + Ba.y) * Ta.y, q2 = (1.0f + Bb.x) * Tb.x,
-                    q3 = (1.0f + Bb.y) * Tb.y, q4 = (1.0f + Bc.x) * Tc.x, q5 = (1.0f + Bc.y) * Tc.y;
-        const float du0 = ((F_D1A * (Ub.y - Ua.y)) + (A_D1B * (Uc.x - Ua.x))) * a.rh;
-        const float dd0 = ((((F_D2A * q2) + (F_D2B * (q3 + q1))) + (A_D2C * (q4 + q0))) * a.rh) * a.rh;
-        const float dt0 = ((F_D1A * (Tb.y - Ta.y)) + (A_D1B * (Tc.x - Ta.x))) * a.rh;
-        const float du1 = ((F_D1A * (Uc.x - Ub.x)) + (A_D1B * (Uc.y - Ua.y))) * a.rh;
-        const float dd1 = ((((F_D2A * q3) + (F_D2B * (q4 + q2))) + (A_D2C * (q5 + q1))) * a.rh) * a.rh;
-        const float dt1 = ((F_D1A * (Tc.x - Tb.x)) + (A_D1B * (Tc.y - Ta.y))) * a.rh;
-        w0 = (-du0) + dd0;
-        w1 = (-du1) + dd1;
+        const float2 qa = pk.mul(make_float2(1.0f + Ba.x, 1.0f + Ba.y), Ta), qb = pk.mul(make_float2(1.0f + Bb.x, 1.0f + Bb.y), Tb),
+                     qc = pk.mul(make_float2(1.0f + Bc.x, 1.0f + Bc.y), Tc);
+        const float2 du = pk.first(side_diff(Ua, Ub, Uc), sub2(Uc, Ua), a.rh);
+        const float2 dd = pk.second(qb, side_sum(qa, qb, qc), add2(qc, qa), a.rh, a.rh);
+        const float2 dt = pk.first(side_diff(Ta, Tb, Tc), sub2(Tc, Ta), a.rh);
+        w = sub2(dd, du);
         const int xo = z * 2 * ssw + xc;
-        const float2 P = ld2(LPXc + xo), Z = ld2(LZXc + xo);
-        const float2 ax = ldg2(sAX + x);
-        st2(LPXn + xo, ((-ax.x) * dt0) + (ax.x * P.x), ((-ax.y) * dt1) + (ax.y * P.y));
-        st2(LZXn + xo, (ax.x * Vb.x) + (ax.x * Z.x), (ax.y * Vb.y) + (ax.y * Z.y));
+        put2(LPXn + xo, sub2(pk.mul(ax, xP[r]), pk.mul(ax, dt)));
+        put2(LZXn + xo, add2(pk.mul(ax, Vb), pk.mul(ax, xZ[r])));
       } else {
         const float2 Va = lds2(VS + so - 2), Vc = lds2(VS + so + 2);
-        w0 = ((((F_D2A * Vb.x) + (F_D2B * (Vb.y + Va.y))) + (A_D2C * (Vc.x + Va.x))) * a.rh) * a.rh;
-        w1 = ((((F_D2A * Vb.y) + (F_D2B * (Vc.x + Vb.x))) + (A_D2C * (Vc.y + Va.y))) * a.rh) * a.rh;
+        w = pk.second(Vb, side_sum(Va, Vb, Vc), add2(Vc, Va), a.rh, a.rh);
       }
       if (z < region || z >= nz - region) {
         const float2 Tm2 = lds2(TZs + so - 2 * BX), Tm1 = lds2(TZs + so - BX), T0 = lds2(TZs + so),
@@ -931,51 +953,39 @@ __global__ void __launch_bounds__(NTH) adj_stream_kernel(const __grid_constant__
                      Up2 = lds2(U1Zs + so + 2 * BX);
         const float om2 = 1.0f + __ldg(&sBZ[z - 2]), om1 = 1.0f + __ldg(&sBZ[z - 1]), o0 = 1.0f + __ldg(&sBZ[z]),
                     op1 = 1.0f + __ldg(&sBZ[z + 1]), op2 = 1.0f + __ldg(&sBZ[z + 2]);
-        const float du0 = ((F_D1A * (Up1.x - Um1.x)) + (A_D1B * (Up2.x - Um2.x))) * a.rh;
-        const float du1 = ((F_D1A * (Up1.y - Um1.y)) + (A_D1B * (Up2.y - Um2.y))) * a.rh;
-        const float dd0 = ((((F_D2A * (o0 * T0.x)) + (F_D2B * ((op1 * Tp1.x) + (om1 * Tm1.x)))) +
-                            (A_D2C * ((op2 * Tp2.x) + (om2 * Tm2.x)))) * a.rh) * a.rh;
-        const float dd1 = ((((F_D2A * (o0 * T0.y)) + (F_D2B * ((op1 * Tp1.y) + (om1 * Tm1.y)))) +
-                            (A_D2C * ((op2 * Tp2.y) + (om2 * Tm2.y)))) * a.rh) * a.rh;
-        const float dt0 = ((F_D1A * (Tp1.x - Tm1.x)) + (A_D1B * (Tp2.x - Tm2.x))) * a.rh;
-        const float dt1 = ((F_D1A * (Tp1.y - Tm1.y)) + (A_D1B * (Tp2.y - Tm2.y))) * a.rh;
-        w0 = w0 + ((-du0) + dd0);
-        w1 = w1 + ((-du1) + dd1);
-        const int zc = z < ssw ? z : z - (nz - 2 * ssw);
-        const int zo = zc * nx + x;
+        const float2 du = pk.first(sub2(Up1, Um1), sub2(Up2, Um2), a.rh);
+        const float2 dd = pk.second(scale2(o0, T0), add2(pk.scale(op1, Tp1), pk.scale(om1, Tm1)),
+                                    add2(pk.scale(op2, Tp2), pk.scale(om2, Tm2)), a.rh, a.rh);
+        const float2 dt = pk.first(sub2(Tp1, Tm1), sub2(Tp2, Tm2), a.rh);
+        w = add2(w, sub2(dd, du));
+        const int zo = (z < ssw ? z : z - (nz - 2 * ssw)) * nx + x;
         const float az = __ldg(&sAZ[z]);
-        const float2 P = ld2(LPZc + zo), Z = ld2(LZZc + zo);
-        st2(LPZn + zo, ((-az) * dt0) + (az * P.x), ((-az) * dt1) + (az * P.y));
-        st2(LZZn + zo, (az * Vb.x) + (az * Z.x), (az * Vb.y) + (az * Z.y));
+        put2(LPZn + zo, sub2(pk.scale(az, zP[r]), pk.scale(az, dt)));
+        put2(LZZn + zo, add2(pk.scale(az, Vb), pk.scale(az, zZ[r])));
       } else {
         const float2 Vm2 = lds2(VS + so - 2 * BX), Vm1 = lds2(VS + so - BX), Vp1 = lds2(VS + so + BX),
                      Vp2 = lds2(VS + so + 2 * BX);
-        w0 = w0 + ((((F_D2A * Vb.x) + (F_D2B * (Vp1.x + Vm1.x))) + (A_D2C * (Vp2.x + Vm2.x))) * a.rh) * a.rh;
-        w1 = w1 + ((((F_D2A * Vb.y) + (F_D2B * (Vp1.y + Vm1.y))) + (A_D2C * (Vp2.y + Vm2.y))) * a.rh) * a.rh;
+        w = add2(w, pk.second(Vb, add2(Vp1, Vm1), add2(Vp2, Vm2), a.rh, a.rh));
       }
       const float2 lc = lds2(L + so);
-      const float2 lp = lpv[r];
-      float n0 = (w0 + (2.0f * lc.x)) - lp.x;
-      float n1 = (w1 + (2.0f * lc.y)) - lp.y;
-      const float2 sv = stv[r];
-      float g0 = 0.0f + ((lc.x * sv.x) * 1.0f);
-      float g1 = 0.0f + ((lc.y * sv.y) * 1.0f);
+      const float2 n = sub2(add2(w, add2(lc, lc)), lpv[r]);
+      float n0 = n.x, n1 = n.y;
+      float2 gr = pk.mul(lc, stv[r]);
       if (rec_rows) {
         const int e0 = a.st.csr[cell], e1 = a.st.csr[cell + 1], e2 = a.st.csr[cell + 2];
         for (int e = e0; e < e1; ++e) n0 = n0 + (a.st.ent_w[e] * res_t[a.st.ent_rec[e]]);
         for (int e = e1; e < e2; ++e) n1 = n1 + (a.st.ent_w[e] * res_t[a.st.ent_rec[e]]);
       }
-      const int ci = cell;
       if (srcm & (3u << (2 * r))) {
-        const float2 v = ldg2(vel + cell);
+        const float2 v = vv[r];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float wk = a.st.src_w[4 * shot + k];
-          if (ci == sc[k]) g0 = g0 + lc.x * (((((-2.0f) * v.x) * a.dt2) * wk) * f);
-          if (ci + 1 == sc[k]) g1 = g1 + lc.y * (((((-2.0f) * v.y) * a.dt2) * wk) * f);
+          if (cell == sc[k]) gr.x = gr.x + lc.x * (((((-2.0f) * v.x) * a.dt2) * wk) * f);
+          if (cell + 1 == sc[k]) gr.y = gr.y + lc.y * (((((-2.0f) * v.y) * a.dt2) * wk) * f);
         }
       }
-      st2(gacc + cell, gav[r].x + g0, gav[r].y + g1);
+      put2(gacc + cell, add2(gav[r], gr));
       st2(Ln + cell, n0, n1);
     }
     __syncthreads();  // stage and derived arrays are reused by the next tile
@@ -1178,6 +1188,7 @@ SArgs base_args(StreamWork* w, const EngineView& v, int units) {
   a.tile_rec_start = static_cast<const int*>(w->tile_rec_start.p);
   a.tile_rec = static_cast<const int*>(w->tile_rec.p);
   a.status = v.d_status;
+  a.nz2[0] = a.nz2[1] = -0.0f;
   return a;
 }
 
@@ -1201,18 +1212,33 @@ int alloc_forward(StreamWork* w, const EngineView& v, int units, cudaStream_t st
 }
 
 // One forward step over all units.
+// A step's launch, allowed to be scheduled while the step before it drains (see wait_for_previous_step).
+template <class... P, class... A>
+cudaError_t launch_step(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int fwd_step(StreamWork* w, const FwdMaps& map, SArgs a, int t, bool traces, bool store, cudaStream_t st) {
   a.t = t;
   const int jobs = a.units * a.tiles_x * a.tiles_z;
   const int blocks = std::min(jobs, w->fwd_blocks);
   note_launch();
   if (traces && store)
-    fwd_stream_kernel<true, true><<<blocks, FWD_THREADS, kFwdSmem, st>>>(map, a);
+    SW_CK(launch_step(fwd_stream_kernel<true, true>, blocks, FWD_THREADS, kFwdSmem, st, map, a));
   else if (traces)
-    fwd_stream_kernel<true, false><<<blocks, FWD_THREADS, kFwdSmem, st>>>(map, a);
+    SW_CK(launch_step(fwd_stream_kernel<true, false>, blocks, FWD_THREADS, kFwdSmem, st, map, a));
   else
-    fwd_stream_kernel<false, true><<<blocks, FWD_THREADS, kFwdSmem, st>>>(map, a);
-  SW_CK(cudaGetLastError());
+    SW_CK(launch_step(fwd_stream_kernel<false, true>, blocks, FWD_THREADS, kFwdSmem, st, map, a));
   return WG_OK;
 }
 
@@ -1221,8 +1247,7 @@ int adj_step(StreamWork* w, const CUtensorMap& map, SArgs a, int t, cudaStream_t
   const int jobs = a.units * a.tiles_x * a.tiles_z;
   const int blocks = std::min(jobs, w->adj_blocks);
   note_launch();
-  adj_stream_kernel<<<blocks, NTH, kAdjSmem, st>>>(map, a);
-  SW_CK(cudaGetLastError());
+  SW_CK(launch_step(adj_stream_kernel, blocks, NTH, kAdjSmem, st, map, a));
   return WG_OK;
 }
 
@@ -1266,15 +1291,26 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
     p.set_in = k & 1;
     note_launch();
     if (stored)
-      fwd_tb_kernel<true, true><<<blocks, TB_THREADS, kTbSmem, st>>>(um, vm, p);
+      SW_CK(launch_step(fwd_tb_kernel<true, true>, blocks, TB_THREADS, kTbSmem, st, um, vm, p));
     else
-      fwd_tb_kernel<true, false><<<blocks, TB_THREADS, kTbSmem, st>>>(um, vm, p);
-    SW_CK(cudaGetLastError());
+      SW_CK(launch_step(fwd_tb_kernel<true, false>, blocks, TB_THREADS, kTbSmem, st, um, vm, p));
   }
   return WG_OK;
 }
 
 // Checkpoint slot layout: [W(t) | W(t-1) | PX(t) | ZX | PZ(t) | ZZ] for all units.
+// Whether a pass that starts from the zero state and writes no checkpoints runs temporally blocked: as
+// the engine option says, or, where it was not set, when its tiles fit the chip in three waves: a step is then
+// mostly the latency of its launch and copies, which four steps share.
+// us per step (recording traces), blocked against one step per launch: 50 tiles (2 shots of 284 x 154
+// cells) 3.4 / 7.3, 150 tiles 3.4 / 7.5, 210 tiles 6.1 / 7.7, 420 tiles 8.1 / 10.4, 560 tiles 9.9 / 9.3.
+constexpr int kTbWaves = 3;
+bool blocked(const StreamWork* w, const EngineView& v, int units) {
+  if (v.tblock >= 0) return v.tblock != 0;
+  const long jobs = static_cast<long>(units) * ((v.nx + TX_ - 1) / TX_) * ((v.nz + TZ_ - 1) / TZ_);
+  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks;
+}
+
 size_t ckpt_slot_floats(const EngineView& v, int units) {
   const size_t cells = static_cast<size_t>(v.nx) * v.nz;
   return static_cast<size_t>(units) * (2 * cells + 2 * xs_floats(v) + 2 * zs_floats(v));
@@ -1324,7 +1360,7 @@ int stream_simulate(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   SW_CK(w->vpad.ensure(models * cells * 4));
   note_launch();
   SW_CK(launch_pad_velocity(d_vis, models, v.nx_vis, v.nz_vis, v.pad, v.vmin, v.vmax, w->vpad.f(), nullptr, st));
-  if (v.tblock) {
+  if (blocked(w, v, units)) {
     timer.mark(0, true, st);
     if ((rc = tb_forward(w, v, units, models, d_traces, nullptr, st)) != WG_OK) return rc;
     timer.mark(0, false, st);
@@ -1422,7 +1458,7 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   f.seg = seg;
   f.seg_t0 = 0;
   timer.mark(0, true, st);
-  if (store_all && v.tblock) {
+  if (store_all && blocked(w, v, units)) {
     if ((rc = tb_forward(w, v, units, models, w->traces.f(), w->stored.f(), st)) != WG_OK) return rc;
   } else {
     for (int t = 0; t < v.nt; ++t) {

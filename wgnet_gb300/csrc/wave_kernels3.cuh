@@ -19,6 +19,7 @@
 #include "wave_kernels.cuh"
 #include "wave_kernels3_layout.h"
 #include "wave_launch.h"
+#include "wave_packed.cuh"
 
 namespace wg {
 
@@ -149,52 +150,6 @@ struct FastCoef {
   __device__ __forceinline__ float d1(float dd1, float dd2) const { return fmaf(e2, dd2, e1 * dd1); }
 };
 
-// Packed FP32 arithmetic: a thread's column pair is one operand, each half rounded to nearest as the
-// scalar operation is. ptxas contracts a packed product and sum into a packed fma even under
-// -fmad=false and with explicit .rn, which would round once where the reference rounds twice. So a
-// product that feeds a sum is formed as fma(a, b, -0) with the -0 taken from the kernel's arguments,
-// where the compiler cannot see it: a b + (-0) is the rounded product bit for bit (signs of zeros
-// included), and an fma is not contracted again.
-//
-// The forward's row update is packed: 320 units x 200 steps on the 70 x 70 grid take 2.98 against
-// 3.15 ms recording traces and 1.50 against 1.61 ms storing terms (100 steps). The packed fma issues
-// at half rate, so the arithmetic itself is no faster; what is saved are issue slots. The adjoint
-// stays scalar: packed, it took 5.28 against 4.84 ms (it waits on shared memory and instruction
-// fetch, not on issue slots).
-struct Pk {
-  float2 nz;  // (-0, -0), opaque
-  __device__ __forceinline__ float2 mul(float2 a, float2 b) const { return __ffma2_rn(a, b, nz); }
-  __device__ __forceinline__ float2 scale(float a, float2 b) const { return mul(make_float2(a, a), b); }
-  // (((D2A u + D2B s1) - D2C s2) ka) kb; s1 / s2: sums of the neighbours at distance 1 / 2 (the
-  // adjoint's (x + (-D2C) s2) is the same value)
-  __device__ __forceinline__ float2 second(float2 u, float2 s1, float2 s2, float ka, float kb) const;
-  // ((D1A d1) - D1B d2) rh; d1 / d2: differences of the neighbours at distance 1 / 2
-  __device__ __forceinline__ float2 first(float2 d1, float2 d2, float rh) const;
-};
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tsub.rn.f32x2 z, x, y;\n\t"
-      "mov.b64 {%0, %1}, z;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-// a product that no sum reads (its reader is a store or another product)
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 scale2(float a, float2 b) { return mul2(dup2(a), b); }
-// Sums and differences at distance 1 along x of the own pair u between the pairs a (left) and b
-// (right): they join an own column and a neighbour's, so they are formed per column.
-__device__ __forceinline__ float2 side_sum(float2 a, float2 u, float2 b) { return make_float2(u.y + a.y, b.x + u.x); }
-__device__ __forceinline__ float2 side_diff(float2 a, float2 u, float2 b) { return make_float2(u.y - a.y, b.x - u.x); }
-__device__ __forceinline__ float2 Pk::second(float2 u, float2 s1, float2 s2, float ka, float kb) const {
-  return scale(kb, scale2(ka, add2(add2(scale(F_D2A, u), scale(F_D2B, s1)), scale(-F_D2C, s2))));
-}
-__device__ __forceinline__ float2 Pk::first(float2 d1, float2 d2, float rh) const {
-  return scale(rh, add2(scale(F_D1A, d1), scale(-F_D1B, d2)));
-}
-
 __device__ __forceinline__ float2 lds2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void sts2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 __device__ __forceinline__ void sts2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
@@ -284,6 +239,12 @@ struct HaloLink {
 enum : int { LAY_RUNTIME = 0, LAY_EVEN = 1, LAY_SQUARE = 2, LAY_RAGGED = 3 };
 
 // FA: fast arithmetic (see FastCoef); otherwise the reference's operation order, unfused.
+//
+// The exact row update is packed (wave_packed.cuh): 320 units x 200 steps on the 70 x 70 grid take 2.98 against
+// 3.15 ms recording traces and 1.50 against 1.61 ms storing terms (100 steps). The packed fma issues
+// at half rate, so the arithmetic itself is no faster; what is saved are issue slots. The adjoint
+// stays scalar: packed, it took 5.28 against 4.84 ms (it waits on shared memory and instruction
+// fetch, not on issue slots).
 template <int NX, int PMLP, int C, int S, int NSEG, int NI, int LAY, bool TRACES, bool STORE, bool FA = false>
 __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __grid_constant__ FwdArgs p) {
   constexpr bool RAG = LAY == LAY_RAGGED;

@@ -96,7 +96,7 @@ struct EngineView {
   int* d_status;
   int adj_prefetch;
   int fast;    // fast-arithmetic kernels (engine option "arith")
-  int tblock;  // streamed path: temporally blocked forward where it applies (engine option "temporal_block")
+  int tblock;  // streamed path: temporally blocked forward where it applies (engine option "temporal_block"; -1: not set)
 };
 
 // Event marks around groups of launches (kind 0 forward, 1 forward recompute, 2 adjoint) for the
