@@ -220,7 +220,7 @@ int wg_pc_mse(const float* d_out, int ld, const float* d_target, float scale, lo
 int wg_pc_adam(const float* d_partial, int splits, int n, int kp, float* d_w32, float* d_m1, float* d_m2, float lr,
                float b1, float b2, float eps, int step, void* d_w_bf16, void* d_wt_bf16, void* stream);
 
-/* Same-padded 3x3 convolution (dilation dil <= 60) of activations [batch][h][w][64] bf16 with a fused
+/* Same-padded 3x3 convolution (dilation dil <= 10) of activations [batch][h][w][64] bf16 with a fused
  * epilogue; y is the FP32 result per pixel and channel. mode
  *   0: out16 = bf16(max(y, 0))
  *   1: out16 = bf16(max(y, 0)), out32 = out16 > 0 ? y : 0; d_act is a matrix [pixels][kp] (columns)

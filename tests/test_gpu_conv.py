@@ -151,7 +151,7 @@ def test_bad_arguments_are_refused(cuda_lib):
     st = torch.zeros(4, device="cuda", dtype=torch.int32)
     z = ctypes.c_void_p(0)
     out = torch.empty((72, 64), device="cuda", dtype=torch.bfloat16)
-    for mode, kp, dil, o16 in ((7, 576, 1, out), (0, 128, 1, out), (0, 576, 0, out), (0, 576, 61, out), (2, 576, 1, out)):
+    for mode, kp, dil, o16 in ((7, 576, 1, out), (0, 128, 1, out), (0, 576, 0, out), (0, 576, 11, out), (2, 576, 1, out)):
         assert cuda_lib.wg_pc_conv(mode, _p(act), 1, 8, 9, dil, _p(w), kp, z, z, z, _p(o16), _p(st), None) != 0
     part = torch.empty((1, 576, 64), device="cuda")
     assert cuda_lib.wg_pc_conv_wgrad(_p(act), 0, _p(act), 1, 8, 9, 1, 1, _p(part), _p(st), None) != 0  # 72 pixels

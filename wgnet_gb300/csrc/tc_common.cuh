@@ -62,6 +62,24 @@ __device__ __forceinline__ uint64_t sdesc_sw128(const void* p) {
   return d;
 }
 
+// The same descriptor in halves: the upper one is constant, the lower one advances by (bytes >> 4), so that
+// the lane that issues the MMAs spends two instructions on a pair of operands instead of some thirty
+// (they, not the tensor core, set the pace of N = 64 tiles: 70 cycles per MMA).
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo = 16) {
+  return ((smem_addr >> 4) & 0x3FFF) | ((lbo >> 4) << 16);
+}
+__device__ __forceinline__ void mma_bf16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(static_cast<uint32_t>(acc)), "n"(kDescHi)
+      : "memory");
+}
+
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 D, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
   return (1u << 4)                                 // D format F32
@@ -113,6 +131,32 @@ inline int map_bf16(CUtensorMap* m, const void* base, long rows, long K, int box
 }
 
 
+// Activations [batch][h][w][64] bf16 as boxes of 8 columns x `rows` rows of one image, 128 bytes per
+// pixel, 128-byte swizzle: a box row of 8 pixels is one 1024-byte swizzle atom. Pixels outside the
+// image read zero.
+inline int map_image(CUtensorMap* m, const void* base, int batch, int h, int w, int rows) {
+  auto fn = encode();
+  if (!fn) return report_error(WG_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t dims[4] = {64, static_cast<cuuint64_t>(w), static_cast<cuuint64_t>(h), static_cast<cuuint64_t>(batch)};
+  const cuuint64_t strides[3] = {128, static_cast<cuuint64_t>(w) * 128, static_cast<cuuint64_t>(w) * h * 128};
+  const cuuint32_t box[4] = {64, 8, static_cast<cuuint32_t>(rows), 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return report_error(WG_ERR_CUDA, ("cuTensorMapEncodeTiled(image) failed: " + std::to_string(r)).c_str());
+  return WG_OK;
+}
+
+__device__ __forceinline__ void tma_image(void* dst, const CUtensorMap* map, int x, int y, int n, uint64_t* b) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(su32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(x), "r"(y), "r"(n), "r"(su32(b))
+      : "memory");
+}
+
 // Activations [batch][h][w][64] bf16 read pixel by pixel in their linear order, shifted by one tap of
 // a same-padded 3x3 convolution of dilation `dil` (im2col mode: the base pixel runs over the image
 // shifted by (-dil, -dil), the tap's offset (0..2) dil comes with the load; pixels outside the image
@@ -139,14 +183,35 @@ inline int map_im2col(CUtensorMap* m, const void* base, int batch, int h, int w,
   return WG_OK;
 }
 
-// Load of `pixels` shifted pixels from linear pixel m on, for the tap offset (ox, oy).
-__device__ __forceinline__ void tma_im2col(void* dst, const CUtensorMap* map, int m, int h, int w, int dil, int ox, int oy,
+// Position of a linear pixel: the divisions are done once per tile, not once per tap (with one lane
+// issuing the loads they bounded the convolutions).
+struct Pixel {
+  int n, y, x;
+  __device__ __forceinline__ Pixel(int m, int h, int w) {
+    n = m / (h * w);
+    const int r = m - n * h * w;
+    y = r / w;
+    x = r - y * w;
+  }
+  __device__ __forceinline__ void advance(int pixels, int h, int w) {
+    x += pixels;
+    while (x >= w) {
+      x -= w;
+      if (++y == h) {
+        y = 0;
+        ++n;
+      }
+    }
+  }
+};
+
+// Load of `pixels` (of the map) shifted pixels from p on, for the tap offset (ox, oy).
+__device__ __forceinline__ void tma_im2col(void* dst, const CUtensorMap* map, const Pixel& p, int dil, int ox, int oy,
                                            uint64_t* b) {
-  const int n = m / (h * w), r = m - n * h * w, y = r / w, x = r - y * w;
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
       "[%6], {%7, %8};" ::"r"(su32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(x - dil), "r"(y - dil), "r"(n), "r"(su32(b)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(p.x - dil), "r"(p.y - dil), "r"(p.n), "r"(su32(b)),
       "h"(static_cast<unsigned short>(ox)), "h"(static_cast<unsigned short>(oy))
       : "memory");
 }

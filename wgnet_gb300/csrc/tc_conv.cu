@@ -1,16 +1,21 @@
 // 3x3 convolutions of the update network on the 5th-generation tensor cores, with no im2col matrix:
 // forward, data gradient and weight gradient read the activations' shifted pixels straight from
-// [batch][h][w][64] bf16 by TMA (im2col mode, zero fill outside the image) and finish in the
-// epilogue what separate passes did (ReLU, residual add, bf16 casts, ReLU masks, the sum over taps
-// of the data gradient). The arithmetic is that of gemm_bf16_kernel on im2col columns followed by
-// those passes, in the same order: every output is bit-identical to that route.
+// [batch][h][w][64] bf16 by TMA (zero fill outside the image) and finish in the epilogue what separate
+// passes did (ReLU, residual add, bf16 casts, ReLU masks, the sum over taps of the data gradient). The
+// arithmetic is that of gemm_bf16_kernel on im2col columns followed by those passes, in the same
+// order: every output is bit-identical to that route.
 //
 // What bounds them: a 64 -> 64 convolution of 32 x 70 x 70 pixels needs 11.6 GFLOP (6 us at the bf16
-// rate) but feeds each output tile 9 x 16 KB of shifted pixels from L2, 180 MB in all, and reads or
-// writes 20 to 120 MB of activations. So the weights (72 KB) stay in shared memory, one persistent CTA
-// per SM keeps 7 taps in flight, and the accumulators are double-buffered in tensor memory so that
-// the epilogue of a tile overlaps the loads of the next.
+// rate) and reads or writes 20 to 120 MB of activations (3 to 18 us at the HBM rate); feeding every
+// tap of every output tile from L2 is more than either (180 MB: 34 us with one TMA load per tap). So
+// an output tile is 8 columns x 16 rows of an image and the three taps of a column come from one box
+// of 16 + 2 dil rows (a row of 8 pixels is one swizzle atom, so a tap's operand starts dil atoms
+// further): 3 to 6 loads' worth of bytes instead of 9. The weights (72 KB) stay in shared memory, one
+// persistent CTA per SM keeps the next tile's boxes in flight, and the accumulators are double-buffered
+// in tensor memory so that the epilogue of a tile overlaps the loads of the next.
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "tc_common.cuh"
 
@@ -28,9 +33,12 @@ enum Epi : int {
   EPI_ACC_MASK = 6,  // data gradient: out16 = bf16(mask16 > 0 ? add32 + y : 0)
 };
 
-constexpr int CBM = 128;                         // pixels per tile
-constexpr int CST = 7;                           // taps in flight
+constexpr int CTW = 8, CTH = 16;                 // columns and rows of an output tile
+constexpr int CBM = CTW * CTH;                   // pixels per tile
+constexpr int CST = 8;                           // most boxes in flight
 constexpr unsigned kTapBytes = CBM * 128;        // one tap of a tile: 128 pixels x 64 channels
+constexpr unsigned kRing = 7 * kTapBytes;        // shared memory of the boxes in flight
+constexpr int kMaxDil = 10;                      // three boxes of 16 + 2 dil rows fit the ring
 constexpr int CEPI = 8;                          // epilogue warps
 constexpr int CTHR = 64 + 32 * CEPI;             // producer warp, MMA warp, epilogue warps
 constexpr int CLD = 68;                          // row stride (floats) of the epilogue's staging tile
@@ -38,7 +46,10 @@ constexpr int CKT = 9;                           // most k tiles (taps) of a til
 
 struct ConvArgs {
   int M, h, w, dil;
+  int tiles, tiles_x, tiles_img; // output tiles: all, per row of tiles, per image
   int kt;                        // k tiles per output tile: 9 taps, or the 64-wide column blocks of a matrix
+  int stages;                    // boxes in flight
+  unsigned box;                  // bytes of a box
   const float* add32;            // [M][64]
   const __nv_bfloat16* mask16;   // [M][64]
   float* out32;
@@ -46,8 +57,8 @@ struct ConvArgs {
   int* status;
 };
 
-// Shared memory: weights [kt][N rows][128 B] | stages [CST][128][128 B] | staging tile | barriers.
-constexpr size_t kConvSmem = CKT * 64 * 128 + CST * kTapBytes + CBM * CLD * 4 + 256 + 1024;
+// Shared memory: weights [kt][N rows][128 B] | boxes in flight | staging tile | barriers.
+constexpr size_t kConvSmem = CKT * 64 * 128 + kRing + CBM * CLD * 4 + 256 + 1024;
 
 __device__ __forceinline__ void bar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
@@ -91,8 +102,8 @@ __device__ __forceinline__ bool bf16_positive(uint32_t pair, int hi) {
   return __uint_as_float(bits) > 0.0f;
 }
 
-// One tile is 128 pixels in linear order x N channels. Warp 0 (one lane) loads the tile's shifted
-// pixels, warp 1 (one lane) issues the MMAs, warps 2-9 run the epilogue. The data gradient keeps
+// One tile is 128 pixels x N channels: 8 x 16 pixels of an image (in MATRIX mode 128 rows of the
+// matrix). Warp 0 (one lane) loads the tile's boxes, warp 1 (one lane) issues the MMAs, warps 2-9 run the epilogue. The data gradient keeps
 // one accumulator per tap (the reference route rounds each tap's product to FP32 before it sums the
 // taps): the epilogue adds the nine in tap order. Every wait is bounded; a warp that gives up
 // records the error, the others follow through their own waits, and the CTA drains the copies and
@@ -110,7 +121,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
   unsigned char* smem = smem_raw + ((1024 - (su32(smem_raw) & 1023)) & 1023);
   unsigned char* sB = smem;
   unsigned char* sA = sB + CKT * 64 * 128;
-  float* tile = reinterpret_cast<float*>(sA + CST * kTapBytes);
+  float* tile = reinterpret_cast<float*>(sA + kRing);
   uint64_t* full = reinterpret_cast<uint64_t*>(tile + CBM * CLD);
   uint64_t* empty = full + CST;
   uint64_t* acc_full = empty + CST;
@@ -120,8 +131,8 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
   __shared__ int fail;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kt = a.kt;
-  const int tiles = (a.M + CBM - 1) / CBM;
+  const int kt = a.kt, tiles = a.tiles, stages = a.stages;
+  const int boxes = MATRIX ? kt : 3;  // per tile
   if (tid == 0) {
     for (int s = 0; s < CST; ++s) {
       bar_init(&full[s], 1);
@@ -151,64 +162,104 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       for (int t = 0; t < kt; ++t) tma2d(sB + t * N * 128, &mapB, DGRAD ? 0 : 64 * t, DGRAD ? 64 * t : 0, wbar);
       int it = 0;
       bool ok = true;
+      int s = 0, phase = 1;  // ring position; the parity of the phase before it, complete at first
       for (int tl = blockIdx.x; ok && tl < tiles; tl += gridDim.x) {
-        for (int t = 0; t < kt; ++t, ++it) {
-          const int s = it % CST;
-          if (it >= CST && !bar_wait(&empty[s], (it / CST - 1) & 1)) {
+        const int n = tl / a.tiles_img, r = tl - n * a.tiles_img, ty = r / a.tiles_x, tx = r - ty * a.tiles_x;
+        for (int t = 0; t < boxes; ++t, ++it) {
+          if (it >= stages && !bar_wait(&empty[s], phase)) {
             ok = false;
             break;
           }
-          bar_expect(&full[s], kTapBytes);
-          if (MATRIX) {
-            tma2d(sA + s * kTapBytes, &mapA, 64 * t, tl * CBM, &full[s]);
-          } else {
-            const int ky = DGRAD ? 2 - t / 3 : t / 3, kx = DGRAD ? 2 - t % 3 : t % 3;
-            tma_im2col(sA + s * kTapBytes, &mapA, tl * CBM, a.h, a.w, a.dil, kx * a.dil, ky * a.dil, &full[s]);
+          bar_expect(&full[s], a.box);
+          if (MATRIX)
+            tma2d(sA + s * a.box, &mapA, 64 * t, tl * CBM, &full[s]);
+          else  // columns shifted by the tap's, rows from dil above the tile on
+            tma_image(sA + s * a.box, &mapA, CTW * tx + (DGRAD ? 1 - t : t - 1) * a.dil, CTH * ty - a.dil, n, &full[s]);
+          if (++s == stages) {
+            s = 0;
+            phase ^= 1;
           }
         }
       }
       if (!ok) {
         fail = 1;
         atomicCAS(a.status, 0, ST_CUDA);
-        for (int k = 1; k <= CST && it - k >= 0; ++k) bar_wait(&full[(it - k) % CST], ((it - k) / CST) & 1);
+        for (int k = 1; k <= stages && it - k >= 0; ++k) bar_wait(&full[(it - k) % stages], ((it - k) / stages) & 1);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = idesc_bf16(CBM, N);
-      const int rounds = DGRAD ? kt : 1, per = DGRAD ? 1 : kt;
+      const uint32_t a0 = desc_lo(su32(sA)), b0 = desc_lo(su32(sB));
+      const uint32_t box = a.box >> 4, row = a.dil * (CTW * 128 >> 4);  // a box, dil of its rows
       bool ok = bar_wait(wbar, 0);
-      int it = 0, r = 0;
-      for (int tl = blockIdx.x; ok && tl < tiles; tl += gridDim.x) {
-        for (int q = 0; ok && q < rounds; ++q, ++r) {
-          const int b = r % NACC;
-          if (r >= NACC && !bar_wait(&acc_empty[b], (r / NACC - 1) & 1)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          for (int k = 0; k < per; ++k, ++it) {
-            const int s = it % CST;
-            if (!bar_wait(&full[s], (it / CST) & 1)) {
-              ok = false;
-              break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned char* wt = sB + (DGRAD ? q : k) * N * 128;
+      int s = 0, phase = 0;                 // ring position of the next box and its parity
+      int acc = 0, acc_phase = 1;           // next accumulator; the parity of the phase before it
+      int it = 0, freed = 0;                // boxes taken, and released
+      // one lane's loop over 36 MMAs per tile: descriptors and ring positions advance by additions
+      auto take = [&](uint32_t& lo) {       // wait for the next box; its operand's descriptor
+        if (!bar_wait(&full[s], phase)) return false;
+        lo = a0 + s * box;
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1;
+        }
+        ++it;
+        return true;
+      };
+      auto mmas = [&](uint32_t at, uint32_t wt, bool first) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              mma_bf16(tmem + b * N, sdesc_sw128(sA + s * kTapBytes + kk * 32), sdesc_sw128(wt + kk * 32), idesc,
-                       (k > 0 || kk > 0) ? 1u : 0u);
-            mma_commit(&empty[s]);
+        for (int kk = 0; kk < 4; ++kk) mma_bf16_lo(tmem + acc * N, at + 2 * kk, wt + 2 * kk, idesc, !first || kk > 0);
+      };
+      auto open = [&]() {                   // wait until the next accumulator has been read
+        if (!bar_wait(&acc_empty[acc], acc_phase)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return true;
+      };
+      auto close = [&]() {
+        mma_commit(&acc_full[acc]);
+        if (++acc == NACC) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+      };
+      for (int tl = blockIdx.x; ok && tl < tiles; tl += gridDim.x) {
+        if constexpr (MATRIX) {
+          if (!(ok = open())) break;
+          for (int t = 0; ok && t < kt; ++t) {
+            const int at = s;
+            uint32_t lo;
+            if (!(ok = take(lo))) break;
+            mmas(lo, b0 + t * (N * 128 >> 4), t == 0);
+            mma_commit(&empty[at]);
+            freed = it;
           }
-          if (ok) mma_commit(&acc_full[b]);
+          if (ok) close();
+        } else {
+          int at[3];
+          uint32_t lo[3];
+#pragma unroll
+          for (int t = 0; t < 9; ++t) {
+            if ((DGRAD || t == 0) && !(ok = open())) break;
+            if (t < 3) {
+              at[t] = s;
+              if (!(ok = take(lo[t]))) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            mmas(lo[t % 3] + (DGRAD ? 2 - t / 3 : t / 3) * row, b0 + t * (N * 128 >> 4), DGRAD || t == 0);
+            if (t >= 6) {
+              mma_commit(&empty[at[t - 6]]);
+              freed = it - 8 + t;
+            }
+            if (DGRAD || t == 8) close();
+          }
         }
       }
       if (!ok) {
         fail = 1;
         atomicCAS(a.status, 0, ST_CUDA);
-        for (int k = 1; k <= CST && it - k >= 0; ++k) bar_wait(&empty[(it - k) % CST], ((it - k) / CST) & 1);
+        for (int k = 1; k <= stages && freed - k >= 0; ++k) bar_wait(&empty[(freed - k) % stages], ((freed - k) / stages) & 1);
       }
     }
     __syncwarp();
@@ -221,7 +272,13 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
     bool ok = true;
     int r = 0;
     for (int tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
-      const long m0 = static_cast<long>(tl) * CBM;
+      const int n = tl / a.tiles_img, rr = tl - n * a.tiles_img, ty = rr / a.tiles_x, tx = rr - ty * a.tiles_x;
+      // linear pixel of a row of the tile; -1 outside the image
+      auto pixel = [&](int i) -> long {
+        if (MATRIX) return static_cast<long>(tl) * CBM + i < a.M ? static_cast<long>(tl) * CBM + i : -1;
+        const int y = CTH * ty + i / CTW, x = CTW * tx + i % CTW;
+        return y < a.h && x < a.w ? (static_cast<long>(n) * a.h + y) * a.w + x : -1;
+      };
       if constexpr (MODE == EPI_OUT1) {
         const int b = r % NACC;
         ok = __all_sync(0xffffffffu, bar_wait(&acc_full[b], (r / NACC) & 1));
@@ -231,7 +288,8 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
           uint32_t v;
           asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(lane_addr + b * N));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (m0 + row < a.M) a.out32[m0 + row] = __uint_as_float(v);
+          const long m = pixel(row);
+          if (m >= 0) a.out32[m] = __uint_as_float(v);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -245,12 +303,12 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
         const int e = et + 32 * CEPI * k;
-        const long m = m0 + e / 16;
+        const long m = pixel(e / 16);
         const long o = m * 64 + 4 * (e % 16);
         if (MODE == EPI_RESID || MODE == EPI_ACC || MODE == EPI_ACC_MASK)
-          add[k] = m < a.M ? *reinterpret_cast<const float4*>(a.add32 + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+          add[k] = m >= 0 ? *reinterpret_cast<const float4*>(a.add32 + o) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (MODE == EPI_MASK16 || MODE == EPI_ACC_MASK)
-          msk[k] = m < a.M ? *reinterpret_cast<const uint2*>(a.mask16 + o) : make_uint2(0, 0);
+          msk[k] = m >= 0 ? *reinterpret_cast<const uint2*>(a.mask16 + o) : make_uint2(0, 0);
       }
       float v[32];
       if (DGRAD) {
@@ -284,8 +342,8 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
         const int e = et + 32 * CEPI * k;
-        const long m = m0 + e / 16;
-        if (m >= a.M) continue;
+        const long m = pixel(e / 16);
+        if (m < 0) continue;
         const int c = 4 * (e % 16);
         const long o = m * 64 + c;
         float4 y = *reinterpret_cast<const float4*>(tile + (e / 16) * CLD + c);
@@ -336,18 +394,6 @@ struct WgradArgs {
   int* status;
 };
 
-// MN-major descriptor with the 128-byte swizzle: 64 channels (128 bytes) per pixel row, 8 pixel rows
-// per 1024-byte atom; `lbo` is the distance between 64-channel blocks.
-__device__ __forceinline__ uint64_t sdesc_mn_sw128(const void* p, unsigned lbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((su32(p) >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>(lbo >> 4) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
 template <bool MATRIX>  // x is a matrix [M][kdim] of columns instead of activations read per tap
 __global__ void __launch_bounds__(WTHR, 3) wgrad_kernel(const __grid_constant__ CUtensorMap mapX,
                                                         const __grid_constant__ CUtensorMap mapY,
@@ -384,6 +430,7 @@ __global__ void __launch_bounds__(WTHR, 3) wgrad_kernel(const __grid_constant__ 
   const uint32_t tmem = *tmem_slot;
 
   if (tid == 0 && KT > 0) {
+    Pixel pos(MATRIX ? 0 : kt0 * 64, g.h, g.w);  // of the next tile to load
     auto load = [&](int i) {
       const int s = i % WST, px = (kt0 + i) * 64;
       unsigned char* st = smem + s * kWStage;
@@ -393,9 +440,10 @@ __global__ void __launch_bounds__(WTHR, 3) wgrad_kernel(const __grid_constant__ 
         if (MATRIX)
           tma2d(st + j * kWTile, &mapX, 64 * t, px, &full[s]);
         else
-          tma_im2col(st + j * kWTile, &mapX, px, g.h, g.w, g.dil, (t % 3) * g.dil, (t / 3) * g.dil, &full[s]);
+          tma_im2col(st + j * kWTile, &mapX, pos, g.dil, (t % 3) * g.dil, (t / 3) * g.dil, &full[s]);
       }
       tma2d(st + 2 * kWTile, &mapY, 0, px, &full[s]);
+      if (!MATRIX) pos.advance(64, g.h, g.w);
     };
     for (int i = 0; i < KT && i < WST; ++i) load(i);
     constexpr uint32_t idesc = idesc_bf16(128, 64) | (1u << 15) | (1u << 16);  // both operands MN-major
@@ -408,11 +456,12 @@ __global__ void __launch_bounds__(WTHR, 3) wgrad_kernel(const __grid_constant__ 
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const unsigned char* st = smem + s * kWStage;
+      // MN-major operands: 64 channels (128 bytes) per pixel row, 8 pixel rows per 1024-byte atom, 64-channel
+      // blocks kWTile apart
+      const uint32_t lo = desc_lo(su32(smem + s * kWStage), kWTile);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)  // 16 pixels = two 8-row atoms further
-        mma_bf16(tmem, sdesc_mn_sw128(st + kk * 2048, kWTile), sdesc_mn_sw128(st + 2 * kWTile + kk * 2048, kWTile), idesc,
-                 (i > 0 || kk > 0) ? 1u : 0u);
+        mma_bf16_lo(tmem, lo + (kk * 2048 >> 4), lo + ((2 * kWTile + kk * 2048) >> 4), idesc, i > 0 || kk > 0);
       mma_commit(&empty[s]);
       if (i >= 1 && i - 1 + WST < KT) {  // refill the stage of the tile before: its MMAs are mostly done
         const int p = i - 1;
@@ -510,9 +559,8 @@ int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const ConvArgs& a,
   if (sms < 1) return report_error(WG_ERR_CUDA, "no device");
   const int rc = allow_smem(conv_kernel<MODE>, kConvSmem);
   if (rc != WG_OK) return rc;
-  const int tiles = (a.M + CBM - 1) / CBM;
   note_launch();
-  conv_kernel<MODE><<<tiles < sms ? tiles : sms, CTHR, kConvSmem, st>>>(ma, mb, a);
+  conv_kernel<MODE><<<a.tiles < sms ? a.tiles : sms, CTHR, kConvSmem, st>>>(ma, mb, a);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? WG_OK : report_error(WG_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -520,7 +568,7 @@ int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const ConvArgs& a,
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 bool bad_image(int batch, int h, int w, int dil) {
-  return batch < 1 || h < 1 || w < 1 || dil < 1 || dil > 60 || static_cast<long>(batch) * h * w > (1L << 30);
+  return batch < 1 || h < 1 || w < 1 || dil < 1 || dil > kMaxDil || static_cast<long>(batch) * h * w > (1L << 30);
 }
 
 }  // namespace
@@ -553,8 +601,15 @@ int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, co
   a.out32 = d_out32;
   a.out16 = static_cast<__nv_bfloat16*>(d_out16);
   a.status = d_status;
+  a.tiles_x = (w + CTW - 1) / CTW;
+  a.tiles_img = a.tiles_x * ((h + CTH - 1) / CTH);
+  a.tiles = matrix ? (a.M + CBM - 1) / CBM : batch * a.tiles_img;
+  if (matrix) a.tiles_x = a.tiles_img = a.tiles;  // not an image: one row of tiles
+  const int rows = CTH + 2 * dil;
+  a.box = matrix ? kTapBytes : rows * CTW * 128;
+  a.stages = std::min<int>(CST, kRing / a.box);
   CUtensorMap ma, mb;
-  int rc = matrix ? map_bf16(&ma, d_act, a.M, kp, CBM) : map_im2col(&ma, d_act, batch, h, w, dil, CBM);
+  int rc = matrix ? map_bf16(&ma, d_act, a.M, kp, CBM) : map_image(&ma, d_act, batch, h, w, rows);
   if (rc != WG_OK) return rc;
   // weights: [n][kp] (boxes of 64 k x n rows), or for the data gradient [kp][64] (64 x 64 boxes)
   rc = dgrad ? map_bf16(&mb, d_wgt, kp, 64, 64) : map_bf16(&mb, d_wgt, 64, kp, mode == EPI_OUT1 ? 16 : 64);
