@@ -219,6 +219,13 @@ int wg_pc_mse(const float* d_out, int ld, const float* d_target, float scale, lo
  * refresh the bf16 copies. */
 int wg_pc_adam(const float* d_partial, int splits, int n, int kp, float* d_w32, float* d_m1, float* d_m2, float lr,
                float b1, float b2, float eps, int step, void* d_w_bf16, void* d_wt_bf16, void* stream);
+/* The same for up to 16 layers in one launch; the arguments are host arrays of `layers` entries
+ * (d_partial or one of its entries NULL: only refresh that layer's bf16 copies). d_grad: NULL, or per
+ * layer NULL or where the summed gradient [n][kp] goes. */
+int wg_pc_adam_layers(int layers, const float* const* d_partial, const int* splits, const int* n, const int* kp,
+                      float* const* d_w32, float* const* d_m1, float* const* d_m2, float* const* d_grad,
+                      void* const* d_w_bf16, void* const* d_wt_bf16, float lr, float b1, float b2, float eps, int step,
+                      void* stream);
 
 /* Same-padded 3x3 convolution (dilation dil <= 10) of activations [batch][h][w][64] bf16 with a fused
  * epilogue; y is the FP32 result per pixel and channel. mode

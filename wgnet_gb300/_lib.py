@@ -83,6 +83,7 @@ SIGNATURES: dict[str, tuple] = {
     "wg_pc_features": (_I, [_P, _P, _P, _I, _I, _I, _P, _P, _P]),
     "wg_pc_mse": (_I, [_P, _I, _P, _F, ctypes.c_long, _P, _P, _P]),
     "wg_pc_adam": (_I, [_P, _I, _I, _I, _P, _P, _P, _F, _F, _F, _F, _I, _P, _P, _P]),
+    "wg_pc_adam_layers": (_I, [_I] + [_P] * 10 + [_F, _F, _F, _F, _I, _P]),
     "wg_render_fwd_dev": (_I, [_P, _I, _P, _P]),
     "wg_render_bwd_dev": (_I, [_P, _P, _I, _P, _P]),
     "wg_profile": (_I, [_P, _I]),

@@ -162,30 +162,44 @@ __global__ void mse_kernel(const float* __restrict__ out, int ld, const float* _
 }
 
 // Adam on FP32 master weights w32 [N][Kp]; the gradient is the sum, in split order, of the partials
-// of the transposed weight gradient [S][Kp][N]. Writes the BF16 weights [N][Kp] and their transpose.
-// Reading the partials bounds it (9.3 MB for 63 splits of a 64 -> 64 layer), so a warp takes 32
-// neighbouring n of one k: 128-byte lines of the partials, against which the strided accesses to the
-// four weight-sized arrays are few (with neighbouring k per warp it read eight times the bytes).
-__global__ void adam_kernel(const float* __restrict__ partial, int S, int N, int Kp, float* __restrict__ w32,
-                            float* __restrict__ m1, float* __restrict__ m2, float lr, float b1, float b2, float eps,
-                            float c1, float c2, __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt) {
+// of the transposed weight gradient [S][Kp][N], kept in grad [N][Kp] if given. Writes the BF16 weights
+// [N][Kp] and their transpose. All layers in one launch (blockIdx.y). Reading the partials bounds it (110
+// MB for 63 splits of the network), so a warp takes 32 neighbouring n of one k: 128-byte lines of the
+// partials, against which the strided accesses to the weight-sized arrays are few (with neighbouring k
+// per warp it read eight times the bytes; one launch per layer left most SMs idle: 13 x 8.6 us).
+constexpr int kAdamLayers = 16;
+struct AdamLayer {
+  const float* partial;
+  float *w32, *m1, *m2, *grad;
+  __nv_bfloat16 *w, *wt;
+  int S, N, Kp;
+};
+struct AdamArgs {
+  AdamLayer layer[kAdamLayers];
+  float lr, b1, b2, eps, c1, c2;
+};
+
+__global__ void adam_kernel(const __grid_constant__ AdamArgs a) {
+  const AdamLayer& L = a.layer[blockIdx.y];
   const long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  const int N = L.N, Kp = L.Kp;
   if (t >= static_cast<long>(N) * Kp) return;
   const int n = static_cast<int>(t % N), k = static_cast<int>(t / N);
   const long i = static_cast<long>(n) * Kp + k;
   float g = 0.0f;
-  if (partial) {
-#pragma unroll 8
-    for (int s = 0; s < S; ++s) g += partial[static_cast<long>(s) * Kp * N + t];
-    const float a = b1 * m1[i] + (1.0f - b1) * g;
-    const float v = b2 * m2[i] + (1.0f - b2) * g * g;
-    m1[i] = a;
-    m2[i] = v;
-    w32[i] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+  if (L.partial) {
+#pragma unroll 16
+    for (int s = 0; s < L.S; ++s) g += __ldcs(L.partial + static_cast<long>(s) * Kp * N + t);
+    const float m = a.b1 * L.m1[i] + (1.0f - a.b1) * g;
+    const float v = a.b2 * L.m2[i] + (1.0f - a.b2) * g * g;
+    L.m1[i] = m;
+    L.m2[i] = v;
+    L.w32[i] -= a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+    if (L.grad) L.grad[i] = g;
   }
-  const __nv_bfloat16 q = __float2bfloat16(w32[i]);
-  w[i] = q;
-  wt[t] = q;
+  const __nv_bfloat16 q = __float2bfloat16(L.w32[i]);
+  L.w[i] = q;
+  L.wt[t] = q;
 }
 
 inline unsigned blocks(long n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
@@ -262,16 +276,36 @@ int wg_pc_mse(const float* out, int ld, const float* target, float scale, long M
                                                                                      dout));
 }
 
+int wg_pc_adam_layers(int layers, const float* const* partial, const int* splits, const int* n, const int* kp,
+                      float* const* w32, float* const* m1, float* const* m2, float* const* grad, void* const* w,
+                      void* const* wt, float lr, float b1, float b2, float eps, int step, void* stream) {
+  if (layers < 1 || layers > kAdamLayers || !n || !kp || !w32 || !m1 || !m2 || !w || !wt || (partial && !splits))
+    return wg::report_error(WG_ERR_ARG, "adam: bad argument");
+  AdamArgs a{};
+  long most = 0;
+  bool steps = false;
+  for (int i = 0; i < layers; ++i) {
+    const float* p = partial ? partial[i] : nullptr;
+    if (!w32[i] || !m1[i] || !m2[i] || !w[i] || !wt[i] || n[i] < 1 || kp[i] < 1 || (p && (splits[i] < 1 || step < 1)))
+      return wg::report_error(WG_ERR_ARG, "adam: bad argument");
+    a.layer[i] = {p, w32[i], m1[i], m2[i], grad ? grad[i] : nullptr, static_cast<__nv_bfloat16*>(w[i]),
+                  static_cast<__nv_bfloat16*>(wt[i]), p ? splits[i] : 0, n[i], kp[i]};
+    const long c = static_cast<long>(n[i]) * kp[i];
+    most = c > most ? c : most;
+    steps = steps || p;
+  }
+  a.lr = lr;
+  a.b1 = b1;
+  a.b2 = b2;
+  a.eps = eps;
+  a.c1 = steps ? 1.0f - powf(b1, static_cast<float>(step)) : 1.0f;
+  a.c2 = steps ? 1.0f - powf(b2, static_cast<float>(step)) : 1.0f;
+  PC_LAUNCH(adam_kernel<<<dim3(blocks(most, 256), layers), 256, 0, static_cast<cudaStream_t>(stream)>>>(a));
+}
+
 int wg_pc_adam(const float* partial, int S, int N, int Kp, float* w32, float* m1, float* m2, float lr, float b1,
                float b2, float eps, int step, void* w, void* wt, void* stream) {
-  if (!w32 || !m1 || !m2 || !w || !wt || N < 1 || Kp < 1 || (partial && (S < 1 || step < 1)))
-    return wg::report_error(WG_ERR_ARG, "adam: bad argument");
-  const float c1 = partial ? 1.0f - powf(b1, static_cast<float>(step)) : 1.0f;
-  const float c2 = partial ? 1.0f - powf(b2, static_cast<float>(step)) : 1.0f;
-  const long n = static_cast<long>(N) * Kp;
-  PC_LAUNCH(adam_kernel<<<blocks(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      partial, S, N, Kp, w32, m1, m2, lr, b1, b2, eps, c1, c2, static_cast<__nv_bfloat16*>(w),
-      static_cast<__nv_bfloat16*>(wt)));
+  return wg_pc_adam_layers(1, &partial, &S, &N, &Kp, &w32, &m1, &m2, nullptr, &w, &wt, lr, b1, b2, eps, step, stream);
 }
 
 }  // extern "C"

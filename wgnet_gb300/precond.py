@@ -97,10 +97,31 @@ class UpdateNet:
                                  torch.empty((n, kp), device=dev, dtype=torch.bfloat16),
                                  torch.empty((kp, n), device=dev, dtype=torch.bfloat16)))
 
+    def _adam(self, parts=None, grads=None, lr: float = 0.0):
+        """One Adam step of every layer from its gradient partials (which also leaves the summed gradients
+        in `grads`), or, without partials, a refresh of the bf16 weights."""
+        n = len(self.layers)
+
+        def array(kind, values):
+            return (kind * n)(*values)
+
+        def ptrs(tensors):
+            return array(ctypes.c_void_p, [t.data_ptr() for t in tensors])
+
+        Ls = self.layers
+        check(self._lib.wg_pc_adam_layers(
+            n, ptrs([parts[L.name] for L in Ls]) if parts else None,
+            array(ctypes.c_int, [parts[L.name].shape[0] for L in Ls]) if parts else None,
+            array(ctypes.c_int, [L.n for L in Ls]), array(ctypes.c_int, [L.kp for L in Ls]), ptrs([L.w32 for L in Ls]),
+            ptrs([L.m1 for L in Ls]), ptrs([L.m2 for L in Ls]), ptrs([grads[L.name] for L in Ls]) if grads else None,
+            ptrs([L.w for L in Ls]), ptrs([L.wt for L in Ls]), float(lr), 0.9, 0.999, 1e-8, self.step, _stream()), "adam")
+
+    def _by_layer(self, flat) -> dict:
+        sizes = [L.n * L.kp for L in self.layers]
+        return {L.name: t.view(L.n, L.kp) for L, t in zip(self.layers, flat.split(sizes))}
+
     def _sync_bf16(self):
-        for L in self.layers:
-            check(self._lib.wg_pc_adam(None, 0, L.n, L.kp, _p(L.w32), _p(L.m1), _p(L.m2), 0.0, 0.0, 0.0, 0.0, 0,
-                                       _p(L.w), _p(L.wt), _stream()), "adam")
+        self._adam()
 
     @property
     def parameters(self) -> int:
@@ -253,11 +274,9 @@ class UpdateNet:
         Li = self.layers[0]
         parts["in"] = self._wgrad(Li, s["col0"], dh16, shape, splits, columns=Li.kp)
         self.step += 1
-        for L in self.layers:
-            p = parts[L.name]
-            check(self._lib.wg_pc_adam(_p(p), p.shape[0], L.n, L.kp, _p(L.w32), _p(L.m1), _p(L.m2), float(lr), 0.9,
-                                       0.999, 1e-8, self.step, _p(L.w), _p(L.wt), _stream()), "adam")
-        self._last_parts = parts
+        flat = torch.empty(sum(L.n * L.kp for L in self.layers), device=self.device, dtype=torch.float32)
+        self._adam(parts, self._by_layer(flat), lr)
+        self._last_grads = flat
         self._saved = None
         self.last_activations = None
         return float(loss.item())
@@ -268,7 +287,7 @@ class UpdateNet:
 
     def weight_gradients(self) -> dict:
         """{layer: dL/dW [n][kp]} of the last train_step (for tests)."""
-        return {k: p.sum(0).t().contiguous() for k, p in self._last_parts.items()}
+        return self._by_layer(self._last_grads.clone())
 
 
 __all__ = ["UpdateNet", "BANDS", "band_index", "DILATIONS", "OUT_SCALE"]
