@@ -249,7 +249,8 @@ int wg_pc_conv(int mode, const void* d_act_bf16, int batch, int h, int w, int di
 int wg_pc_conv_wgrad(const void* d_act_bf16, int columns, const void* d_dy_bf16, int batch, int h, int w, int dil,
                      int splits, float* d_partial, int* d_status, void* stream);
 /* Data gradient of a 64 -> 1 convolution: dh [pixels][64] and its bf16 copy from dL/dy [pixels] and
- * column 0 of the transposed weights [576][64]; dout16[pixel][0] = bf16(dL/dy). */
+ * column 0 of the transposed weights [576][64]; dout16 [pixels][64] = bf16(dL/dy) in channel 0, zero
+ * elsewhere. */
 int wg_pc_out_dgrad(const float* d_dout, const void* d_wt_bf16, int batch, int h, int w, float* d_dh, void* d_dh16,
                     void* d_dout16, void* stream);
 

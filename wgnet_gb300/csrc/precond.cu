@@ -17,24 +17,28 @@
 
 namespace {
 
-__global__ void im2col_kernel(const __nv_bfloat16* __restrict__ act, int B, int H, int W, int C, int dil, int Kp,
+// One block per image row and 32-bit arithmetic: writing the columns bounds it (40 MB for 32 images of
+// 70 x 70 with 8 channels, 6 us at the HBM rate, now 12); with 64-bit
+// divisions for each 16 bytes it took 21.
+__global__ void im2col_kernel(const __nv_bfloat16* __restrict__ act, int H, int W, int C, int dil, int Kp,
                               __nv_bfloat16* __restrict__ col) {
-  const long M = static_cast<long>(B) * H * W;
-  const int kv = Kp / 8;
-  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (i >= M * kv) return;
-  const long m = i / kv;
-  const int k8 = static_cast<int>(i % kv) * 8;
-  uint4 v = make_uint4(0, 0, 0, 0);
-  if (k8 < 9 * C) {
-    const int tap = k8 / C, c = k8 % C;
-    const int x = static_cast<int>(m % W), y = static_cast<int>((m / W) % H);
-    const long b = m / (static_cast<long>(W) * H);
-    const int ys = y + (tap / 3 - 1) * dil, xs = x + (tap % 3 - 1) * dil;
-    if (ys >= 0 && ys < H && xs >= 0 && xs < W)
-      v = *reinterpret_cast<const uint4*>(act + ((b * H + ys) * W + xs) * C + c);
+  const long row = blockIdx.x;  // b H + y
+  const int y = static_cast<int>(row % H);
+  const unsigned kv = Kp / 8, n = W * kv;
+  const __nv_bfloat16* in = act + row * W * C;
+  uint4* out = reinterpret_cast<uint4*>(col + row * W * Kp);
+  for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned x = i / kv, k8 = (i - x * kv) * 8;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (k8 < 9u * C) {
+      const unsigned tap = k8 / C, c = k8 - tap * C, ty = tap / 3;
+      const int dy = (static_cast<int>(ty) - 1) * dil, dx = (static_cast<int>(tap - 3 * ty) - 1) * dil;
+      const int xs = static_cast<int>(x) + dx;
+      if (y + dy >= 0 && y + dy < H && xs >= 0 && xs < W)
+        v = *reinterpret_cast<const uint4*>(in + (static_cast<long>(dy) * W + xs) * C + c);
+    }
+    out[i] = v;
   }
-  *reinterpret_cast<uint4*>(col + m * Kp + k8) = v;
 }
 
 // dact[m][c] (+)= sum over taps of dcol[m'][tap C + c], m' the pixel whose tap reads m.
@@ -103,19 +107,23 @@ __global__ void relu_grad_kernel(const float* __restrict__ d, const __nv_bfloat1
   out[i] = __bfloat162float(mask[i]) > 0.0f ? d[i] : 0.0f;
 }
 
-// Per-sample RMS of the gradient (f64 reduction, one block per sample).
-__global__ void rms_kernel(const float* __restrict__ g, int P, float* __restrict__ rms) {
-  __shared__ double red[256];
+// Per-sample RMS of the gradient (f64 reduction, one block per sample: its chain of f64 additions
+// bounds it, so 1024 threads take few terms each and the warps reduce in registers: 70 x 70 in 9.8 us, in
+// 15.6 with 256 threads and a tree in shared memory).
+constexpr int kRmsThreads = 1024;
+__global__ void __launch_bounds__(kRmsThreads) rms_kernel(const float* __restrict__ g, int P, float* __restrict__ rms) {
+  __shared__ double red[32];
   const float* x = g + static_cast<long>(blockIdx.x) * P;
   double s = 0.0;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) s += static_cast<double>(x[i]) * x[i];
-  red[threadIdx.x] = s;
+  for (int i = threadIdx.x; i < P; i += kRmsThreads) s += static_cast<double>(x[i]) * x[i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) rms[blockIdx.x] = static_cast<float>(sqrt(s / P));
   }
-  if (threadIdx.x == 0) rms[blockIdx.x] = static_cast<float>(sqrt(red[0] / P));
 }
 
 // Input features [B][H][W][8]: (v - 3) km/s, g / rms(g), one-hot band (4), depth z / H, 0.
@@ -163,10 +171,11 @@ __global__ void mse_kernel(const float* __restrict__ out, int ld, const float* _
 
 // Adam on FP32 master weights w32 [N][Kp]; the gradient is the sum, in split order, of the partials
 // of the transposed weight gradient [S][Kp][N], kept in grad [N][Kp] if given. Writes the BF16 weights
-// [N][Kp] and their transpose. All layers in one launch (blockIdx.y). Reading the partials bounds it (110
-// MB for 63 splits of the network), so a warp takes 32 neighbouring n of one k: 128-byte lines of the
-// partials, against which the strided accesses to the weight-sized arrays are few (with neighbouring k
-// per warp it read eight times the bytes; one launch per layer left most SMs idle: 13 x 8.6 us).
+// [N][Kp] and their transpose. All layers in one launch (blockIdx.y; one launch per layer left most SMs
+// idle: 14 x 8.6 us). Reading the partials bounds it (110 MB for 63 splits of the network): a warp sums
+// 32 neighbouring n of one k, 128-byte lines; a tile of 32 n x 8 k then turns over in shared memory so
+// that every other access is whole 32-byte sectors too (from the summing layout each took 4 bytes of a
+// sector: 94 us; now 23, 19 of them the partials at the HBM rate).
 constexpr int kAdamLayers = 16;
 struct AdamLayer {
   const float* partial;
@@ -179,27 +188,55 @@ struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;
 };
 
-__global__ void adam_kernel(const __grid_constant__ AdamArgs a) {
+constexpr int ATN = 32, ATK = 8;  // tile of a block
+
+__global__ void __launch_bounds__(ATN * ATK) adam_kernel(const __grid_constant__ AdamArgs a) {
+  __shared__ float gs[ATN][ATK + 1];
+  __shared__ __nv_bfloat16 qs[ATK][ATN + 2];
   const AdamLayer& L = a.layer[blockIdx.y];
-  const long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  const int N = L.N, Kp = L.Kp;
-  if (t >= static_cast<long>(N) * Kp) return;
-  const int n = static_cast<int>(t % N), k = static_cast<int>(t / N);
-  const long i = static_cast<long>(n) * Kp + k;
-  float g = 0.0f;
+  const int N = L.N, Kp = L.Kp, across = (N + ATN - 1) / ATN;
+  const int n0 = static_cast<int>(blockIdx.x % across) * ATN;
+  const long k0 = static_cast<long>(blockIdx.x / across) * ATK;
+  if (k0 >= Kp) return;
+  const int tn = threadIdx.x % ATN, tk = threadIdx.x / ATN;  // summing layout
+  const bool in = n0 + tn < N && k0 + tk < Kp;
+  const long t = (k0 + tk) * N + n0 + tn;
   if (L.partial) {
-#pragma unroll 16
-    for (int s = 0; s < L.S; ++s) g += __ldcs(L.partial + static_cast<long>(s) * Kp * N + t);
-    const float m = a.b1 * L.m1[i] + (1.0f - a.b1) * g;
-    const float v = a.b2 * L.m2[i] + (1.0f - a.b2) * g * g;
-    L.m1[i] = m;
-    L.m2[i] = v;
-    L.w32[i] -= a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
-    if (L.grad) L.grad[i] = g;
+    float g = 0.0f;
+    if (in) {
+      const float* p = L.partial + t;
+      const long step = static_cast<long>(Kp) * N;
+      for (int s = 0; s < L.S; s += 16) {  // whole rounds of 16 loads in flight, also at the end
+        float v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = s + u < L.S ? __ldcs(p + (s + u) * step) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) g = s + u < L.S ? g + v[u] : g;
+      }
+    }
+    gs[tn][tk] = g;
+    __syncthreads();
   }
-  const __nv_bfloat16 q = __float2bfloat16(L.w32[i]);
-  L.w[i] = q;
-  L.wt[t] = q;
+  const int un = threadIdx.x / ATK, uk = threadIdx.x % ATK;  // updating layout
+  if (n0 + un < N && k0 + uk < Kp) {
+    const long i = static_cast<long>(n0 + un) * Kp + k0 + uk;
+    float w = L.w32[i];
+    if (L.partial) {
+      const float g = gs[un][uk];
+      const float m = a.b1 * L.m1[i] + (1.0f - a.b1) * g;
+      const float v = a.b2 * L.m2[i] + (1.0f - a.b2) * g * g;
+      L.m1[i] = m;
+      L.m2[i] = v;
+      w -= a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+      L.w32[i] = w;
+      if (L.grad) L.grad[i] = g;
+    }
+    const __nv_bfloat16 q = __float2bfloat16(w);
+    L.w[i] = q;
+    qs[uk][un] = q;
+  }
+  __syncthreads();
+  if (in) L.wt[t] = qs[tk][tn];
 }
 
 inline unsigned blocks(long n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
@@ -220,9 +257,8 @@ extern "C" {
 int wg_pc_im2col(const void* act, int B, int H, int W, int C, int dil, int Kp, void* col, void* stream) {
   if (!act || !col || B < 1 || H < 1 || W < 1 || C < 8 || C % 8 || Kp % 64 || Kp < 9 * C || dil < 1)
     return wg::report_error(WG_ERR_ARG, "im2col: bad shape");
-  const long n = static_cast<long>(B) * H * W * (Kp / 8);
-  PC_LAUNCH(im2col_kernel<<<blocks(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(act), B, H, W, C, dil, Kp, static_cast<__nv_bfloat16*>(col)));
+  PC_LAUNCH(im2col_kernel<<<static_cast<unsigned>(static_cast<long>(B) * H), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(act), H, W, C, dil, Kp, static_cast<__nv_bfloat16*>(col)));
 }
 
 int wg_pc_col2im(const float* dcol, int B, int H, int W, int C, int dil, int Kp, float* dact, int accumulate,
@@ -263,7 +299,7 @@ int wg_pc_features(const float* vel_km, const float* grad, const int* band, int 
   if (!vel_km || !grad || !band || !rms || !out || B < 1) return wg::report_error(WG_ERR_ARG, "features: bad argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   wg::note_launch();
-  rms_kernel<<<B, 256, 0, st>>>(grad, H * W, rms);
+  rms_kernel<<<B, kRmsThreads, 0, st>>>(grad, H * W, rms);
   const long n = static_cast<long>(B) * H * W;
   PC_LAUNCH(features_kernel<<<blocks(n, 256), 256, 0, st>>>(vel_km, grad, rms, band, B, H, W,
                                                             static_cast<__nv_bfloat16*>(out)));
@@ -290,8 +326,8 @@ int wg_pc_adam_layers(int layers, const float* const* partial, const int* splits
       return wg::report_error(WG_ERR_ARG, "adam: bad argument");
     a.layer[i] = {p, w32[i], m1[i], m2[i], grad ? grad[i] : nullptr, static_cast<__nv_bfloat16*>(w[i]),
                   static_cast<__nv_bfloat16*>(wt[i]), p ? splits[i] : 0, n[i], kp[i]};
-    const long c = static_cast<long>(n[i]) * kp[i];
-    most = c > most ? c : most;
+    const long tiles = static_cast<long>((n[i] + ATN - 1) / ATN) * ((kp[i] + ATK - 1) / ATK);
+    most = tiles > most ? tiles : most;
     steps = steps || p;
   }
   a.lr = lr;
@@ -300,7 +336,7 @@ int wg_pc_adam_layers(int layers, const float* const* partial, const int* splits
   a.eps = eps;
   a.c1 = steps ? 1.0f - powf(b1, static_cast<float>(step)) : 1.0f;
   a.c2 = steps ? 1.0f - powf(b2, static_cast<float>(step)) : 1.0f;
-  PC_LAUNCH(adam_kernel<<<dim3(blocks(most, 256), layers), 256, 0, static_cast<cudaStream_t>(stream)>>>(a));
+  PC_LAUNCH(adam_kernel<<<dim3(static_cast<unsigned>(most), layers), ATN * ATK, 0, static_cast<cudaStream_t>(stream)>>>(a));
 }
 
 int wg_pc_adam(const float* partial, int S, int N, int Kp, float* w32, float* m1, float* m2, float lr, float b1,

@@ -257,7 +257,7 @@ class UpdateNet:
         Lo = self.layers[-1]
         dh = torch.empty((M, CH), device=self.device, dtype=torch.float32)
         dh16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
-        dout16 = torch.zeros((M, CH), device=self.device, dtype=torch.bfloat16)
+        dout16 = torch.empty((M, CH), device=self.device, dtype=torch.bfloat16)
         check(self._lib.wg_pc_out_dgrad(_p(dout), _p(Lo.wt), B, H, W, _p(dh), _p(dh16), _p(dout16), _stream()), "out dgrad")
         parts["out"] = self._wgrad(Lo, s["hlast"], dout16, shape, splits)
         t16 = dout16  # read for the last time above
