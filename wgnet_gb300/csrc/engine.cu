@@ -331,11 +331,14 @@ int find_shape(const wg_engine* e, int which, int cluster, int threads, int cpt,
 bool pick_shapes(wg_engine* e) {
   // Preference order; the first compiled shape that fits the grid is the default (the autotuner
   // can choose another among wg_shape_candidates).
-  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 896, 4}, {4, 448, 8},
-                                 {4, 448, 10}, {1, 1024, 12},
-                                 {2, 1024, 6}, {2, 512, 12}, {2, 1024, 10}, {4, 1024, 8}, {2, 1024, 16},
-                                 {4, 512, 16}};
-  static const int apref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8}, {4, 480, 14}, {6, 384, 20}, {4, 448, 10}, {2, 1024, 6}, {4, 896, 4}, {4, 448, 8},
+  static const int fpref[][3] = {{2, 704, 10}, {4, 672, 10}, {6, 640, 12}, {2, 896, 8},  {4, 864, 8},  {6, 768, 10}, {4, 480, 14},
+                                 {6, 384, 20}, {4, 896, 4},  {4, 448, 8},  {4, 768, 6},  {1, 1024, 12}, {2, 1024, 6},
+                                 {2, 512, 12}, {2, 1024, 10}, {4, 1024, 8}, {2, 1024, 16}, {4, 512, 16}};
+  // The adjoint holds more per row and waits more: it takes the shapes of more warps (64 models of 70 x 70:
+  // 4.66 ms per 200 steps against 4.80 with {2, 704, 10}; 100 x 100: 5.76 against 6.01 with {4, 672, 10};
+  // 140 x 140: 5.80 against 6.91 with {6, 640, 12}).
+  static const int apref[][3] = {{2, 896, 8},  {2, 704, 10}, {4, 864, 8},  {4, 672, 10}, {6, 768, 10}, {6, 640, 12},
+                                 {4, 480, 14}, {6, 384, 20}, {4, 768, 6},  {2, 1024, 6}, {4, 896, 4},  {4, 448, 8},
                                  {2, 512, 12}, {4, 1024, 4}, {4, 1024, 8}, {4, 512, 16}};
   e->fshape = wg::Shape{0, 0, 0};
   e->ashape = wg::Shape{0, 0, 0};
@@ -359,10 +362,11 @@ bool pick_shapes(wg_engine* e) {
   static const struct {
     int nxc, rag, cluster, threads, cpt;
     float fwd, adj;
-  } costs[] = {{114, 0, 2, 704, 10, 2.69f, 4.67f}, {114, 0, 3, 832, 6, 2.16f, 4.00f}, {114, 0, 3, 640, 8, 2.22f, 3.79f},
-               {114, 0, 4, 448, 8, 1.85f, 3.37f},  {114, 0, 4, 896, 4, 1.86f, 3.25f}, {144, 0, 4, 672, 10, 2.68f, 4.95f},
-               {144, 0, 3, 768, 12, 3.42f, 0.0f},  {116, 1, 4, 448, 10, 2.40f, 5.19f}, {116, 1, 3, 768, 8, 2.74f, 5.07f},
-               {144, 1, 4, 672, 10, 3.02f, 5.32f}, {144, 1, 3, 768, 10, 3.30f, 5.64f}, {144, 1, 3, 768, 12, 4.06f, 7.33f}};
+  } costs[] = {{114, 0, 2, 704, 10, 2.60f, 0.0f},  {114, 0, 2, 896, 8, 0.0f, 4.53f},  {114, 0, 3, 832, 6, 2.16f, 4.00f},
+               {114, 0, 3, 640, 8, 2.14f, 3.69f},  {114, 0, 4, 448, 8, 1.85f, 3.37f}, {114, 0, 4, 896, 4, 1.86f, 3.25f},
+               {144, 0, 4, 672, 10, 2.68f, 0.0f},  {144, 0, 4, 864, 8, 0.0f, 4.59f},  {144, 0, 3, 768, 12, 3.42f, 0.0f},
+               {116, 1, 4, 768, 6, 2.22f, 3.78f},  {116, 1, 3, 768, 8, 2.74f, 5.07f}, {144, 1, 4, 864, 8, 2.81f, 4.60f},
+               {144, 1, 3, 768, 10, 3.30f, 5.64f}, {144, 1, 3, 768, 12, 4.06f, 7.33f}};
   for (int which = 0; which < 2; ++which) {
     const int n = which == 0 ? wg::fwd_shape_count() : wg::adj_shape_count();
     for (int i = 0; i < n; ++i) {

@@ -10,6 +10,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "wave_warp_map.h"
+
 namespace wg {
 
 constexpr int FD_PAD = 2;
@@ -74,6 +76,7 @@ __host__ __device__ inline size_t adjstate_floats(int nx, int nz, int swa) {
 struct FwdArgs {
   Grid g;
   Stations st;
+  WarpMap warps;
   const float* vel;      // [models][nz][nx] clamped, edge-replicated velocity (m/s)
   int units;             // models * shots
   int t0, t1;            // steps [t0, t1)
@@ -91,6 +94,7 @@ struct FwdArgs {
 struct AdjArgs {
   Grid g;
   Stations st;
+  WarpMap warps;
   const float* vel;
   int units;
   int t_hi, t_lo;        // process t = t_hi - 1 down to t_lo

@@ -86,15 +86,24 @@ struct PairIo {
   }
 };
 
-// Role of warp `warp` within its segment (0: the PML warp). Warp w issues from scheduler w % 4; with
-// 2 or 4 warps per segment a fixed role per position would put every PML warp (the heavier work) on
-// the same schedulers, so the roles rotate from segment to segment.
-template <int NI>
-__device__ __forceinline__ int warp_role(int warp) {
+// Shapes whose warps take the host's assignment (map_warps). Measured (us; 64 models of 70 x 70, or 4 in
+// clusters of three; 200 steps forward / adjoint), fixed roles -> map: {C 2, S 5} 4139 -> 4012 / 4800 ->
+// 4880 (the adjoint takes {2, 4}), {2, 4} 4680 -> 4590 / 5240 -> 4660, {3, 4} 716 -> 692 / 771 -> 750.
+// Elsewhere the map's registers or its order cost more than the balance gives: {3, 3} 696 -> 717, {4, 4}
+// 590 -> 607, and with several interior warps per segment the adjoint spills (6.0 -> 6.6 ms on 100 x 100).
+template <int C, int S, int NI>
+constexpr bool kMapped = NI == 1 && (C == 2 || (C == 3 && S == 4));
+
+// Part of warp `warp`: segment * (1 + NI) + role (0: the PML warp). Without a map the warps follow the
+// segments; with 2 or 4 warps per segment a fixed role per position would put every PML warp on the
+// same schedulers (warp w issues from scheduler w % 4), so there the roles rotate.
+template <int C, int S, int NI>
+__device__ __forceinline__ int warp_part(const WarpMap& m, int rank, int warp) {
+  if constexpr (kMapped<C, S, NI>) return m.id[rank][warp];
   constexpr int W = 1 + NI;
-  const int seg = warp / W, j = warp % W;
-  if constexpr (4 % W == 0) return (j + (seg * W) / 4) % W;
-  return j;
+  if constexpr (4 % W != 0) return warp;
+  const int seg = warp / W;
+  return seg * W + (warp % W + (seg * W) / 4) % W;
 }
 
 // Wavelet ring in shared memory: the sample of step u (counted from the launch's first step, in
@@ -265,8 +274,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   const FastCoef fc = FastCoef::make(rh);
   const Pk pk{make_float2(g.nz2[0], g.nz2[1])};
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int seg = warp / (1 + NI), wk = warp_role<NI>(warp);
   const int rank = (C > 1) ? static_cast<int>(cluster_rank()) : 0;
+  const int part = warp_part<C, S, NI>(p.warps, rank, warp), seg = part / (1 + NI), wk = part % (1 + NI);
   const int unit = blockIdx.x / C;
   const int shot = unit % p.st.shots;
   const int model = unit / p.st.shots;
@@ -307,7 +316,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) fwd3_kernel(const __g
   const bool pml = (wk == 0);
   const int x = cl.x_of(wk, lane);
   const int zb = r0 + seg * S;
-  const int ltid = light_tid<NSEG, NI, C>(tid, rank);
+  const int ltid = light_tid<NSEG, NI, C>(32 * part + lane, rank);
   const int nrows = cl.active(wk, lane) ? (FULL ? S : max(0, min(S, r1 - zb))) : 0;
   const PairIo<RAG> io{(nx & 1) == 0, cl.half(x)};
   // warps with rows that read a halo (and are sent to the neighbour)
@@ -675,8 +684,8 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   const int swa = g.swa, region = g.region_adj, nrec = p.st.nrec, nt = g.nt;
   const float rh = g.rh, dt2 = g.dt2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int seg = warp / (1 + NI), wk = warp_role<NI>(warp);
   const int rank = (C > 1) ? static_cast<int>(cluster_rank()) : 0;
+  const int part = warp_part<C, S, NI>(p.warps, rank, warp), seg = part / (1 + NI), wk = part % (1 + NI);
   const int unit = blockIdx.x / C;
   const int shot = unit % p.st.shots;
   const int model = unit / p.st.shots;
@@ -758,7 +767,7 @@ __global__ void __launch_bounds__(NSEG * 32 * (1 + NI), 1) adj3_kernel(const __g
   const int E0 = p.st.csr[r0 * nx];
   const int ecnt = p.st.csr[r1 * nx] - E0;
   const bool stage = ecnt <= L.pcap && ecnt <= NT;
-  const int ltid = light_tid<NSEG, NI, C>(tid, rank);
+  const int ltid = light_tid<NSEG, NI, C>(32 * part + lane, rank);
   const float* resu = p.residual + static_cast<size_t>(unit) * nt * nrec;
   float rnext = 0.0f;
   if (stage && ltid < ecnt) {

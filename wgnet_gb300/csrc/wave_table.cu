@@ -31,9 +31,11 @@ namespace wg {
   X(114, 12, 3, 3, 13, 1)       \
   X(114, 12, 3, 4, 10, 1)       \
   X(144, 12, 4, 5, 7, 2)        \
+  X(144, 12, 4, 4, 9, 2)        \
   X(144, 12, 4, 7, 5, 2)        \
   X(144, 12, 3, 6, 8, 2)        \
   X(184, 12, 6, 6, 5, 3)        \
+  X(184, 12, 6, 5, 6, 3)        \
   X(184, 12, 6, 10, 3, 3)
 
 // generation-3 shapes that also have a fast-arithmetic forward (one instantiation file each): the
@@ -46,12 +48,12 @@ namespace wg {
 // generation-3 shapes for any width up to NX (one instantiation file each), for the grids whose width
 // none of the above was compiled for
 #define WG_G3_RAGGED_SHAPES(X)  \
-  X(116, 12, 4, 5, 7, 1)        \
+  X(116, 12, 4, 3, 12, 1)       \
   X(116, 12, 3, 4, 12, 1)       \
-  X(144, 12, 4, 5, 7, 2)        \
+  X(144, 12, 4, 4, 9, 2)        \
   X(144, 12, 3, 5, 8, 2)        \
   X(144, 12, 3, 6, 8, 2)        \
-  X(184, 12, 6, 6, 5, 3)
+  X(184, 12, 6, 5, 6, 3)
 
 #define WG_ADJ_SHAPES(X) \
   X(2, 1024, 6)          \
@@ -194,7 +196,19 @@ int resident_clusters(int cluster) {
   return known[dev][cluster] = n;
 }
 
-cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a, cudaStream_t stream) {
+// Costs for map_warps. Of those tried (strip and PML rows at 1.2 to 4 times an interior row) the kernels'
+// own instruction counts balance the adjoint worse than nearly even ones: its warps mostly wait.
+static constexpr WarpCosts kFwdCosts{10, 5, 5, 0}, kAdjCosts{10, 2, 2, 0};
+
+static WarpMap warps_of(const Shape& s, int nz, int region, const WarpCosts& c) {
+  int bounds[9];
+  for (int r = 0; r <= s.cluster; ++r) bounds[r] = split_row(nz, s.cluster, r);
+  return map_warps(bounds, s.cluster, s.seg_rows, s.nseg, s.ni, nz, region, c);
+}
+
+cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& args, cudaStream_t stream) {
+  FwdArgs a = args;
+  if (s.kind == 3 && s.ni == 1) a.warps = warps_of(s, a.g.nz, a.g.region, kFwdCosts);
   const size_t smem = fwd_smem_bytes(s, a.g.nx, a.g.nz, a.g.sw, a.st.nrec);
   if (s.kind == 3 && s.rag) {
 #define WG_FWD3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
@@ -226,7 +240,9 @@ cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_adj(const Shape& s, const AdjArgs& a, cudaStream_t stream) {
+cudaError_t launch_adj(const Shape& s, const AdjArgs& args, cudaStream_t stream) {
+  AdjArgs a = args;
+  if (s.kind == 3 && s.ni == 1) a.warps = warps_of(s, a.g.nz, a.g.region_adj, kAdjCosts);
   const size_t smem = adj_smem_bytes(s, a.g.nx, a.g.nz, a.g.swa, a.st.nrec);
   if (s.kind == 3 && s.rag) {
 #define WG_ADJ3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
