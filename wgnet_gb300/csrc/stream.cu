@@ -6,7 +6,7 @@
 // CTAs share halos in L2) with a two-stage TMA pipeline: while it updates one tile, the next tile's
 // wavefield with its halo (72 x 36 floats; the x halo is rounded to 16 bytes) is already being
 // copied into shared memory by cp.async.bulk.tensor, completion signalled on an mbarrier. Each
-// thread owns a column pair over 4 rows; the vertical neighbours come from its column in shared
+// thread owns a column pair over 2 (forward) or 4 rows; the vertical neighbours come from its column in shared
 // memory, the horizontal ones from float2 loads beside it. Tiles that touch the C-PML read and
 // write the packed PML strips (global memory, L1/L2 resident); interior tiles skip them entirely.
 //
@@ -35,8 +35,8 @@ constexpr int TX_ = 64, TZ_ = 32;           // tile of cells per CTA iteration
 constexpr int HX = 4, HZ = 2;               // halo loaded on each side (x rounded to 16 bytes)
 constexpr int BX = TX_ + 2 * HX;            // 72 columns in shared memory
 constexpr int BZ = TZ_ + 2 * HZ;            // 36 rows
-constexpr int NTH = 256;                    // 32 column pairs x 8 groups of 4 rows
-constexpr int RPT = 4;                      // rows per thread
+constexpr int NTH = 256;                    // adjoint: 32 column pairs x 8 groups of 4 rows
+constexpr int RPT = 4;                      // its rows per thread
 constexpr unsigned kTileBytes = BX * BZ * 4;
 constexpr long kWaitLimit = 1L << 22;       // mbarrier polls before giving up
 
@@ -126,11 +126,12 @@ struct FwdMaps {
   CUtensorMap p;  // wavefield without halo (the previous step): 64 x 32 boxes
   CUtensorMap v;  // velocity: 64 x 32 boxes over [models][nz][nx]
 };
-constexpr int FST = 3;                                        // forward pipeline stages
+constexpr int FST = 2;                                        // forward pipeline stages
 constexpr int FSTAGE_F = BZ * BX + 2 * TZ_ * TX_;             // floats per stage: U | P | V
 constexpr size_t kFwdSmem = FST * FSTAGE_F * 4 + 128 + 16 * FST;
 
-constexpr int FWD_THREADS = NTH + 32;  // 8 consumer warps + 1 producer warp
+constexpr int FNTH = 512, FRPT = 2;    // forward: consumer threads, rows per thread
+constexpr int FWD_THREADS = FNTH + 32;  // consumer warps + 1 producer warp
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -194,6 +195,7 @@ __device__ __forceinline__ void prefetch_map(const CUtensorMap* m) {
 }
 
 // Bit 2 r + j: cell (zr + r, x + j) is a corner of the source.
+template <int RPT>
 __device__ __forceinline__ unsigned source_bits(const SArgs& a, int shot, int zr, int x) {
   unsigned m = 0;
 #pragma unroll
@@ -217,15 +219,18 @@ __device__ __forceinline__ void issue_fwd(const SArgs& a, const FwdMaps& m, floa
   tma_load(st + BZ * BX + TZ_ * TX_, &m.v, j.x0, j.z0, j.model, bar);
 }
 
-// Warp-specialised: warp 8 (one lane) streams the jobs' tiles into FST stages (waiting on each
-// stage's "empty" barrier before refilling it), warps 0-7 update the tiles and release each stage
+// Warp-specialised: the last warp (one lane) streams the jobs' tiles into FST stages (waiting on each
+// stage's "empty" barrier before refilling it), the others update the tiles and release each stage
 // with one arrival per warp. No CTA-wide barrier per tile: consumer warps run up to FST tiles
 // apart. Every wait is bounded; a consumer that gives up records the error and leaves; the
 // producer that gives up records it and waits (bounded) for the copies it issued.
-// Decoding a job once per CTA, packed arithmetic (wave_packed.cuh) and the overlapped launch took a step of
-// 16 shots of the 844 x 344 grid from 38.5 to 31.5 us (storing terms) and from 36.2 to 30.9 (not). What
-// is left is latency: the C-PML tiles (43 % of them) wait on their strips' values in L2. Loading them
-// for all four rows ahead spills at 96 registers and measured slower (44 us).
+// Latency bounds it: the C-PML tiles (43 % of those of the 844 x 344 grid) wait on their strips' values in
+// L2. Decoding a job once per CTA, packed arithmetic (wave_packed.cuh) and the overlapped launch took a step
+// of 16 shots of that grid from 38.5 to 31.5 us (storing terms) and from 36.2 to 30.9 (not); 16 warps of
+// two rows a thread instead of 8 of four, with two stages, to 27.9 and 25.8, for all that they spill a
+// little at 56 registers (three stages: 28.6 and 26.0; three CTAs of 8 warps: 29.0 and 26.8; four: 40.4
+// and 37.4). Loading the strips ahead for four rows spilled and measured slower (44 us). The adjoint holds
+// more and stays at 8 warps of four rows (16 of two: 55.8 against 51.3 us).
 template <bool TRACES, bool STORE>
 __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid_constant__ FwdMaps maps,
                                                                     const __grid_constant__ SArgs a) {
@@ -243,11 +248,11 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
   if (tid == 0) {
     for (int k = 0; k < FST; ++k) {
       mbar_init(&full[k], 1);
-      mbar_init(&empty[k], NTH / 32);
+      mbar_init(&empty[k], FNTH / 32);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (tid == NTH) {
+  if (tid == FNTH) {
     prefetch_map(&maps.u);
     prefetch_map(&maps.p);
     prefetch_map(&maps.v);
@@ -255,8 +260,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
   __syncthreads();
   wait_for_previous_step();
   let_next_step_launch();
-  if (tid >= NTH) {  // producer warp
-    if (tid == NTH) {
+  if (tid >= FNTH) {  // producer warp
+    if (tid == FNTH) {
       int issued = 0;
       JobWalk walk(a);
       for (int job = blockIdx.x; job < jobs; job += gridDim.x, ++issued, walk.advance(a)) {
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
   const int pc = tid & 31, grp = tid >> 5;
   const size_t xs_unit = static_cast<size_t>(nz) * 2 * ssw;  // floats per unit of an x strip array
   const size_t zs_unit = static_cast<size_t>(2) * ssw * nx;
-  const int sx = 2 * pc + HX, sz = RPT * grp + HZ;
+  const int sx = 2 * pc + HX, sz = FRPT * grp + HZ;
   int job = blockIdx.x;
   for (int i = 0; job < jobs; ++i, job += gridDim.x) {
     const int s = i % FST;
@@ -289,20 +294,20 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
     }
     const Job j = info[s];
     const int x = j.x0 + 2 * pc;
-    const int zr = j.z0 + RPT * grp;
+    const int zr = j.z0 + FRPT * grp;
     float* Wn = a.W + (static_cast<size_t>(1 - par) * a.units + j.unit) * cells;
     const float* T = stage + s * FSTAGE_F;
-    const float* Pt = T + BZ * BX + RPT * grp * TX_ + 2 * pc;
+    const float* Pt = T + BZ * BX + FRPT * grp * TX_ + 2 * pc;
     const float* Vt = Pt + TZ_ * TX_;
     float* stp = STORE ? a.stored + (static_cast<size_t>(j.unit) * a.seg + (a.t - a.seg_t0)) * cells : nullptr;
-    float2 col[RPT + 4];
+    float2 col[FRPT + 4];
 #pragma unroll
-    for (int k = 0; k < RPT + 4; ++k) col[k] = lds2(T + (sz - 2 + k) * BX + sx);
+    for (int k = 0; k < FRPT + 4; ++k) col[k] = lds2(T + (sz - 2 + k) * BX + sx);
 
     if (j.inner) {
       // interior tile: no frame, PML, receivers or sources
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) {
+      for (int r = 0; r < FRPT; ++r) {
         const int cell = (zr + r) * nx + x;
         const float2 A = lds2(T + (sz + r) * BX + sx - 2), B = lds2(T + (sz + r) * BX + sx + 2), u = col[r + 2];
         const float2 w = add2(pk.second(u, side_sum(A, u, B), add2(B, A), a.d2a, a.d2b),
@@ -319,7 +324,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
 
     if (TRACES) {
       const int r0 = a.tile_rec_start[j.tile], r1 = a.tile_rec_start[j.tile + 1];
-      for (int k = r0 + tid; k < r1; k += NTH) {
+      for (int k = r0 + tid; k < r1; k += FNTH) {
         const int r = a.tile_rec[k];
         float acc = 0.0f;
 #pragma unroll
@@ -334,7 +339,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
 
     const bool xok = x >= FD_PAD && x + 1 < nx - FD_PAD;
     const bool xpml = x < region || x + 1 >= nx - region;
-    const unsigned srcm = j.src ? source_bits(a, j.shot, zr, x) : 0u;
+    const unsigned srcm = j.src ? source_bits<FRPT>(a, j.shot, zr, x) : 0u;
     float2 ax = make_float2(0.f, 0.f), bx = ax, dbx = ax;
     if (xok && xpml) {
       ax = ldg2(a.prof + x);
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid
     auto rows = [&](float* __restrict__ wn, float* __restrict__ pxn, float* __restrict__ zxo, float* __restrict__ pzn,
                     float* __restrict__ zzo, float* __restrict__ sto) {
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) {
+      for (int r = 0; r < FRPT; ++r) {
         const int z = zr + r;
         if (!xok || z < FD_PAD || z >= nz - FD_PAD) continue;
         const int cell = z * nx + x;
@@ -910,7 +915,7 @@ __global__ void __launch_bounds__(NTH, 2) adj_stream_kernel(const __grid_constan
     const int* sc = a.st.src_cell + 4 * shot;
     const float* res_t = a.residual + (static_cast<size_t>(unit) * a.nt + a.t) * a.st.nrec;
     const bool rec_rows = zr + RPT > a.rec_z0 && zr <= a.rec_z1;
-    const unsigned srcm = j.src ? source_bits(a, shot, zr, x) : 0u;
+    const unsigned srcm = j.src ? source_bits<RPT>(a, shot, zr, x) : 0u;
     float* LPXn = a.PX + (static_cast<size_t>(1 - q) * a.units + unit) * xs_unit;
     float* LZXn = a.ZX + (static_cast<size_t>(1 - q) * a.units + unit) * xs_unit;
     float* LPZn = a.PZ + (static_cast<size_t>(1 - q) * a.units + unit) * zs_unit;
@@ -1303,7 +1308,7 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
 // the engine option says, or, where it was not set, when its tiles fit the chip in three waves: a step is then
 // mostly the latency of its launch and copies, which four steps share.
 // us per step (recording traces), blocked against one step per launch: 50 tiles (2 shots of 284 x 154
-// cells) 3.4 / 7.3, 150 tiles 3.4 / 7.5, 210 tiles 6.1 / 7.7, 420 tiles 8.1 / 10.4, 560 tiles 9.9 / 9.3.
+// cells) 3.4 / 5.8, 150 tiles 3.4 / 6.0, 252 tiles 6.1 / 6.7, 420 tiles 8.1 / 9.0, 546 tiles 10.7 / 9.4.
 constexpr int kTbWaves = 3;
 bool blocked(const StreamWork* w, const EngineView& v, int units) {
   if (v.tblock >= 0) return v.tblock != 0;
