@@ -1256,17 +1256,24 @@ int adj_step(StreamWork* w, const CUtensorMap& map, SArgs a, int t, cudaStream_t
   return WG_OK;
 }
 
+// The blocked kernels' two state sets.
+cudaError_t tb_state(StreamWork* w, const EngineView& v, int units) {
+  const size_t nW = static_cast<size_t>(units) * v.nx * v.nz, nX = units * xs_floats(v), nZ = units * zs_floats(v);
+  cudaError_t e = w->Wtb.ensure(4 * nW * 4);
+  if (e == cudaSuccess) e = w->PXtb.ensure(2 * nX * 4);
+  if (e == cudaSuccess) e = w->ZXtb.ensure(2 * nX * 4);
+  if (e == cudaSuccess) e = w->PZtb.ensure(2 * nZ * 4);
+  if (e == cudaSuccess) e = w->ZZtb.ensure(2 * nZ * 4);
+  return e;
+}
+
 // Temporally blocked forward over all units from the zero state, TB_T steps per launch: receivers
 // into `traces` and, when `stored` is given, every step's gradient term (the store-all scheme).
 int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float* traces, float* stored,
                cudaStream_t st) {
   const size_t cells = static_cast<size_t>(v.nx) * v.nz;
   const size_t nW = static_cast<size_t>(units) * cells, nX = units * xs_floats(v), nZ = units * zs_floats(v);
-  SW_CK(w->Wtb.ensure(4 * nW * 4));
-  SW_CK(w->PXtb.ensure(2 * nX * 4));
-  SW_CK(w->ZXtb.ensure(2 * nX * 4));
-  SW_CK(w->PZtb.ensure(2 * nZ * 4));
-  SW_CK(w->ZZtb.ensure(2 * nZ * 4));
+  SW_CK(tb_state(w, v, units));
   SW_CK(cudaMemsetAsync(w->Wtb.p, 0, 4 * nW * 4, st));
   SW_CK(cudaMemsetAsync(w->PXtb.p, 0, 2 * nX * 4, st));
   SW_CK(cudaMemsetAsync(w->ZXtb.p, 0, 2 * nX * 4, st));
@@ -1303,19 +1310,20 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
   return WG_OK;
 }
 
-// Checkpoint slot layout: [W(t) | W(t-1) | PX(t) | ZX | PZ(t) | ZZ] for all units.
 // Whether a pass that starts from the zero state and writes no checkpoints runs temporally blocked: as
-// the engine option says, or, where it was not set, when its tiles fit the chip in three waves: a step is then
+// the engine option says, or, where it was not set, when its tiles fit the chip in three waves (and there is
+// memory for the second state set): a step is then
 // mostly the latency of its launch and copies, which four steps share.
 // us per step (recording traces), blocked against one step per launch: 50 tiles (2 shots of 284 x 154
 // cells) 3.4 / 5.8, 150 tiles 3.4 / 6.0, 252 tiles 6.1 / 6.7, 420 tiles 8.1 / 9.0, 546 tiles 10.7 / 9.4.
 constexpr int kTbWaves = 3;
-bool blocked(const StreamWork* w, const EngineView& v, int units) {
+bool blocked(StreamWork* w, const EngineView& v, int units) {
   if (v.tblock >= 0) return v.tblock != 0;
   const long jobs = static_cast<long>(units) * ((v.nx + TX_ - 1) / TX_) * ((v.nz + TZ_ - 1) / TZ_);
-  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks;
+  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks && tb_state(w, v, units) == cudaSuccess;
 }
 
+// Checkpoint slot layout: [W(t) | W(t-1) | PX(t) | ZX | PZ(t) | ZZ] for all units.
 size_t ckpt_slot_floats(const EngineView& v, int units) {
   const size_t cells = static_cast<size_t>(v.nx) * v.nz;
   return static_cast<size_t>(units) * (2 * cells + 2 * xs_floats(v) + 2 * zs_floats(v));
@@ -1449,6 +1457,14 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   SW_CK(w->stored.ensure(static_cast<size_t>(seg) * step_bytes));
   if (J > 1) SW_CK(w->ckpt.ensure(static_cast<size_t>(J - 1) * slot_bytes));
 
+  // adjoint state (before the blocked forward's, which the pass can do without)
+  const size_t xsf = xs_floats(v), zsf = zs_floats(v);
+  SW_CK(w->L.ensure(2 * units * cells * 4));
+  SW_CK(w->LPX.ensure(2 * units * xsf * 4));
+  SW_CK(w->LZX.ensure(2 * units * xsf * 4));
+  SW_CK(w->LPZ.ensure(2 * units * zsf * 4));
+  SW_CK(w->LZZ.ensure(2 * units * zsf * 4));
+
   FwdMaps fmap;
   if ((rc = make_fwd_maps(&fmap, w->W.f(), w->vpad.f(), v.nx, v.nz, units, models)) != WG_OK) return rc;
   SArgs f = base_args(w, v, units);
@@ -1478,13 +1494,6 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   SW_CK(launch_residual(w->traces.f(), d_obs, w->scale.f(), models, v.shots * tr, w->traces.f(), d_loss,
                         static_cast<double*>(w->part.p), st));
 
-  // adjoint state
-  const size_t xsf = xs_floats(v), zsf = zs_floats(v);
-  SW_CK(w->L.ensure(2 * units * cells * 4));
-  SW_CK(w->LPX.ensure(2 * units * xsf * 4));
-  SW_CK(w->LZX.ensure(2 * units * xsf * 4));
-  SW_CK(w->LPZ.ensure(2 * units * zsf * 4));
-  SW_CK(w->LZZ.ensure(2 * units * zsf * 4));
   SW_CK(cudaMemsetAsync(w->L.p, 0, 2 * units * cells * 4, st));
   SW_CK(cudaMemsetAsync(w->LPX.p, 0, 2 * units * xsf * 4, st));
   SW_CK(cudaMemsetAsync(w->LZX.p, 0, 2 * units * xsf * 4, st));
