@@ -45,14 +45,14 @@ UPDATED_CELLS = (NX + 2 * (PML + 2) - 4) ** 2  # 110 x 110 cells updated per ste
 FLOPS_PER_CELL_UPDATE = 48.0  # average over interior / one-PML-axis / two-PML-axes cells at pml 20
 # DRAM bytes per (unit, step) measured with ncu on the small case (32 models, nt 200: the full
 # 256-model launch is too large for a multi-pass capture), scaled by unit-steps to a full launch
-MEASURED_TRAFFIC_PER_UNIT_STEP = {"adjoint": (813.12e6 + 9.30e6) / 16000, "recompute": (69.86e6 + 735.81e6) / 16000}
+MEASURED_TRAFFIC_PER_UNIT_STEP = {"adjoint": (813.03e6 + 9.68e6) / 16000, "recompute": (70.67e6 + 737.11e6) / 16000}
 # Counters of the same small-case captures (ncu --set full), per kernel: thread-instructions per
 # updated cell and step, issue slots busy, L1/shared throughput, shared-memory bank-conflict share.
 NCU_SMALL_CASE = {
-    "adjoint": {"thread_instructions_per_cell_update": 106.7, "issue_active_pct": 62.7, "l1_shared_pct": 68.0,
-                "bank_conflict_pct_of_shared_wavefronts": 1.7, "warps_active_pct": 34.3},
-    "recompute": {"thread_instructions_per_cell_update": 71.7, "issue_active_pct": 64.9, "l1_shared_pct": 52.0,
-                  "bank_conflict_pct_of_shared_wavefronts": 2.5, "warps_active_pct": 34.3},
+    "adjoint": {"thread_instructions_per_cell_update": 108.2, "issue_active_pct": 65.9, "l1_shared_pct": 71.3,
+                "bank_conflict_pct_of_shared_wavefronts": 1.6, "warps_active_pct": 43.7},
+    "recompute": {"thread_instructions_per_cell_update": 56.3, "issue_active_pct": 59.5, "l1_shared_pct": 62.0,
+                  "bank_conflict_pct_of_shared_wavefronts": 3.4, "warps_active_pct": 34.3},
 }
 
 
@@ -509,7 +509,7 @@ def large_config(nt: int, shots: int) -> dict:
     return {"workload": f"large survey: 800x300 cells at 5 m (padded 844x344), {shots} shots, 800 receivers, "
                         f"dt=0.5ms, nt={nt}, forward + exact adjoint gradient, streamed path",
             "checkpointing": "every step's gradient term stored in HBM when it fits (auto)",
-            "temporal_block": "off (one step per launch); `simulate` also times the engine option",
+            "temporal_block": "one step per launch; `simulate` also times the engine option",
             "l2": "inputs larger than L2 (wavefields ~93 MB + stored terms ~186 GB per gradient)"}
 
 

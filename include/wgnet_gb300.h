@@ -98,7 +98,9 @@ int wg_selftest_wait_timeout(wg_engine* eng, long long polls, void* stream);
  * in reverse. k >= nt stores the gradient term of every step (the reference's scheme,
  * wave_wgpu.rs:181-182); so does k <= 0 on the resident path, while on the streamed path k <= 0
  * (its default) stores every step when that fits in 70% of the free device memory and otherwise
- * picks the interval that fits. No reference counterpart for k > 0. */
+ * picks the interval that fits. An engine whose interval was never set (the getter then says 50) stores
+ * every step of a batch whose terms take at most 4 GiB and an eighth of the free memory, and
+ * checkpoints larger ones; the gradient is the same bit for bit. No reference counterpart for k > 0. */
 int wg_set_checkpoint_interval(wg_engine* eng, int k);
 int wg_get_checkpoint_interval(const wg_engine* eng);
 
@@ -111,17 +113,20 @@ int wg_get_checkpoint_interval(const wg_engine* eng);
  * kernels compute the same discrete operator with 1/h folded into the stencil weights and fused
  * multiply-adds, faster and equal to f32 accuracy, on the resident kernels of the default 70x70,
  * 100x100 and 140x140 shapes; the adjoint, other shapes and the streamed path keep the unfused
- * arithmetic), "temporal_block" (0/1, default 0; 1: on the streamed path, forward passes that
+ * arithmetic), "temporal_block" (0/1: on the streamed path, forward passes that
  * start from the zero state and need no checkpoints (simulate, and the gradient's forward when
  * every step's gradient term is kept) advance each tile 4 steps per launch from a halo of 8 cells
- * held in shared memory, with identical results; slower than the per-step kernels on the 800x300
- * survey, whose per-step forward is not bandwidth-bound). No reference counterpart. */
+ * held in shared memory, with identical results; while it was never set (the getter then says 0) they do
+ * so for surveys of at most three tiles per SM, where a step is mostly launch latency, and take one
+ * step per launch for larger ones, whose forward is not bandwidth-bound). No reference counterpart. */
 int wg_set_option(wg_engine* eng, const char* key, int value);
 int wg_get_option(const wg_engine* eng, const char* key, int* value);
 
 /* Launch shape of the resident kernels (which = 0 forward, 1 adjoint): CTAs per (model, shot)
- * cluster, threads per CTA, cells-per-thread bound. wg_shape_candidates lists the compiled
- * shapes that fit this engine's grid. No reference counterpart (wgpu dispatches 16x16 tiles). */
+ * cluster, threads per CTA, cells-per-thread bound. Until a shape is set, each pass takes the one
+ * whose waves of clusters take the least time for its number of units, and wg_get_launch_shape gives
+ * that of large batches. wg_shape_candidates lists the compiled shapes that fit this engine's grid. No
+ * reference counterpart (wgpu dispatches 16x16 tiles). */
 int wg_set_launch_shape(wg_engine* eng, int which, int cluster, int threads, int cpt);
 int wg_get_launch_shape(const wg_engine* eng, int which, int* cluster, int* threads, int* cpt);
 int wg_shape_candidates(const wg_engine* eng, int which, int* out3, int max_shapes);

@@ -600,8 +600,6 @@ int simulate_dev_impl(wg_engine* e, const float* d_vis, int models, float* d_tra
   return WG_OK;
 }
 
-// obs_ready (optional): an event the observed data's arrival is recorded on; nothing reads them
-// before the first forward pass has been launched, so their host->device copy can overlap it.
 // An engine whose checkpoint interval was never set keeps every step's gradient term (no recompute:
 // the gradient is the same bit for bit) when the batch's terms are small beside the memory: at most
 // kStoreBytes and an eighth of what is free, and the allocation succeeds; the buffer then stays with
@@ -621,6 +619,8 @@ bool store_by_default(wg_engine* e, int models) {
   return need <= free_b / 8 && e->w_stored.ensure(need) == WG_OK;
 }
 
+// obs_ready (optional): an event the observed data's arrival is recorded on; nothing reads them
+// before the first forward pass has been launched, so their host->device copy can overlap it.
 int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int models, double* d_loss, float* d_grad,
                       cudaStream_t st, cudaEvent_t obs_ready = nullptr) {
   if (models < 1) return fail(WG_ERR_ARG, "models must be >= 1");
