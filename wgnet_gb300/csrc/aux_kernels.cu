@@ -184,10 +184,14 @@ __global__ void __launch_bounds__(kFoldThreads) fold_kernel(const float* __restr
 // a row: their inputs slide through registers, so a tap costs one load of x and one of ker for FIR_R
 // products and sums, which FP32 issue then bounds (products and sums are not fused: each rounds as
 // the one-sample-per-thread kernel's did, which two loads per product bounded). 16 models x 5 shots x
-// 2001 x 70 at 377 taps: 0.37 against 3.2 ms; the FP32 bound is 0.21 ms.
+// 2001 x 70 at 377 taps: 0.35 against 3.2 ms; the FP32 bound is 0.21 ms (0.38 with the end of the record
+// tested at every load and each load next to its use).
 constexpr int FIR_R = 16;
 constexpr int FIR_THREADS = 128;
 
+// CHECK: fewer than FIR_R times, so a thread's samples may lie past the last; otherwise the last block of
+// times starts at nt - FIR_R and stores only the samples that the one before it does not.
+template <bool CHECK>
 __global__ void __launch_bounds__(FIR_THREADS) bandlimit_kernel(const float* __restrict__ in, const float* __restrict__ ker,
                                                                 int klen, long traces, int nt, int nrec,
                                                                 float* __restrict__ out) {
@@ -195,9 +199,9 @@ __global__ void __launch_bounds__(FIR_THREADS) bandlimit_kernel(const float* __r
   if (c >= traces) return;
   const long base = (c / nrec) * nt * nrec + c % nrec;
   const float* x = in + base;
-  const int t0 = blockIdx.y * FIR_R;
-  auto at = [&](int t) { return t < nt ? __ldg(x + static_cast<long>(t) * nrec) : 0.0f; };  // t >= 0
-  float acc[FIR_R], win[FIR_R];
+  const int first = blockIdx.y * FIR_R, t0 = CHECK ? first : min(first, nt - FIR_R);
+  auto at = [&](int t) { return !CHECK || t < nt ? __ldg(x + static_cast<long>(t) * nrec) : 0.0f; };  // t >= 0
+  float acc[FIR_R], win[FIR_R], next[FIR_R];
   // from tap k0 on, the taps of all FIR_R samples lie at times >= 0; before it sample j still has
   // the taps of times 0 .. j - 1
   const int k0 = max(0, klen - 1 - t0);
@@ -217,11 +221,20 @@ __global__ void __launch_bounds__(FIR_THREADS) bandlimit_kernel(const float* __r
   for (int j = 0; j < FIR_R - 1; ++j) win[j] = at(ts + j);
   ts += FIR_R - 1;
   int k = k0;
+  auto ahead = [&](int t) {  // the inputs of FIR_R taps, requested one round before their use
+#pragma unroll
+    for (int q = 0; q < FIR_R; ++q) next[q] = at(t + q);
+  };
+  if (k + FIR_R <= klen) ahead(ts);
   for (; k + FIR_R <= klen; k += FIR_R, ts += FIR_R) {
     // sample j reads time ts - (FIR_R - 1) + j + q at tap k + q: slot (j + q) % FIR_R
+    float cur[FIR_R];
+#pragma unroll
+    for (int q = 0; q < FIR_R; ++q) cur[q] = next[q];
+    if (k + 2 * FIR_R <= klen) ahead(ts + FIR_R);
 #pragma unroll
     for (int q = 0; q < FIR_R; ++q) {
-      win[(q + FIR_R - 1) % FIR_R] = at(ts + q);
+      win[(q + FIR_R - 1) % FIR_R] = cur[q];
       const float w = __ldg(ker + k + q);
 #pragma unroll
       for (int j = 0; j < FIR_R; ++j) acc[j] = acc[j] + w * win[(j + q) % FIR_R];
@@ -238,7 +251,7 @@ __global__ void __launch_bounds__(FIR_THREADS) bandlimit_kernel(const float* __r
   }
 #pragma unroll
   for (int j = 0; j < FIR_R; ++j)
-    if (t0 + j < nt) out[base + static_cast<long>(t0 + j) * nrec] = acc[j];
+    if (t0 + j >= first && (!CHECK || t0 + j < nt)) out[base + static_cast<long>(t0 + j) * nrec] = acc[j];
 }
 
 // Zero-phase FIR low-pass and decimation to FP16: out[s][j][r] = sum_k ker[k] in[s][j*factor + k -
@@ -307,7 +320,10 @@ cudaError_t launch_bandlimit(const float* in, const float* ker, int klen, int se
                              cudaStream_t s) {
   const long traces = static_cast<long>(series) * nrec;
   const dim3 grid(static_cast<unsigned>((traces + FIR_THREADS - 1) / FIR_THREADS), (nt + FIR_R - 1) / FIR_R);
-  bandlimit_kernel<<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+  if (nt < FIR_R)
+    bandlimit_kernel<true><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+  else
+    bandlimit_kernel<false><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
   return cudaGetLastError();
 }
 
