@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -545,29 +546,40 @@ wg::StreamTimer timer_of(wg_engine* e) {
   return t;
 }
 
-size_t per_model_grad_bytes(const wg_engine* e, int k, bool store_all) {
-  const size_t S = e->shots, cells = e->cells;
-  size_t b = 2 * cells * 4 + S * e->nt * e->nrec * 4 + 64;
-  const int J = store_all ? 1 : (e->nt + k - 1) / k;
-  const int seg = store_all ? e->nt : k;
-  b += S * static_cast<size_t>(J - 1) * wg::ckpt_floats(e->nx, e->nz, e->sw) * 4;
-  b += S * static_cast<size_t>(seg) * cells * 4;
-  b += S * wg::adjstate_floats(e->nx, e->nz, e->swa) * 4;
-  b += S * cells * 4;
-  return b;
-}
+// A workspace of a pass and the bytes of it that one model takes.
+struct Need {
+  const DevBuf* buf;
+  size_t per_model;
+};
 
-int chunk_models(const wg_engine* e, int models, size_t per_model) {
+// Models per chunk: as many as take at most 70 % of the free memory beyond what their workspaces already
+// hold, and 96 GiB in all. (Without the credit for the workspaces held, a batch that they cover whole was cut
+// into single models once another allocation had taken the rest of the memory.)
+int chunk_models(int models, std::initializer_list<Need> needs) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
     free_b = size_t(8) << 30;
   }
-  size_t budget = std::min<size_t>(free_b / 10 * 7, size_t(96) << 30);
-  long m = static_cast<long>(budget / std::max<size_t>(per_model, 1));
-  m = std::max<long>(1, std::min<long>(m, models));
-  (void)e;
-  return static_cast<int>(m);
+  const size_t budget = free_b / 10 * 7, most = size_t(96) << 30;
+  auto fits = [&](size_t m) {
+    size_t grow = 0, all = 0;
+    for (const Need& n : needs) {
+      const size_t bytes = m * n.per_model;
+      grow += bytes > n.buf->bytes ? bytes - n.buf->bytes : 0;
+      all += bytes;
+    }
+    return all <= most && grow <= budget;
+  };
+  int lo = 1, hi = models;  // one model at least, whatever it takes
+  while (lo < hi) {
+    const int m = lo + (hi - lo + 1) / 2;
+    if (fits(m))
+      lo = m;
+    else
+      hi = m - 1;
+  }
+  return lo;
 }
 
 int simulate_dev_impl(wg_engine* e, const float* d_vis, int models, float* d_traces, cudaStream_t st) {
@@ -578,7 +590,7 @@ int simulate_dev_impl(wg_engine* e, const float* d_vis, int models, float* d_tra
     return wg::stream_simulate(e->swork, view_of(e), e->rec_cell.data(), d_vis, models, d_traces, st, timer_of(e));
   }
   const size_t cells = e->cells;
-  const int M = chunk_models(e, models, cells * 4 + 64);
+  const int M = chunk_models(models, {{&e->w_vpad, cells * 4}});
   WG_TRY(e->w_vpad.ensure(static_cast<size_t>(M) * cells * 4));
   for (int m0 = 0; m0 < models; m0 += M) {
     const int mc = std::min(M, models - m0);
@@ -639,7 +651,15 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
   const size_t S = e->shots, cells = e->cells, tr = static_cast<size_t>(e->nt) * e->nrec;
   const size_t ckf = wg::ckpt_floats(e->nx, e->nz, e->sw);
   const size_t asf = wg::adjstate_floats(e->nx, e->nz, e->swa);
-  const int M = chunk_models(e, models, per_model_grad_bytes(e, k, store_all));
+  const int M = chunk_models(models, {{&e->w_vpad, cells * 4},
+                                      {&e->w_mask, cells * 4},
+                                      {&e->w_traces, S * tr * 4},
+                                      {&e->w_energy, 8},
+                                      {&e->w_scale, 4},
+                                      {&e->w_ckpt, S * slots * ckf * 4},
+                                      {&e->w_stored, S * seg * cells * 4},
+                                      {&e->w_adj, S * asf * 4},
+                                      {&e->w_gacc, S * cells * 4}});
   WG_TRY(e->w_vpad.ensure(M * cells * 4));
   WG_TRY(e->w_mask.ensure(M * cells * 4));
   WG_TRY(e->w_traces.ensure(M * S * tr * 4));
