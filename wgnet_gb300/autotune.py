@@ -3,16 +3,19 @@
 For one engine (one grid and survey) it times every compiled CTA/cluster shape that fits the grid
 (`WaveEngine.shape_candidates`) on a seeded synthetic batch, with CUDA events around each kernel
 launch (`WaveEngine.profile`), and keeps the fastest. Results are cached in a JSON file keyed by
-the GPU (name, SM count), the kernel (forward or adjoint) and the survey dimensions, so a shape is
-measured once per machine type. The reference has no counterpart: its wgpu dispatches use a fixed
+the GPU (name, SM count), the kernel (forward or adjoint), the survey dimensions, the shapes there were to
+choose from and the kernels' sources, so a shape is measured once per machine type and build. The engine
+keeps a tuned shape for every batch size; one that was not tuned chooses by the number of units. The reference has no counterpart: its wgpu dispatches use a fixed
 workgroup size (crates/wave-gauss-rs/src/shaders/splatForward.wgsl:48).
 """
 
 from __future__ import annotations
 
+import functools
 import json
 import os
 import threading
+import zlib
 from pathlib import Path
 
 _CACHE_ENV = "WGNET_GB300_AUTOTUNE_CACHE"
@@ -33,11 +36,23 @@ def device_tag() -> str:
     return f"{props.name}|sm{props.multi_processor_count}"
 
 
+@functools.lru_cache(maxsize=1)
+def kernels_tag() -> str:
+    """Checksum of the resident kernels' sources: a shape timed on other kernels is not the fastest of these."""
+    crc = 0
+    for f in sorted((Path(__file__).resolve().parent / "csrc").glob("wave_*")):
+        crc = zlib.crc32(f.read_bytes(), crc)
+    return f"{crc:08x}"
+
+
 def cache_key(device: str, which: str, eng) -> str:
     """The timing of a shape depends on the padded grid, the stations, the shot count and the
-    arithmetic (fast kernels exist for some shapes only); nt only scales it."""
+    arithmetic (fast kernels exist for some shapes only); nt only scales it. Which is the fastest also
+    depends on the shapes that there are and on the kernels."""
     arith = eng.get_option("arith")
-    return f"{device}|{which}|{eng.nx}x{eng.nz}|pml{eng.pml}|shots{eng.shots}|nrec{eng.nrec}|arith{arith}"
+    shapes = zlib.crc32(repr(sorted(map(tuple, eng.shape_candidates(which)))).encode())
+    return (f"{device}|{which}|{eng.nx}x{eng.nz}|pml{eng.pml}|shots{eng.shots}|nrec{eng.nrec}|arith{arith}"
+            f"|shapes{shapes:08x}|kernels{kernels_tag()}")
 
 
 def load_cache(path: Path | None = None) -> dict:
