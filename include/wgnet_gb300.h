@@ -248,9 +248,12 @@ int wg_pc_adam_layers(int layers, const float* const* d_partial, const int* spli
 int wg_pc_conv(int mode, const void* d_act_bf16, int batch, int h, int w, int dil, const void* d_wgt_bf16, int kp,
                const float* d_add, const void* d_mask_bf16, float* d_out32, void* d_out16, int* d_status,
                void* stream);
-/* Split partials [splits][576][64] of the convolution's transposed weight gradient from its input
- * activations and dL/dy [pixels][64] bf16; columns > 0: the input is a matrix [pixels][columns] and a
- * partial has `columns` rows. batch h w must be a multiple of 64. */
+/* Partials [P][576][64] of the convolution's transposed weight gradient from its input activations and
+ * dL/dy [pixels][64] bf16; columns > 0: the input is a matrix [pixels][columns] and a partial has
+ * `columns` rows. batch h w must be a multiple of 64. P is wg_pc_wgrad_partials(batch, h, w, splits), at
+ * most `splits` (each takes ceil(batch h w / 64 / splits) tiles of 64 pixels, so fewer may cover them):
+ * what to allocate, and the `splits` of wg_pc_adam and wg_pc_adam_layers. */
+int wg_pc_wgrad_partials(int batch, int h, int w, int splits); /* 0: bad argument */
 int wg_pc_conv_wgrad(const void* d_act_bf16, int columns, const void* d_dy_bf16, int batch, int h, int w, int dil,
                      int splits, float* d_partial, int* d_status, void* stream);
 /* Data gradient of a 64 -> 1 convolution: dh [pixels][64] and its bf16 copy from dL/dy [pixels] and

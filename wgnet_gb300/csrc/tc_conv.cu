@@ -655,6 +655,12 @@ int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, co
   }
 }
 
+int wg_pc_wgrad_partials(int batch, int h, int w, int splits) {
+  if (wg::bad_image(batch, h, w, 1) || splits < 1 || batch * h * w % 64) return 0;
+  const int tiles = batch * h * w / 64, per_split = (tiles + splits - 1) / splits;
+  return (tiles + per_split - 1) / per_split;
+}
+
 int wg_pc_conv_wgrad(const void* d_act, int columns, const void* d_dy, int batch, int h, int w, int dil, int splits,
                      float* d_partial, int* d_status, void* stream) {
   using namespace wg;
@@ -680,7 +686,7 @@ int wg_pc_conv_wgrad(const void* d_act, int columns, const void* d_dy, int batch
   if ((rc = map_bf16(&my, d_dy, M, 64, 64)) != WG_OK) return rc;
   if ((rc = columns ? allow_smem(wgrad_kernel<true>, kWgradSmem) : allow_smem(wgrad_kernel<false>, kWgradSmem)) != WG_OK)
     return rc;
-  const dim3 grid((g.kdim + 127) / 128, (g.k_tiles + g.per_split - 1) / g.per_split);
+  const dim3 grid((g.kdim + 127) / 128, wg_pc_wgrad_partials(batch, h, w, splits));
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   note_launch();
   if (columns)

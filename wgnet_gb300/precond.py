@@ -177,9 +177,8 @@ class UpdateNet:
         import torch
 
         B, H, W = shape
-        kt = B * H * W // 64
-        nz = -(-kt // -(-kt // splits)) if kt else 1
-        part = torch.empty((nz, L.kp, L.n), device=self.device, dtype=torch.float32)
+        nz = self._lib.wg_pc_wgrad_partials(B, H, W, splits)
+        part = torch.empty((max(nz, 1), L.kp, L.n), device=self.device, dtype=torch.float32)
         check(self._lib.wg_pc_conv_wgrad(_p(x), columns, _p(dy16), B, H, W, L.dil, splits, _p(part), _p(self._status),
                                          _stream()), "gemm wgrad")
         return part
