@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "wave_launch.h"
 
@@ -180,18 +181,25 @@ __global__ void __launch_bounds__(kFoldThreads) fold_kernel(const float* __restr
 
 // Causal FIR along time of [series][nt][nrec] traces: out[t] = sum over k, in order, of ker[k]
 // x[t - (klen - 1) + k], times before 0 left out. One thread takes one trace (neighbouring threads
-// neighbouring receivers, across series, so that no lane idles on 70 receivers) and FIR_R samples in
-// a row: their inputs slide through registers, so a tap costs one load of x and one of ker for FIR_R
+// neighbouring receivers, across series, so that no lane idles on 70 receivers) and R samples in
+// a row: their inputs slide through registers, so a tap costs one load of x and one of ker for R
 // products and sums, which FP32 issue then bounds (products and sums are not fused: each rounds as
 // the one-sample-per-thread kernel's did, which two loads per product bounded). 16 models x 5 shots x
 // 2001 x 70 at 377 taps: 0.35 against 3.2 ms; the FP32 bound is 0.21 ms (0.38 with the end of the record
 // tested at every load and each load next to its use).
-constexpr int FIR_R = 16;
+//
+// R is 16, or 4 for small calls (few outputs, few taps that any of them has): those are one latency chain per
+// thread, of R (R - 1) / 2 guarded taps and the window's loads, and want many short ones. Us for R = 4 / 16 (one
+// sample per thread): 70 traces x 400 at 31 taps 3.9 / 6.8 (3.5), x 2001 at 31 4.0 / 6.9 (6.5); 1400 x 400 at
+// 31 6.9 / 7.0 (17.4); 350 x 2001 at 101 19.9 / 12.1 (60.9); 70 x 400 at 377 28.3 / 18.6 (22.8). The line lies
+// where the two meet.
 constexpr int FIR_THREADS = 128;
+constexpr long kFirFewProducts = 8L << 20;   // outputs times taps
+constexpr int kFirFewTaps = 128;
 
-// CHECK: fewer than FIR_R times, so a thread's samples may lie past the last; otherwise the last block of
-// times starts at nt - FIR_R and stores only the samples that the one before it does not.
-template <bool CHECK>
+// CHECK: fewer than R times, so a thread's samples may lie past the last; otherwise the last block of
+// times starts at nt - R and stores only the samples that the one before it does not.
+template <int FIR_R, bool CHECK>
 __global__ void __launch_bounds__(FIR_THREADS) bandlimit_kernel(const float* __restrict__ in, const float* __restrict__ ker,
                                                                 int klen, long traces, int nt, int nrec,
                                                                 float* __restrict__ out) {
@@ -319,11 +327,19 @@ cudaError_t launch_fold(const float* gacc, const float* mask, int models, int sh
 cudaError_t launch_bandlimit(const float* in, const float* ker, int klen, int series, int nt, int nrec, float* out,
                              cudaStream_t s) {
   const long traces = static_cast<long>(series) * nrec;
-  const dim3 grid(static_cast<unsigned>((traces + FIR_THREADS - 1) / FIR_THREADS), (nt + FIR_R - 1) / FIR_R);
-  if (nt < FIR_R)
-    bandlimit_kernel<true><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+  const int taps = std::min(klen, nt);  // of an output, at most
+  auto launch = [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    const dim3 grid(static_cast<unsigned>((traces + FIR_THREADS - 1) / FIR_THREADS), (nt + R - 1) / R);
+    if (nt < R)
+      bandlimit_kernel<R, true><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+    else
+      bandlimit_kernel<R, false><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+  };
+  if (taps <= kFirFewTaps && traces * nt <= kFirFewProducts / taps)
+    launch(std::integral_constant<int, 4>());
   else
-    bandlimit_kernel<false><<<grid, FIR_THREADS, 0, s>>>(in, ker, klen, traces, nt, nrec, out);
+    launch(std::integral_constant<int, 16>());
   return cudaGetLastError();
 }
 
