@@ -91,6 +91,36 @@ __device__ __forceinline__ float ex2(float x) {
   return r;
 }
 
+// The gradient of a slot whose log scales lie far outside the activation's bounds (log 0.5 to log 6), where
+// the moments below would overflow or lose their digits: every product formed per pixel, in unscaled
+// distances, and reduced over the warp.
+constexpr float kMomentScale = 4.0f;  // largest |log scale| that takes the moments
+__device__ __noinline__ void render_bwd_direct(const SlotC k, const float* cb, int i, int lane, float* grad) {
+  const int z0 = 2 * (i / SIDE) - WIN, x0 = 2 * (i % SIDE) - WIN;
+  float g[NPAR] = {};
+  for (int q = lane; q < (2 * WIN + 1) * (2 * WIN + 1); q += 32) {
+    const int pz = z0 + q / (2 * WIN + 1), px = x0 + q % (2 * WIN + 1);
+    if (pz < 0 || pz >= GRID || px < 0 || px >= GRID) continue;
+    const float dx = (static_cast<float>(px) + 0.5f) - k.cx, dz = (static_cast<float>(pz) + 0.5f) - k.cz;
+    const float ru = dx * k.c + dz * k.s, rv = dz * k.c - dx * k.s;
+    const float u = ru * k.isx, v = rv * k.isz;
+    const float e = expf(-0.5f * (u * u + v * v)), ct = cb[pz * GRID + px];
+    const float ge = ct * k.w * e;  // cotangent times d/d(-0.5 (u^2 + v^2)) of the contribution
+    // du/dcx = -c isx, dv/dcx = s isz; du/dcz = -s isx, dv/dcz = -c isz; dru/dangle = rv, drv/dangle = -ru
+    g[0] += -ge * (u * (-k.c * k.isx) + v * (k.s * k.isz));
+    g[1] += -ge * (u * (-k.s * k.isx) + v * (-k.c * k.isz));
+    g[2] += ge * u * u;
+    g[3] += ge * v * v;
+    g[4] += -ge * (u * rv * k.isx - v * ru * k.isz);
+    g[5] += ct * e;
+  }
+#pragma unroll
+  for (int j = 0; j < NPAR; ++j) {
+    for (int o = 16; o > 0; o >>= 1) g[j] += __shfl_down_sync(0xffffffffu, g[j], o);
+    if (lane == 0) grad[j] = g[j];
+  }
+}
+
 // One warp per slot: lane l takes window column l (25 of 32 lanes) and walks the window's rows inside
 // the grid, so dx's products are loop constants and the pixel index needs no division. With
 //   u = (dx c + dz s) / sx K,  v = (dz c - dx s) / sz K,  K = sqrt(log2(e) / 2)
@@ -108,6 +138,10 @@ __global__ void __launch_bounds__(256) render_bwd_kernel(const float* __restrict
   const float* p = params + static_cast<size_t>(warp) * NPAR;
   constexpr float K = 0.84932180028801904f;
   const SlotC k = slot_consts(p, i);
+  if (!(fabsf(p[2]) <= kMomentScale && fabsf(p[3]) <= kMomentScale)) {
+    render_bwd_direct(k, cot + static_cast<size_t>(b) * GRID * GRID, i, lane, grad + static_cast<size_t>(warp) * NPAR);
+    return;
+  }
   const float uc = k.c * (k.isx * K), us = k.s * (k.isx * K), vc = k.c * (k.isz * K), vs = k.s * (k.isz * K);
   const int iz = i / SIDE, ix = i % SIDE;
   const int px = 2 * ix + lane - WIN;
