@@ -51,3 +51,34 @@ def test_a_batch_that_the_workspaces_hold_is_not_cut_up(cuda_lib):
     assert runs[1][0] == runs[0][0]
     np.testing.assert_array_equal(runs[1][1], runs[0][1])
     np.testing.assert_array_equal(runs[1][2], runs[0][2])
+
+
+def _survey(shots, nt=24):
+    from wgnet_gb300.engine import WaveEngine
+
+    eng = WaveEngine(shots=shots, nt=nt, dt=0.0005, h=5.0, nx_vis=276, nz_vis=116)
+    eng.set_option("streamed", 1)
+    return eng
+
+
+def test_the_streamed_forward_needs_no_memory_beyond_one_step_per_launch(cuda_lib):
+    """18 shots of 320 x 160 cells are 450 tiles: by default four steps per launch, whose two state sets take 22 MiB.
+    Where these do not fit but one step's state (17 MiB, in pages of two) does, the call takes one step per launch."""
+    import torch
+
+    vel = _models(1, 116, 276)
+    warm = _survey(2)  # every kernel of both ways is loaded before memory is short
+    warm.simulate_torch(vel)
+    warm.set_option("temporal_block", 0)
+    warm.simulate_torch(vel)
+    ref = _survey(18)
+    want = ref.simulate_torch(vel)
+    torch.cuda.synchronize()
+    eng = _survey(18)
+    spare = torch.empty_like(want)  # the call's own output comes from here
+    with _all_held_but(20 << 20) as left:
+        if not 18 << 20 <= left <= 21 << 20:
+            pytest.skip(f"{left} bytes free")
+        del spare
+        got = eng.simulate_torch(vel)
+    assert torch.equal(got, want)

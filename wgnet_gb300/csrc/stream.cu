@@ -1087,7 +1087,7 @@ int wait_timeout_selftest(int* d_status, long long polls, cudaStream_t st) {
 struct StreamWork {
   Buf vpad, mask, traces, energy, scale, part, stored, ckpt, gacc;
   Buf W, PX, ZX, PZ, ZZ;        // forward state
-  Buf Wtb, PXtb, ZXtb, PZtb, ZZtb;  // temporally blocked forward: two state sets
+  Buf tb;                       // temporally blocked forward: two state sets
   Buf L, LPX, LZX, LPZ, LZZ;    // adjoint state
   Buf tile_rec_start, tile_rec;
   int rec_tiles_nx = -1, rec_tiles_nz = -1, rec_z0 = 0, rec_z1 = -1;
@@ -1256,31 +1256,34 @@ int adj_step(StreamWork* w, const CUtensorMap& map, SArgs a, int t, cudaStream_t
   return WG_OK;
 }
 
-// The blocked kernels' two state sets.
-cudaError_t tb_state(StreamWork* w, const EngineView& v, int units) {
+// The blocked kernels' two state sets, in one allocation: a part that fails leaves nothing behind that
+// the kernels of one step per launch, which then run, would miss.
+struct TbLayout {
+  size_t W, PX, ZX, PZ, ZZ, bytes;  // byte offsets, total
+};
+
+TbLayout tb_layout(const EngineView& v, int units) {
   const size_t nW = static_cast<size_t>(units) * v.nx * v.nz, nX = units * xs_floats(v), nZ = units * zs_floats(v);
-  cudaError_t e = w->Wtb.ensure(4 * nW * 4);
-  if (e == cudaSuccess) e = w->PXtb.ensure(2 * nX * 4);
-  if (e == cudaSuccess) e = w->ZXtb.ensure(2 * nX * 4);
-  if (e == cudaSuccess) e = w->PZtb.ensure(2 * nZ * 4);
-  if (e == cudaSuccess) e = w->ZZtb.ensure(2 * nZ * 4);
-  return e;
+  auto up = [](size_t floats) { return (floats * 4 + 255) & ~size_t(255); };
+  TbLayout l{};
+  l.PX = l.W + up(4 * nW);
+  l.ZX = l.PX + up(2 * nX);
+  l.PZ = l.ZX + up(2 * nX);
+  l.ZZ = l.PZ + up(2 * nZ);
+  l.bytes = l.ZZ + up(2 * nZ);
+  return l;
 }
 
 // Temporally blocked forward over all units from the zero state, TB_T steps per launch: receivers
 // into `traces` and, when `stored` is given, every step's gradient term (the store-all scheme).
 int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float* traces, float* stored,
                cudaStream_t st) {
-  const size_t cells = static_cast<size_t>(v.nx) * v.nz;
-  const size_t nW = static_cast<size_t>(units) * cells, nX = units * xs_floats(v), nZ = units * zs_floats(v);
-  SW_CK(tb_state(w, v, units));
-  SW_CK(cudaMemsetAsync(w->Wtb.p, 0, 4 * nW * 4, st));
-  SW_CK(cudaMemsetAsync(w->PXtb.p, 0, 2 * nX * 4, st));
-  SW_CK(cudaMemsetAsync(w->ZXtb.p, 0, 2 * nX * 4, st));
-  SW_CK(cudaMemsetAsync(w->PZtb.p, 0, 2 * nZ * 4, st));
-  SW_CK(cudaMemsetAsync(w->ZZtb.p, 0, 2 * nZ * 4, st));
+  const TbLayout l = tb_layout(v, units);
+  SW_CK(w->tb.ensure(l.bytes));
+  SW_CK(cudaMemsetAsync(w->tb.p, 0, l.bytes, st));
+  auto part = [&](size_t at) { return reinterpret_cast<float*>(static_cast<char*>(w->tb.p) + at); };
   CUtensorMap um, vm;
-  int rc = make_map(&um, w->Wtb.f(), v.nx, v.nz, 4 * units, TB_RX, TB_RZ);
+  int rc = make_map(&um, part(l.W), v.nx, v.nz, 4 * units, TB_RX, TB_RZ);
   if (rc == WG_OK) rc = make_map(&vm, w->vpad.f(), v.nx, v.nz, models, TB_RX, TB_RZ);
   if (rc != WG_OK) return rc;
   TbArgs p{};
@@ -1290,11 +1293,11 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
   p.a.stored = stored;
   p.a.seg = v.nt;
   p.a.seg_t0 = 0;
-  p.W = w->Wtb.f();
-  p.PX = w->PXtb.f();
-  p.ZX = w->ZXtb.f();
-  p.PZ = w->PZtb.f();
-  p.ZZ = w->ZZtb.f();
+  p.W = part(l.W);
+  p.PX = part(l.PX);
+  p.ZX = part(l.ZX);
+  p.PZ = part(l.PZ);
+  p.ZZ = part(l.ZZ);
   const int jobs = units * p.a.tiles_x * p.a.tiles_z;
   const int blocks = std::min(jobs, w->tb_blocks);
   for (int t = 0, k = 0; t < v.nt; t += TB_T, ++k) {
@@ -1320,7 +1323,7 @@ constexpr int kTbWaves = 3;
 bool blocked(StreamWork* w, const EngineView& v, int units) {
   if (v.tblock >= 0) return v.tblock != 0;
   const long jobs = static_cast<long>(units) * ((v.nx + TX_ - 1) / TX_) * ((v.nz + TZ_ - 1) / TZ_);
-  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks && tb_state(w, v, units) == cudaSuccess;
+  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks && w->tb.ensure(tb_layout(v, units).bytes) == cudaSuccess;
 }
 
 // Checkpoint slot layout: [W(t) | W(t-1) | PX(t) | ZX | PZ(t) | ZZ] for all units.
