@@ -82,3 +82,46 @@ def test_the_streamed_forward_needs_no_memory_beyond_one_step_per_launch(cuda_li
         del spare
         got = eng.simulate_torch(vel)
     assert torch.equal(got, want)
+
+
+def _captured(call):
+    """The results of `call`, captured into a graph on the stream it runs on, from a replay."""
+    import torch
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = call()
+    g.replay()
+    torch.cuda.synchronize()
+    return g, out
+
+
+def test_a_smaller_batch_than_the_warm_up_can_be_captured(cuda_lib):
+    """48 models x 5 shots x 400 steps checkpoint (5 GB of terms); 7 of them would keep their terms by default, in a
+    buffer that the warm-up did not allocate. Captured, they take the checkpoints; a later call that does keep
+    terms leaves the captured one's buffers where they are."""
+    import torch
+
+    from wgnet_gb300.engine import WaveEngine
+
+    eng = WaveEngine(shots=5, nt=400, dt=0.001)
+    vel = _models(48)
+    obs = eng.simulate_torch(vel * 1.02)
+    few, few_obs = vel[:7].contiguous(), obs[:7].contiguous()
+    loss, grad = eng.evaluate_adjoint_torch(vel, obs)
+    g, got = _captured(lambda: eng.evaluate_adjoint_torch(few, few_obs, check_status=False))
+    assert torch.equal(got[0], loss[:7]) and torch.equal(got[1], grad[:7])
+    for n in (7, 12):  # eager calls that keep their terms
+        again = eng.evaluate_adjoint_torch(vel[:n], obs[:n])
+        assert torch.equal(again[1], grad[:n])
+    got[1].zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[1], grad[:7])
+    # captured with kept terms: the buffer does not move for a larger batch
+    g2, got2 = _captured(lambda: eng.evaluate_adjoint_torch(few, few_obs, check_status=False))
+    assert torch.equal(eng.evaluate_adjoint_torch(vel[:20], obs[:20])[1], grad[:20])
+    got2[1].zero_()
+    g2.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got2[1], grad[:7])

@@ -169,6 +169,8 @@ struct wg_engine {
   size_t prof_used = 0;
   // workspace
   DevBuf w_vis, w_obs, w_vpad, w_mask, w_traces, w_energy, w_scale, w_loss, w_grad, w_ckpt, w_stored, w_adj, w_gacc;
+  DevBuf w_kept;               // gradient terms kept by default (store_by_default)
+  bool kept_captured = false;  // a captured call reads them: the buffer stays where it is
   std::mutex mu;
 
   wg::Grid grid() const {
@@ -616,19 +618,24 @@ int simulate_dev_impl(wg_engine* e, const float* d_vis, int models, float* d_tra
 // the gradient is the same bit for bit) when the batch's terms are small beside the memory: at most
 // kStoreBytes and an eighth of what is free, and the allocation succeeds; the buffer then stays with
 // the engine, as its other workspaces do. One default-engine gradient (5 shots, nt 2001, 0.5 GB of
-// terms): 1 x 2001 steps of forward saved, 3.7 of 14 ms.
+// terms): 1 x 2001 steps of forward saved, 3.7 of 14 ms. The terms have a buffer of their own, which does
+// not grow while a call is being captured into a graph, nor once a captured call reads it: as with
+// checkpoints alone, a call within what earlier ones have warmed up allocates nothing in a capture and
+// moves no buffer that a captured one reads.
 constexpr size_t kStoreBytes = size_t(4) << 30;
-bool store_by_default(wg_engine* e, int models) {
+bool store_by_default(wg_engine* e, int models, cudaStream_t st) {
   if (e->ck_set) return false;
   const size_t need = static_cast<size_t>(models) * e->shots * e->nt * e->cells * 4;
   if (need > kStoreBytes) return false;
-  if (need <= e->w_stored.bytes) return true;
+  const bool held = need <= e->w_kept.bytes, captured = wg::being_captured(st);
+  if (held && captured) e->kept_captured = true;
+  if (held || captured || e->kept_captured) return held;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return need <= free_b / 8 && e->w_stored.ensure(need) == WG_OK;
+  return need <= free_b / 8 && e->w_kept.ensure(need) == WG_OK;
 }
 
 // obs_ready (optional): an event the observed data's arrival is recorded on; nothing reads them
@@ -643,7 +650,9 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
                                timer_of(e));
   }
   if (e->ashape.cluster == 0) return fail(WG_ERR_UNSUPPORTED, "grid does not fit the resident adjoint kernel");
-  const bool store_all = e->ck_every <= 0 || e->ck_every >= e->nt || store_by_default(e, models);
+  const bool asked = e->ck_every <= 0 || e->ck_every >= e->nt;
+  const bool store_all = asked || store_by_default(e, models, st);
+  DevBuf& terms = store_all && !asked ? e->w_kept : e->w_stored;
   const int k = store_all ? e->nt : e->ck_every;
   const int J = store_all ? 1 : (e->nt + k - 1) / k;
   const int slots = J - 1;
@@ -657,7 +666,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
                                       {&e->w_energy, 8},
                                       {&e->w_scale, 4},
                                       {&e->w_ckpt, S * slots * ckf * 4},
-                                      {&e->w_stored, S * seg * cells * 4},
+                                      {&terms, S * seg * cells * 4},
                                       {&e->w_adj, S * asf * 4},
                                       {&e->w_gacc, S * cells * 4}});
   WG_TRY(e->w_vpad.ensure(M * cells * 4));
@@ -666,7 +675,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
   WG_TRY(e->w_energy.ensure(M * 8));
   WG_TRY(e->w_scale.ensure(M * 4));
   if (slots > 0) WG_TRY(e->w_ckpt.ensure(M * S * slots * ckf * 4));
-  WG_TRY(e->w_stored.ensure(M * S * seg * cells * 4));
+  WG_TRY(terms.ensure(M * S * seg * cells * 4));
   // adjoint state; until the first adjoint pass it is scratch of the misfit's reductions (kRedParts
   // doubles per model: an adjoint state is at least 4 KB even without a C-PML)
   WG_TRY(e->w_adj.ensure(M * S * asf * 4));
@@ -690,7 +699,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
     f.status = e->d_status.as<int>();
     f.fast = e->fast;
     if (store_all) {
-      f.stored = e->w_stored.as<float>();
+      f.stored = terms.as<float>();
       WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, true, f, st); }));
     } else {
       // Steps [0, (J-1) k] with receivers and checkpoints (the last checkpoint is written at the
@@ -708,7 +717,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
       l.ck_out = nullptr;
       l.ck_in = e->w_ckpt.as<float>();
       l.ck_in_slot = J - 2;
-      l.stored = e->w_stored.as<float>();
+      l.stored = terms.as<float>();
       WG_LAUNCH(timed(e, K_FWD, st, [&] { return wg::launch_fwd(fs, true, true, l, st); }));
     }
     if (obs_ready && m0 == 0) WG_CK(cudaStreamWaitEvent(st, obs_ready, 0));
@@ -723,7 +732,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
     a.vel = e->w_vpad.as<float>();
     a.units = units;
     a.residual = e->w_traces.as<float>();
-    a.stored = e->w_stored.as<float>();
+    a.stored = terms.as<float>();
     a.state = e->w_adj.as<float>();
     a.gacc = e->w_gacc.as<float>();
     a.status = e->d_status.as<int>();
@@ -747,7 +756,7 @@ int gradient_dev_impl(wg_engine* e, const float* d_vis, const float* d_obs, int 
         r.ck_in_slot = j - 1;
         r.ck_slots = slots;
         r.ck_every = k;
-        r.stored = e->w_stored.as<float>();
+        r.stored = terms.as<float>();
         r.status = e->d_status.as<int>();
         r.fast = e->fast;
         if (j < J - 1)  // the last segment's terms are already stored by the first pass

@@ -48,6 +48,16 @@ cudaError_t fwd3f_dispatch(bool traces, bool store, const FwdArgs& a, size_t sme
 cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a, cudaStream_t stream);
 cudaError_t launch_adj(const Shape& s, const AdjArgs& a, cudaStream_t stream);
 
+// Whether `s` is being captured into a graph (or cannot be asked): nothing may be allocated then.
+inline bool being_captured(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
 // --- auxiliary kernels (aux_kernels.cu) ---
 
 // Edge-replicate [models][nz_vis][nx_vis] velocities onto the padded grid, clamp to [vmin, vmax]
