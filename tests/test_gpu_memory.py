@@ -125,3 +125,24 @@ def test_a_smaller_batch_than_the_warm_up_can_be_captured(cuda_lib):
     g2.replay()
     torch.cuda.synchronize()
     assert torch.equal(got2[1], grad[:7])
+
+
+def test_fewer_streamed_models_than_the_warm_up_can_be_captured(cuda_lib):
+    """10 models x 2 shots are 500 tiles (one step per launch), 2 models 100 (four by default, from a state that the
+    warm-up did not allocate)."""
+    import torch
+
+    eng = _survey(2)
+    vel = _models(10, 116, 276)
+    want = eng.simulate_torch(vel)
+    few = vel[:2].contiguous()
+    g, got = _captured(lambda: eng.simulate_torch(few, check_status=False))
+    assert torch.equal(got, want[:2])
+    assert torch.equal(eng.simulate_torch(few), want[:2])  # four steps per launch
+    g2, got2 = _captured(lambda: eng.simulate_torch(few, check_status=False))
+    assert torch.equal(eng.simulate_torch(vel[:4]), want[:4])  # its state would not fit the captured call's
+    for graph, out in ((g, got), (g2, got2)):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[:2])

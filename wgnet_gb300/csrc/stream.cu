@@ -1088,6 +1088,7 @@ struct StreamWork {
   Buf vpad, mask, traces, energy, scale, part, stored, ckpt, gacc;
   Buf W, PX, ZX, PZ, ZZ;        // forward state
   Buf tb;                       // temporally blocked forward: two state sets
+  bool tb_captured = false;     // a captured call reads them: the buffer stays where it is
   Buf L, LPX, LZX, LPZ, LZZ;    // adjoint state
   Buf tile_rec_start, tile_rec;
   int rec_tiles_nx = -1, rec_tiles_nz = -1, rec_z0 = 0, rec_z1 = -1;
@@ -1320,10 +1321,17 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
 // us per step (recording traces), blocked against one step per launch: 50 tiles (2 shots of 284 x 154
 // cells) 3.4 / 5.8, 150 tiles 3.4 / 6.0, 252 tiles 6.1 / 6.7, 420 tiles 8.1 / 9.0, 546 tiles 10.7 / 9.4.
 constexpr int kTbWaves = 3;
-bool blocked(StreamWork* w, const EngineView& v, int units) {
+bool blocked(StreamWork* w, const EngineView& v, int units, cudaStream_t st) {
   if (v.tblock >= 0) return v.tblock != 0;
   const long jobs = static_cast<long>(units) * ((v.nx + TX_ - 1) / TX_) * ((v.nz + TZ_ - 1) / TZ_);
-  return jobs <= static_cast<long>(kTbWaves) * w->tb_blocks && w->tb.ensure(tb_layout(v, units).bytes) == cudaSuccess;
+  if (jobs > static_cast<long>(kTbWaves) * w->tb_blocks) return false;
+  // the choice is the library's: it does not allocate where the call is being captured into a graph, nor move
+  // a buffer that a captured call reads
+  const size_t need = tb_layout(v, units).bytes;
+  const bool held = need <= w->tb.bytes, captured = being_captured(st);
+  if (held && captured) w->tb_captured = true;
+  if (held || captured || w->tb_captured) return held;
+  return w->tb.ensure(need) == cudaSuccess;
 }
 
 // Checkpoint slot layout: [W(t) | W(t-1) | PX(t) | ZX | PZ(t) | ZZ] for all units.
@@ -1376,7 +1384,7 @@ int stream_simulate(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   SW_CK(w->vpad.ensure(models * cells * 4));
   note_launch();
   SW_CK(launch_pad_velocity(d_vis, models, v.nx_vis, v.nz_vis, v.pad, v.vmin, v.vmax, w->vpad.f(), nullptr, st));
-  if (blocked(w, v, units)) {
+  if (blocked(w, v, units, st)) {
     timer.mark(0, true, st);
     if ((rc = tb_forward(w, v, units, models, d_traces, nullptr, st)) != WG_OK) return rc;
     timer.mark(0, false, st);
@@ -1482,7 +1490,7 @@ int stream_gradient(StreamWork* w, const EngineView& v, const int* h_rec_cell, c
   f.seg = seg;
   f.seg_t0 = 0;
   timer.mark(0, true, st);
-  if (store_all && blocked(w, v, units)) {
+  if (store_all && blocked(w, v, units, st)) {
     if ((rc = tb_forward(w, v, units, models, w->traces.f(), w->stored.f(), st)) != WG_OK) return rc;
   } else {
     for (int t = 0; t < v.nt; ++t) {
