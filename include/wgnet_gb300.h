@@ -248,6 +248,11 @@ int wg_pc_adam_layers(int layers, const float* const* d_partial, const int* spli
 int wg_pc_conv(int mode, const void* d_act_bf16, int batch, int h, int w, int dil, const void* d_wgt_bf16, int kp,
                const float* d_add, const void* d_mask_bf16, float* d_out32, void* d_out16, int* d_status,
                void* stream);
+/* Self-test of wg_pc_conv's time-out path (mode 0, dilation 1): no wait polls, so every one gives up at once,
+ * with copies in flight. The kernel sets *d_status, waits (bounded) for what is in flight and returns; d_out16
+ * holds nothing of meaning. */
+int wg_selftest_conv_timeout(const void* d_act_bf16, int batch, int h, int w, const void* d_wgt_bf16, void* d_out16,
+                             int* d_status, void* stream);
 /* Partials [P][576][64] of the convolution's transposed weight gradient from its input activations and
  * dL/dy [pixels][64] bf16; columns > 0: the input is a matrix [pixels][columns] and a partial has
  * `columns` rows. batch h w must be a multiple of 64. P is wg_pc_wgrad_partials(batch, h, w, splits), at

@@ -79,6 +79,7 @@ SIGNATURES: dict[str, tuple] = {
     "wg_pc_relu_grad": (_I, [_P, _P, ctypes.c_long, _P, _P]),
     "wg_pc_conv": (_I, [_I, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _P, _P]),
     "wg_pc_conv_wgrad": (_I, [_P, _I, _P, _I, _I, _I, _I, _I, _P, _P, _P]),
+    "wg_selftest_conv_timeout": (_I, [_P, _I, _I, _I, _P, _P, _P, _P]),
     "wg_pc_wgrad_partials": (_I, [_I, _I, _I, _I]),
     "wg_pc_out_dgrad": (_I, [_P, _P, _I, _I, _I, _P, _P, _P, _P]),
     "wg_pc_features": (_I, [_P, _P, _P, _I, _I, _I, _P, _P, _P]),

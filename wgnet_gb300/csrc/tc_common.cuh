@@ -25,9 +25,9 @@ __device__ __forceinline__ void bar_init(uint64_t* b, unsigned n) {
 __device__ __forceinline__ void bar_expect(uint64_t* b, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned parity) {
+__device__ __forceinline__ bool bar_wait(uint64_t* b, unsigned parity, long limit = kTcWaitLimit) {
   const unsigned a = su32(b);
-  for (long i = 0; i < kTcWaitLimit; ++i) {
+  for (long i = 0; i < limit; ++i) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"

@@ -55,6 +55,7 @@ struct ConvArgs {
   float* out32;
   __nv_bfloat16* out16;
   int* status;
+  long polls;                    // limit of a wait
 };
 
 // Shared memory: weights [kt][N rows][128 B] | boxes in flight | staging tile | barriers.
@@ -106,8 +107,9 @@ __device__ __forceinline__ bool bf16_positive(uint32_t pair, int hi) {
 // matrix). Warp 0 (one lane) loads the tile's boxes, warp 1 (one lane) issues the MMAs, warps 2-9 run the epilogue. The data gradient keeps
 // one accumulator per tap (the reference route rounds each tap's product to FP32 before it sums the
 // taps): the epilogue adds the nine in tap order. Every wait is bounded; a warp that gives up
-// records the error, the others follow through their own waits, and the CTA drains the copies and
-// MMAs in flight (bounded) before it frees its tensor memory.
+// records the error and the others follow through their own waits; then the MMA lane waits (bounded) for
+// every MMA it issued, those of an unfinished tile included, before the tensor memory is freed, and a
+// thread for every copy before the CTA ends.
 template <int MODE>
 __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ CUtensorMap mapA,
                                                        const __grid_constant__ CUtensorMap mapB,
@@ -127,8 +129,9 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
   uint64_t* acc_full = empty + CST;
   uint64_t* acc_empty = acc_full + NACC;
   uint64_t* wbar = acc_empty + NACC;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wbar + 1);
-  __shared__ int fail;
+  uint64_t* drained = wbar + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  __shared__ int fail, boxes_issued;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kt = a.kt, tiles = a.tiles, stages = a.stages;
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       bar_init(&acc_empty[b], CEPI);
     }
     bar_init(wbar, 1);
+    bar_init(drained, 1);
     fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       for (int tl = blockIdx.x; ok && tl < tiles; tl += gridDim.x) {
         const int n = tl / a.tiles_img, r = tl - n * a.tiles_img, ty = r / a.tiles_x, tx = r - ty * a.tiles_x;
         for (int t = 0; t < boxes; ++t, ++it) {
-          if (it >= stages && !bar_wait(&empty[s], phase)) {
+          if (it >= stages && !bar_wait(&empty[s], phase, a.polls)) {
             ok = false;
             break;
           }
@@ -181,10 +185,10 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
           }
         }
       }
+      boxes_issued = it;
       if (!ok) {
         fail = 1;
         atomicCAS(a.status, 0, ST_CUDA);
-        for (int k = 1; k <= stages && it - k >= 0; ++k) bar_wait(&full[(it - k) % stages], ((it - k) / stages) & 1);
       }
     }
     __syncwarp();
@@ -193,19 +197,17 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       constexpr uint32_t idesc = idesc_bf16(CBM, N);
       const uint32_t a0 = desc_lo(su32(sA)), b0 = desc_lo(su32(sB));
       const uint32_t box = a.box >> 4, row = a.dil * (CTW * 128 >> 4);  // a box, dil of its rows
-      bool ok = bar_wait(wbar, 0);
+      bool ok = bar_wait(wbar, 0, a.polls);
       int s = 0, phase = 0;                 // ring position of the next box and its parity
       int acc = 0, acc_phase = 1;           // next accumulator; the parity of the phase before it
-      int it = 0, freed = 0;                // boxes taken, and released
       // one lane's loop over 36 MMAs per tile: descriptors and ring positions advance by additions
       auto take = [&](uint32_t& lo) {       // wait for the next box; its operand's descriptor
-        if (!bar_wait(&full[s], phase)) return false;
+        if (!bar_wait(&full[s], phase, a.polls)) return false;
         lo = a0 + s * box;
         if (++s == stages) {
           s = 0;
           phase ^= 1;
         }
-        ++it;
         return true;
       };
       auto mmas = [&](uint32_t at, uint32_t wt, bool first) {
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
         for (int kk = 0; kk < 4; ++kk) mma_bf16_lo(tmem + acc * N, at + 2 * kk, wt + 2 * kk, idesc, !first || kk > 0);
       };
       auto open = [&]() {                   // wait until the next accumulator has been read
-        if (!bar_wait(&acc_empty[acc], acc_phase)) return false;
+        if (!bar_wait(&acc_empty[acc], acc_phase, a.polls)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         return true;
       };
@@ -233,7 +235,6 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
             if (!(ok = take(lo))) break;
             mmas(lo, b0 + t * (N * 128 >> 4), t == 0);
             mma_commit(&empty[at]);
-            freed = it;
           }
           if (ok) close();
         } else {
@@ -248,10 +249,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             mmas(lo[t % 3] + (DGRAD ? 2 - t / 3 : t / 3) * row, b0 + t * (N * 128 >> 4), DGRAD || t == 0);
-            if (t >= 6) {
-              mma_commit(&empty[at[t - 6]]);
-              freed = it - 8 + t;
-            }
+            if (t >= 6) mma_commit(&empty[at[t - 6]]);
             if (DGRAD || t == 8) close();
           }
         }
@@ -259,7 +257,6 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       if (!ok) {
         fail = 1;
         atomicCAS(a.status, 0, ST_CUDA);
-        for (int k = 1; k <= stages && freed - k >= 0; ++k) bar_wait(&empty[(freed - k) % stages], ((freed - k) / stages) & 1);
       }
     }
     __syncwarp();
@@ -281,7 +278,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
       };
       if constexpr (MODE == EPI_OUT1) {
         const int b = r % NACC;
-        ok = __all_sync(0xffffffffu, bar_wait(&acc_full[b], (r / NACC) & 1));
+        ok = __all_sync(0xffffffffu, bar_wait(&acc_full[b], (r / NACC) & 1, a.polls));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (half == 0) {
@@ -319,7 +316,7 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
 #pragma unroll 1
       for (int q = 0; q < rounds; ++q, ++r) {
         const int b = r % NACC;
-        ok = ok && __all_sync(0xffffffffu, bar_wait(&acc_full[b], (r / NACC) & 1));
+        ok = ok && __all_sync(0xffffffffu, bar_wait(&acc_full[b], (r / NACC) & 1, a.polls));
         if (ok) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           float t[32];
@@ -372,7 +369,17 @@ __global__ void __launch_bounds__(CTHR, 1) conv_kernel(const __grid_constant__ C
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (fail && tid == 32) {  // the MMAs still running (a commit follows those of its own thread)
+    mma_commit(drained);
+    bar_wait(drained, 0);
+  }
+  __syncwarp();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
+  if (fail && tid == 0) {  // the copies still landing
+    bar_wait(wbar, 0);
+    for (int k = 1; k <= stages && boxes_issued - k >= 0; ++k)
+      bar_wait(&full[(boxes_issued - k) % stages], ((boxes_issued - k) / stages) & 1);
+  }
 }
 
 // Weight gradient partials: part[z][k][n] = sum over the pixels of split z of x[pixel + tap(k)][c(k)]
@@ -603,11 +610,11 @@ bool bad_image(int batch, int h, int w, int dil) {
 }  // namespace
 }  // namespace wg
 
-extern "C" {
+namespace wg {
+namespace {
 
-int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, const void* d_wgt, int kp,
-               const float* d_add, const void* d_mask, float* d_out32, void* d_out16, int* d_status, void* stream) {
-  using namespace wg;
+int conv(int mode, const void* d_act, int batch, int h, int w, int dil, const void* d_wgt, int kp, const float* d_add,
+         const void* d_mask, float* d_out32, void* d_out16, int* d_status, void* stream, long polls) {
   const bool matrix = mode == EPI_FIRST, dgrad = mode >= EPI_MASK16;
   const bool needs_add = mode == EPI_RESID || mode == EPI_ACC || mode == EPI_ACC_MASK;
   const bool needs_mask = mode == EPI_MASK16 || mode == EPI_ACC_MASK;
@@ -630,6 +637,7 @@ int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, co
   a.out32 = d_out32;
   a.out16 = static_cast<__nv_bfloat16*>(d_out16);
   a.status = d_status;
+  a.polls = polls;
   a.tiles_x = (w + CTW - 1) / CTW;
   a.tiles_img = a.tiles_x * ((h + CTH - 1) / CTH);
   a.tiles = matrix ? (a.M + CBM - 1) / CBM : batch * a.tiles_img;
@@ -653,6 +661,23 @@ int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, co
     case EPI_ACC: return conv_launch<EPI_ACC>(ma, mb, a, st);
     default: return conv_launch<EPI_ACC_MASK>(ma, mb, a, st);
   }
+}
+
+}  // namespace
+}  // namespace wg
+
+extern "C" {
+
+int wg_pc_conv(int mode, const void* d_act, int batch, int h, int w, int dil, const void* d_wgt, int kp,
+               const float* d_add, const void* d_mask, float* d_out32, void* d_out16, int* d_status, void* stream) {
+  return wg::conv(mode, d_act, batch, h, w, dil, d_wgt, kp, d_add, d_mask, d_out32, d_out16, d_status, stream,
+                  wg::kTcWaitLimit);
+}
+
+int wg_selftest_conv_timeout(const void* d_act, int batch, int h, int w, const void* d_wgt, void* d_out16, int* d_status,
+                             void* stream) {
+  return wg::conv(wg::EPI_RELU16, d_act, batch, h, w, 1, d_wgt, 64 * wg::CKT, nullptr, nullptr, nullptr, d_out16, d_status,
+                  stream, 0);
 }
 
 int wg_pc_wgrad_partials(int batch, int h, int w, int splits) {
