@@ -38,9 +38,12 @@ __device__ __forceinline__ SlotC slot_consts(const float* p, int i) {
 // iz in [n-6, n+6], row 2n+1 by [n-5, n+6] (and the same for the columns), so each slot's
 // constants, loaded once (two 128-bit loads), serve up to four pixels. Every pixel still sums its
 // slots in increasing slot order. Blocks (QBLK threads, blockIdx.y) split a model's 1225 quads; each
-// block stages all slot constants of its model (blockIdx.x). The arithmetic is the reference's, order
-// and all: refinement takes decisions on misfits that a differently rounded field moves by 1e-4.
-constexpr int QBLK = 416;
+// block stages all slot constants of its model (blockIdx.x). Small blocks spread a few models over the SMs and
+// waste little in a last wave: 1 / 30 / 64 / 256 models take 39 / 40 / 54 / 157 us with 160 threads, 40 / 38 / 63 /
+// 162 with 256, 47 / 45 / 71 / 173 with 416 (seven 32-bit loads per slot and 256 threads: 41 / 39 / 66 / 171).
+// The arithmetic is the reference's, order and all: refinement takes decisions on misfits that a
+// differently rounded field moves by 1e-4.
+constexpr int QBLK = 160;
 constexpr int QBLOCKS = (SLOTS + QBLK - 1) / QBLK;
 
 __global__ void __launch_bounds__(QBLK) render_fwd_kernel(const float* __restrict__ params, float* __restrict__ field) {
