@@ -1,6 +1,7 @@
 // Kernels of the learned update network (a dilated residual conv net on the 70x70 model grid):
-// lowering of 3x3 convolutions to the tensor-core GEMM (im2col / col2im), layout transposes, the
-// elementwise glue of the residual blocks, input features, the training loss and the Adam update.
+// im2col of its 8-channel input, input features, the training loss and the Adam update. The convolutions
+// themselves are tc_conv.cu's; col2im, the transposes, casts, sums and masks here are the separate passes
+// that those fuse (with gemm_bf16_kernel the route that their results equal bit for bit).
 // No reference counterpart: WGNet's refine() (python/wgnet/refine.py:41-169) has no learned part.
 //
 // Layouts: activations [B][H][W][C] (channels contiguous); im2col columns [M][Kp] with

@@ -41,7 +41,7 @@ constexpr unsigned kTileBytes = BX * BZ * 4;
 constexpr long kWaitLimit = 1L << 22;       // mbarrier polls before giving up
 
 struct SArgs {
-  int nx, nz, units, shots, models_unused;
+  int nx, nz, units, shots;
   int tiles_x, tiles_z;
   int ssw;         // packed strip width per side (x strips: columns, z strips: rows)
   int region;      // PML region used for both axes (the adjoint's, pml + 3 FD_PAD)
@@ -230,7 +230,7 @@ __device__ __forceinline__ void issue_fwd(const SArgs& a, const FwdMaps& m, floa
 // two rows a thread instead of 8 of four, with two stages, to 27.9 and 25.8, for all that they spill a
 // little at 56 registers (three stages: 28.6 and 26.0; three CTAs of 8 warps: 29.0 and 26.8; four: 40.4
 // and 37.4). Loading the strips ahead for four rows spilled and measured slower (44 us). The adjoint holds
-// more and stays at 8 warps of four rows (16 of two: 55.8 against 51.3 us).
+// more and stays at 8 warps of four rows (16 of two: 55.8 against 51.5 us).
 template <bool TRACES, bool STORE>
 __global__ void __launch_bounds__(FWD_THREADS, 2) fwd_stream_kernel(const __grid_constant__ FwdMaps maps,
                                                                     const __grid_constant__ SArgs a) {
@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(NTH, 2) adj_stream_kernel(const __grid_constan
     // cell the velocity, lambda_prev, the stored term, the gradient and the strips' psi and zeta, and
     // the halo pair's. (Read between the rows' stores, each strip value cost an L2 latency; with the
     // overlapped launch, packed arithmetic and one barrier less a step of 16 shots of the 844 x 344
-    // grid went from 62 to 51.6 us, one of 10 shots of 344 x 194 from 18.3 to 14.4.)
+    // grid went from 62 to 51.5 us, one of 10 shots of 344 x 194 from 18.3 to 14.4.)
     float2 vv[RPT], lpv[RPT], stv[RPT], gav[RPT], xP[RPT], xZ[RPT], zP[RPT], zZ[RPT];
     float2 hv = make_float2(0.f, 0.f), hP = hv, hZ = hv;
     const bool in_x = x < nx;                                     // own pair inside the grid (nx is even)
@@ -1217,7 +1217,6 @@ int alloc_forward(StreamWork* w, const EngineView& v, int units, cudaStream_t st
   return WG_OK;
 }
 
-// One forward step over all units.
 // A step's launch, allowed to be scheduled while the step before it drains (see wait_for_previous_step).
 template <class... P, class... A>
 cudaError_t launch_step(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t st, const A&... args) {
@@ -1234,6 +1233,7 @@ cudaError_t launch_step(void (*kernel)(P...), int blocks, int threads, size_t sm
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// One forward step over all units.
 int fwd_step(StreamWork* w, const FwdMaps& map, SArgs a, int t, bool traces, bool store, cudaStream_t st) {
   a.t = t;
   const int jobs = a.units * a.tiles_x * a.tiles_z;
@@ -1318,8 +1318,11 @@ int tb_forward(StreamWork* w, const EngineView& v, int units, int models, float*
 // the engine option says, or, where it was not set, when its tiles fit the chip in three waves (and there is
 // memory for the second state set): a step is then
 // mostly the latency of its launch and copies, which four steps share.
-// us per step (recording traces), blocked against one step per launch: 50 tiles (2 shots of 284 x 154
-// cells) 3.4 / 5.8, 150 tiles 3.4 / 6.0, 252 tiles 6.1 / 6.7, 420 tiles 8.1 / 9.0, 546 tiles 10.7 / 9.4.
+// us per step (recording traces), blocked against one step per launch, shots of 284 x 154 cells (25 tiles):
+// 50 to 150 tiles 3.5 / 5.9, 200 5.8 / 6.7, 300 5.9 / 7.0, 325 (a third wave just begun) 8.8 / 9.0, 375 8.9 / 9.7,
+// 450 8.8 / 10.3, 475 10.5 / 10.4, 525 11.2 / 10.6; shots of 464 x 224 cells (56 tiles): 280 6.0 / 6.7, 336 8.5 /
+// 8.1, 392 8.5 / 9.1, 448 8.5 / 9.6, 504 11.1 / 9.7. A wave costs the same however full; the start of the third is
+// the one place within the line where one step per launch can be as fast.
 constexpr int kTbWaves = 3;
 bool blocked(StreamWork* w, const EngineView& v, int units, cudaStream_t st) {
   if (v.tblock >= 0) return v.tblock != 0;

@@ -1,4 +1,4 @@
-// Explicit instantiation of the generation-3 kernels for grids of any width up to 116 (see wave_table.cu).
+// Explicit instantiation of the generation-3 kernels for grids of any width up to 144 (see wave_table.cu).
 #include "wave_kernels3.cuh"
 
 namespace wg {

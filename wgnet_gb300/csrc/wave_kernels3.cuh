@@ -86,20 +86,12 @@ struct PairIo {
   }
 };
 
-// Shapes whose warps take the host's assignment (map_warps). Measured (us; 64 models of 70 x 70, or 4 in
-// clusters of three; 200 steps forward / adjoint), fixed roles -> map: {C 2, S 5} 4139 -> 4012 / 4800 ->
-// 4880 (the adjoint takes {2, 4}), {2, 4} 4680 -> 4590 / 5240 -> 4660, {3, 4} 716 -> 692 / 771 -> 750.
-// Elsewhere the map's registers or its order cost more than the balance gives: {3, 3} 696 -> 717, {4, 4}
-// 590 -> 607, and with several interior warps per segment the adjoint spills (6.0 -> 6.6 ms on 100 x 100).
-template <int C, int S, int NI>
-constexpr bool kMapped = NI == 1 && (C == 2 || (C == 3 && S == 4));
-
 // Part of warp `warp`: segment * (1 + NI) + role (0: the PML warp). Without a map the warps follow the
 // segments; with 2 or 4 warps per segment a fixed role per position would put every PML warp on the
 // same schedulers (warp w issues from scheduler w % 4), so there the roles rotate.
 template <int C, int S, int NI>
 __device__ __forceinline__ int warp_part(const WarpMap& m, int rank, int warp) {
-  if constexpr (kMapped<C, S, NI>) return m.id[rank][warp];
+  if constexpr (warps_mapped(C, S, NI)) return m.id[rank][warp];
   constexpr int W = 1 + NI;
   if constexpr (4 % W != 0) return warp;
   const int seg = warp / W;

@@ -208,7 +208,7 @@ static WarpMap warps_of(const Shape& s, int nz, int region, const WarpCosts& c) 
 
 cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& args, cudaStream_t stream) {
   FwdArgs a = args;
-  if (s.kind == 3 && s.ni == 1) a.warps = warps_of(s, a.g.nz, a.g.region, kFwdCosts);
+  if (s.kind == 3 && warps_mapped(s.cluster, s.seg_rows, s.ni)) a.warps = warps_of(s, a.g.nz, a.g.region, kFwdCosts);
   const size_t smem = fwd_smem_bytes(s, a.g.nx, a.g.nz, a.g.sw, a.st.nrec);
   if (s.kind == 3 && s.rag) {
 #define WG_FWD3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \
@@ -242,7 +242,7 @@ cudaError_t launch_fwd(const Shape& s, bool traces, bool store, const FwdArgs& a
 
 cudaError_t launch_adj(const Shape& s, const AdjArgs& args, cudaStream_t stream) {
   AdjArgs a = args;
-  if (s.kind == 3 && s.ni == 1) a.warps = warps_of(s, a.g.nz, a.g.region_adj, kAdjCosts);
+  if (s.kind == 3 && warps_mapped(s.cluster, s.seg_rows, s.ni)) a.warps = warps_of(s, a.g.nz, a.g.region_adj, kAdjCosts);
   const size_t smem = adj_smem_bytes(s, a.g.nx, a.g.nz, a.g.swa, a.st.nrec);
   if (s.kind == 3 && s.rag) {
 #define WG_ADJ3R(NXs, PMLPs, Cc, Ss, NSEGs, NIs)                                                                 \

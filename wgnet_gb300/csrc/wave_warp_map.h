@@ -14,6 +14,13 @@ struct WarpCosts {
   int row, pml, strip, halo;
 };
 
+// Shapes whose warps take the host's assignment. Measured (us; 64 models of 70 x 70, or 4 in
+// clusters of three; 200 steps forward / adjoint), fixed roles -> map: {C 2, S 5} 4139 -> 4012 / 4800 ->
+// 4880 (the adjoint takes {2, 4}), {2, 4} 4680 -> 4590 / 5240 -> 4660, {3, 4} 716 -> 692 / 771 -> 750.
+// Elsewhere the map's registers or its order cost more than the balance gives: {3, 3} 696 -> 717, {4, 4}
+// 590 -> 607, and with several interior warps per segment the adjoint spills (6.0 -> 6.6 ms on 100 x 100).
+constexpr bool warps_mapped(int C, int S, int NI) { return NI == 1 && (C == 2 || (C == 3 && S == 4)); }
+
 // Warp w issues from scheduler w % 4, and the parts of a CTA differ by up to a factor of four (PML warp or
 // interior warp, z-strip rows or not): the heaviest part left goes to the scheduler with the least to
 // issue so far that has a warp free. CTA r has the rows [bounds[r], bounds[r + 1]) of nz; segments of S
