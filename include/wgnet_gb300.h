@@ -100,7 +100,9 @@ int wg_selftest_wait_timeout(wg_engine* eng, long long polls, void* stream);
  * (its default) stores every step when that fits in 70% of the free device memory and otherwise
  * picks the interval that fits. An engine whose interval was never set (the getter then says 50) stores
  * every step of a batch whose terms take at most 4 GiB and an eighth of the free memory, and
- * checkpoints larger ones; the gradient is the same bit for bit. No reference counterpart for k > 0. */
+ * checkpoints larger ones; the gradient is the same bit for bit. While a call is captured into a graph those
+ * terms are kept only in a buffer that an earlier call has allocated, which then stays in place. No
+ * reference counterpart for k > 0. */
 int wg_set_checkpoint_interval(wg_engine* eng, int k);
 int wg_get_checkpoint_interval(const wg_engine* eng);
 
